@@ -5,6 +5,7 @@
 // the FP32 results reproducible operation by operation on the CPU.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <cuda_fp16.h>
@@ -19,6 +20,31 @@ struct GridDev {
     int64_t pitch, plane, vol;
 };
 
+// a / b rounded to nearest from y = recip_of(b), for divisors that many
+// quotients share: two residual corrections (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990: with a correctly rounded reciprocal and a quotient within one
+// unit, q + y (a - b q) is correctly rounded). The residuals are exact while
+// their last bits stay above the smallest subnormal: b in 2^-40 .. 2^40 (y is
+// NaN elsewhere) and a quotient in 2^-60 .. 2^80. A zero is its own quotient
+// (silent cells are common); everything else takes the division itself.
+__host__ __device__ inline float recip_of(float b) { return b >= 0x1p-40f && b <= 0x1p40f ? 1.0f / b : NAN; }
+__device__ __forceinline__ float div_shared(float a, float b, float y) {
+    const float q0 = a * y;
+    const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+    float q = __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+    if (!(fabsf(q) >= 0x1p-60f && fabsf(q) <= 0x1p80f)) q = a == 0.0f && y == y ? q0 : a / b;
+    return q;
+}
+
+// Quotients of one material that every point of it uses, each formed by the
+// point update's own operations, so that using them changes no rounding:
+// ratio = l a0 / b0, t1 = l2 / b0, t3 = a0 / (l b0), t4 = 1 / a0; rb = 1 / b0
+// and rden = 1 / (1 + ratio) for div_shared.
+struct alignas(16) LrsMat {
+    float b0, ratio, t1, t3, t4, rb, rden, pad;
+};
+
 // Compact boundary (LRS) list. Entry e: linear cell index, packed info
 // (group | mat0 << 5 | mat1 << 13 | mat2 << 21) and filter state
 // st_in/st_out[(b*S + slot)*n + e], S = 3*K slots per entry.
@@ -31,6 +57,7 @@ struct LrsDev {
     float* st_out;
     const float* ca;  // [nmat][K]
     const float* cb;  // [nmat][K]
+    const LrsMat* mat;  // [nmat]
     float l, l2, c2;  // coefficient l, l*l and 2(1-3*l*l)
 };
 
@@ -84,6 +111,20 @@ struct RcvDev {
     int64_t cap;
 };
 
+// Source cells and receivers taken by the step's own kernels (on != 0; see
+// src_rcv_role): n distinct source cells over all members; entry = the
+// cell's boundary entry, kSrcInterior for another cell 1..n-2, kSrcOuter on
+// an outer face; sources begin[k] .. begin[k+1]-1 of cell k in insertion
+// order, with their member, signal length and offset.
+struct SrcRcvDev {
+    int32_t on, n;
+    const int32_t *cell, *entry, *begin, *member;
+    const int64_t *len, *off;
+};
+constexpr int32_t kSrcInterior = -1, kSrcOuter = -2;
+// bit of an entry's packed info: a source lies in its cell
+constexpr uint32_t kSrcEntry = 1u << 31;
+
 // FP16 field storage (AFD_STORE_FP16, FIXED scheme): the three levels as
 // binary16 holding p * s, one power-of-two scale s per stored level and
 // batch member. The scale of level L (written at global step L) follows
@@ -98,18 +139,30 @@ struct F16Dev {
     const float* src_max;     // [batch] largest |source sample| of the member
 };
 
+// What global step g uses of everything that rotates: the levels' buffers
+// (new, p^n, p^{n-1}), the filters' ring slot, the PML level written and the
+// FP16 maximum slot (g mod 5). Kernels read it from a table of the chunk's
+// steps: formed in every thread, the 64-bit remainders were a third of the
+// list kernels' instructions.
+struct alignas(32) StepIdx {
+    long long g;
+    int wn, wc, wo, ix, lv, s5;
+};
+constexpr int kChunkSteps = 256;  // entries of the table; chunks have at most 200 steps
+
 struct StepArgs {
     GridDev g;
     int32_t batch;
     int32_t mode;             // AFD_MODE_REF / AFD_MODE_FIXED
     float* p[3];              // three rotating field buffers, each [batch][vol]
     F16Dev f16;
-    const long long* d_step;  // global step index at the start of the chunk
+    const StepIdx* idx;       // the steps of the chunk, by their offset j in it
     float lambda2, cint;      // interior: lambda^2 and 2(1-3 lambda^2)
     LrsDev lrs;
     PmlDev pml;
     SrcDev src;
     RcvDev rcv;
+    SrcRcvDev sr;
     int* flag;                // watchdog flag (bit0: |p| left the bound)
     // step timeline (off when tl_start is null): for global steps
     // tl_g0 .. tl_g0 + tl_steps - 1 and each of TL_SLOTS kernel kinds, the
@@ -158,6 +211,13 @@ __host__ __device__ inline int buf_old(long long g) { return (buf_new(g) + 2) % 
 // Ring slot written at global step g (simulation.hpp:365: decremented
 // before every step, starting from 0).
 __host__ __device__ inline int ring_index(long long g, int K) { return K - 1 - (int)(g % K); }
+
+// Step j of the chunk, in two 16-byte loads.
+__device__ __forceinline__ StepIdx step_at(const StepArgs& a, int j) {
+    const int4* p = reinterpret_cast<const int4*>(a.idx + j);
+    const int4 u = __ldg(p), v = __ldg(p + 1);
+    return StepIdx{(long long)(((unsigned long long)(uint32_t)u.y << 32) | (uint32_t)u.x), u.z, u.w, v.x, v.y, v.z, v.w};
+}
 
 // ---- FP16 storage ----------------------------------------------------------
 __host__ __device__ inline int max_slot(long long L) { return (int)(((L % 5) + 5) % 5); }
@@ -210,14 +270,17 @@ __device__ __forceinline__ uint32_t ld_slot(const uint32_t* p) {
     return v;
 }
 
+// Slot of level g - back (0 <= back < 5) from s5 = slot of level g.
+__host__ __device__ inline int slot_back(int s5, int back) { return s5 >= back ? s5 - back : s5 - back + 5; }
+
 // Scales of levels g, g-1, g-2 from the slots of levels g-2..g-4. 1/s is
 // 2^-k exactly (what 1.0f / s gives for a power of two).
-__device__ __forceinline__ StepScales step_scales(const F16Dev& f, int b, long long g) {
+__device__ __forceinline__ StepScales step_scales(const F16Dev& f, int b, int s5) {
     const uint32_t* mx = f.mx + (size_t)b * 5;
     const float smax = __ldg(f.src_max + b);
-    const int kn = level_scale_exp(ld_slot(mx + max_slot(g - 2)), smax);
-    const int kc = level_scale_exp(ld_slot(mx + max_slot(g - 3)), smax);
-    const int ko = level_scale_exp(ld_slot(mx + max_slot(g - 4)), smax);
+    const int kn = level_scale_exp(ld_slot(mx + slot_back(s5, 2)), smax);
+    const int kc = level_scale_exp(ld_slot(mx + slot_back(s5, 3)), smax);
+    const int ko = level_scale_exp(ld_slot(mx + slot_back(s5, 4)), smax);
     StepScales s;
     s.s_new = pow2_exact(kn);
     s.s_cur = pow2_exact(kc);
@@ -335,6 +398,12 @@ __device__ __forceinline__ float lrs_neighbour_sum(unsigned mask, const float nb
 
 __constant__ uint8_t c_group_mask[26];
 
+__device__ __forceinline__ LrsMat lrs_mat(const LrsDev& L, int m) {
+    const float4* p = reinterpret_cast<const float4*>(L.mat + m);
+    const float4 u = __ldg(p), v = __ldg(p + 1);
+    return LrsMat{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+}
+
 // One boundary point update. Returns p^{n+1} of the cell and writes the
 // filter state of every face. `pint` is the interior (leapfrog) value of
 // the cell, kept by the corner group that the reference never updates
@@ -356,19 +425,17 @@ __device__ __forceinline__ float lrs_point(const LrsDev& L, int e, int b, uint32
     // ring width per filter: K, except REF corners (lrs_3.cl:70, size_a_0/2)
     const int size_f = (REF && nf == 3) ? K / 2 : K;
     const size_t n = (size_t)L.n;
+    auto at = [&](int slot) { return (size_t)(uint32_t)slot * (uint32_t)L.n; };  // one wide multiply
     float* sin_ = L.st_in + (size_t)b * L.S * n + e;
     float* sout = L.st_out + (size_t)b * L.S * n + e;
 
-    float a0[3], b0[3], gn[3];
+    float gn[3];
+    LrsMat M[3];
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
         gn[f] = 0.0f;
-        a0[f] = 1.0f;
-        b0[f] = 1.0f;
-        if (f < nf) {
-            a0[f] = __ldg(L.ca + mat[f] * K);
-            b0[f] = __ldg(L.cb + mat[f] * K);
-        }
+        M[f] = LrsMat{};
+        if (f < nf) M[f] = lrs_mat(L, mat[f]);
     }
     auto tap = [&](int i) {
 #pragma unroll
@@ -377,7 +444,7 @@ __device__ __forceinline__ float lrs_point(const LrsDev& L, int e, int b, uint32
                 const int slot = (ix_buf + i) % size_f + f * size_f;
                 const float bi = __ldg(L.cb + mat[f] * K + i);
                 const float ai = __ldg(L.ca + mat[f] * K + i);
-                gn[f] += bi * sin_[(size_t)slot * n] - ai * sout[(size_t)slot * n];
+                gn[f] += bi * sin_[at(slot)] - ai * sout[at(slot)];
             }
         }
     };
@@ -388,32 +455,34 @@ __device__ __forceinline__ float lrs_point(const LrsDev& L, int e, int b, uint32
         for (int i = 1; i < K; ++i) tap(i);
     }
 
-    const float l = L.l, l2 = L.l2;
+    const float l2 = L.l2;
     const float S = lrs_neighbour_sum(c_group_mask[group], nb);
+    float gb[3];  // gn / b0
+#pragma unroll
+    for (int f = 0; f < 3; ++f) gb[f] = f < nf ? div_shared(gn[f], M[f].b0, M[f].rb) : 0.0f;
     float pn;
     if (nf == 1) {
-        pn = (l2 * S + L.c2 * pc + l2 / b0[0] * gn[0] + (l * a0[0] / b0[0] - 1.0f) * pold) /
-             (1.0f + l * a0[0] / b0[0]);
+        pn = div_shared(l2 * S + L.c2 * pc + M[0].t1 * gn[0] + (M[0].ratio - 1.0f) * pold, 1.0f + M[0].ratio,
+                        M[0].rden);
     } else if (nf == 2 || REF) {
         if (REF && group == 25) {
             pn = pint;  // no variant define reaches lrs_3.cl for this group
         } else {
-            pn = (l2 * S + l2 * (gn[0] / b0[0] + gn[1] / b0[1]) + L.c2 * pc +
-                  (l * a0[0] / b0[0] + l * a0[1] / b0[1] - 1.0f) * pold) /
-                 (1.0f + l * a0[0] / b0[0] + l * a0[1] / b0[1]);
+            pn = (l2 * S + l2 * (gb[0] + gb[1]) + L.c2 * pc + (M[0].ratio + M[1].ratio - 1.0f) * pold) /
+                 (1.0f + M[0].ratio + M[1].ratio);
         }
     } else {
-        pn = (l2 * S + l2 * (gn[0] / b0[0] + gn[1] / b0[1] + gn[2] / b0[2]) + L.c2 * pc +
-              (l * a0[0] / b0[0] + l * a0[1] / b0[1] + l * a0[2] / b0[2] - 1.0f) * pold) /
-             (1.0f + l * a0[0] / b0[0] + l * a0[1] / b0[1] + l * a0[2] / b0[2]);
+        pn = (l2 * S + l2 * (gb[0] + gb[1] + gb[2]) + L.c2 * pc +
+              (M[0].ratio + M[1].ratio + M[2].ratio - 1.0f) * pold) /
+             (1.0f + M[0].ratio + M[1].ratio + M[2].ratio);
     }
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
         if (f < nf) {
-            const float xn = a0[f] / (l * b0[f]) * (pn - pold) - gn[f] / b0[f];
+            const float xn = M[f].t3 * (pn - pold) - gb[f];
             const int slot = ix_buf + f * size_f;
-            sin_[(size_t)slot * n] = xn;
-            sout[(size_t)slot * n] = 1.0f / a0[f] * (b0[f] * xn + gn[f]);
+            sin_[at(slot)] = xn;
+            sout[at(slot)] = M[f].t4 * (M[f].b0 * xn + gn[f]);
         }
     }
     return pn;
@@ -428,16 +497,17 @@ __device__ __forceinline__ float lrs_face(const LrsDev& L, int e, int b, int d, 
                                           float pc, float pold, int ix_buf) {
     const int K = KT > 0 ? KT : L.K;
     const size_t n = (size_t)L.n;
+    auto at = [&](int slot) { return (size_t)(uint32_t)slot * (uint32_t)L.n; };  // one wide multiply
     float* sin_ = L.st_in + (size_t)b * L.S * n + e;
     float* sout = L.st_out + (size_t)b * L.S * n + e;
     const float* ca = L.ca + mat * K;
     const float* cb = L.cb + mat * K;
-    const float a0 = __ldg(ca), b0 = __ldg(cb);
+    const LrsMat M = lrs_mat(L, mat);
     float gn = 0.0f;
     auto tap = [&](int i) {
         int s = ix_buf + i;
         if (s >= K) s -= K;
-        gn += __ldg(cb + i) * sin_[(size_t)s * n] - __ldg(ca + i) * sout[(size_t)s * n];
+        gn += __ldg(cb + i) * sin_[at(s)] - __ldg(ca + i) * sout[at(s)];
     };
     if constexpr (KT > 0) {
 #pragma unroll
@@ -465,11 +535,10 @@ __device__ __forceinline__ float lrs_face(const LrsDev& L, int e, int b, int d, 
         S = S + nb[3];
         S = S + 2.0f * nb[d == 4 ? 5 : 4];
     }
-    const float l = L.l, l2 = L.l2;
-    const float pn = (l2 * S + L.c2 * pc + l2 / b0 * gn + (l * a0 / b0 - 1.0f) * pold) / (1.0f + l * a0 / b0);
-    const float xn = a0 / (l * b0) * (pn - pold) - gn / b0;
-    sin_[(size_t)ix_buf * n] = xn;
-    sout[(size_t)ix_buf * n] = 1.0f / a0 * (b0 * xn + gn);
+    const float pn = div_shared(L.l2 * S + L.c2 * pc + M.t1 * gn + (M.ratio - 1.0f) * pold, 1.0f + M.ratio, M.rden);
+    const float xn = M.t3 * (pn - pold) - div_shared(gn, M.b0, M.rb);
+    sin_[at(ix_buf)] = xn;
+    sout[at(ix_buf)] = M.t4 * (M.b0 * xn + gn);
     return pn;
 }
 

@@ -20,6 +20,7 @@
 #include <functional>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "device.cuh"
@@ -77,12 +78,26 @@ __device__ __forceinline__ void watch(int* flag, float v) {
     if (!(fabsf(v) < 1e30f)) atomicOr(flag, 1);
 }
 
+// Receivers of one member from level g at `p` (mic.cl:32-41), threads t, t +
+// threads, ...; inv and sc: the level's inverse scale and scale.
+template <typename T>
+__device__ __forceinline__ void record_receivers(const StepArgs& a, int b, long long g, const T* p, float inv,
+                                                 float sc, int t, int threads) {
+    for (int r = t; r < a.rcv.n; r += threads) {
+        const float v = fld(p + __ldg(a.rcv.cell + r), inv);
+        a.rcv.out[((size_t)b * a.rcv.n + r) * a.rcv.cap + g] = v;
+        if constexpr (sizeof(T) == 4) watch(a.flag, v);
+        else if (!f16_finite(v * sc)) atomicOr(a.flag, 1);
+    }
+}
+
 // leapfrog.cl:34-55 over 1 <= x,y,z <= n-2 of every batch member. FP16
 // storage: the update on stored values and the largest |p^n| gathered per
 // warp, as in k_stream.
 template <typename T>
 __global__ void __launch_bounds__(256) k_interior(StepArgs a, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const TlMark tl(a, 0, g, blockIdx.z < (unsigned)(a.g.nz - 2));
     const int x = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int y = 1 + blockIdx.y * blockDim.y + threadIdx.y;
@@ -93,23 +108,23 @@ __global__ void __launch_bounds__(256) k_interior(StepArgs a, int j) {
     const int64_t i = (int64_t)z * a.g.plane + (int64_t)y * a.g.pitch + x;
     if constexpr (sizeof(T) == 4) {
         if (x > a.g.nx - 2 || y > a.g.ny - 2) return;
-        float* pn = a.p[buf_new(g)] + base;
-        const float* pc = a.p[buf_cur(g)] + base;
-        const float* po = a.p[buf_old(g)] + base;
+        float* pn = a.p[I.wn] + base;
+        const float* pc = a.p[I.wc] + base;
+        const float* po = a.p[I.wo] + base;
         const float v = slf_update(a.lambda2, a.cint, pc[i + 1], pc[i - 1], pc[i + a.g.pitch],
                                    pc[i - a.g.pitch], pc[i + a.g.plane], pc[i - a.g.plane], pc[i], po[i]);
         pn[i] = v;
         watch(a.flag, v);
     } else {
         if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0)
-            for (int m = 0; m < a.batch; ++m) a.f16.mx[(size_t)m * 5 + max_slot(g)] = 0u;
+            for (int m = 0; m < a.batch; ++m) a.f16.mx[(size_t)m * 5 + I.s5] = 0u;
         const bool in = x <= a.g.nx - 2 && y <= a.g.ny - 2;
-        const StepScales sc = step_scales(a.f16, b, g);
+        const StepScales sc = step_scales(a.f16, b, I.s5);
         uint32_t amax = 0;
         if (in) {
-            __half* pn = a.f16.h[buf_new(g)] + base;
-            const __half* pc = a.f16.h[buf_cur(g)] + base;
-            const __half* po = a.f16.h[buf_old(g)] + base;
+            __half* pn = a.f16.h[I.wn] + base;
+            const __half* pc = a.f16.h[I.wc] + base;
+            const __half* po = a.f16.h[I.wo] + base;
             const float v = slf_update_scaled(
                 a.lambda2, sc.s_new * sc.inv_cur, sc.s_new * sc.inv_old, __half2float(pc[i + 1]),
                 __half2float(pc[i - 1]), __half2float(pc[i + a.g.pitch]), __half2float(pc[i - a.g.pitch]),
@@ -121,7 +136,7 @@ __global__ void __launch_bounds__(256) k_interior(StepArgs a, int j) {
         }
         const uint32_t wmax = __reduce_max_sync(0xffffffffu, amax);
         if ((threadIdx.x & 31) == 0 && wmax)
-            atomicMax(a.f16.mx + (size_t)b * 5 + max_slot(g - 1),
+            atomicMax(a.f16.mx + (size_t)b * 5 + slot_back(I.s5, 1),
                       __float_as_uint(__half2float(__ushort_as_half((unsigned short)wmax)) * sc.inv_cur));
     }
 }
@@ -133,47 +148,150 @@ __global__ void __launch_bounds__(256) k_interior(StepArgs a, int j) {
 // Memory-latency-bound gathers: 5 blocks per SM (48 registers, no spills
 // for the FIXED variants) keep more loads in flight than 4.
 // One boundary point e of batch member b at global step g: reads p^n and
-// p^{n-1} around the cell, writes p^{n+1} of the cell and its filter state.
-template <bool REF, int KT, typename T>
-__device__ __forceinline__ void lrs_update(const StepArgs& a, int b, int e, long long g) {
+// p^{n-1} around the cell, returns p^{n+1} of the cell (unscaled) and writes
+// its filter state. `info`: the entry's packed info. NC: the levels are
+// constant for the launch (read-only cache); the resident kernel, whose
+// other blocks write them between its steps, reads them with plain loads.
+template <bool NC, typename T>
+__device__ __forceinline__ float lvl(const T* p, float inv) {
+    if constexpr (NC) return fldg(p, inv);
+    else return fld(p, inv);
+}
+
+template <bool REF, int KT, typename T, bool NC>
+__device__ __forceinline__ float lrs_value(const StepArgs& a, const StepIdx& I, int b, int e, int64_t c, uint32_t info,
+                                           float ic, float io) {
     const size_t base = (size_t)b * a.g.vol;
-    T* pn = level_ptr<T>(a, buf_new(g)) + base;
-    const T* pc = level_ptr<T>(a, buf_cur(g)) + base;
-    const T* po = level_ptr<T>(a, buf_old(g)) + base;
-    float s_new = 1.0f, ic = 1.0f, io = 1.0f;
-    if constexpr (sizeof(T) == 2) {
-        const StepScales sc = step_scales(a.f16, b, g);
-        s_new = sc.s_new;
-        ic = sc.inv_cur;
-        io = sc.inv_old;
-    }
-    const int64_t c = __ldg(a.lrs.cell + e);
-    const uint32_t info = __ldg(a.lrs.info + e);
-    const float nb[6] = {fldg(pc + c + 1, ic), fldg(pc + c - 1, ic), fldg(pc + c + a.g.pitch, ic),
-                         fldg(pc + c - a.g.pitch, ic), fldg(pc + c + a.g.plane, ic), fldg(pc + c - a.g.plane, ic)};
+    const T* pc = level_ptr<T>(a, I.wc) + base;
+    const T* po = level_ptr<T>(a, I.wo) + base;
+    const float nb[6] = {lvl<NC>(pc + c + 1, ic),           lvl<NC>(pc + c - 1, ic),
+                         lvl<NC>(pc + c + a.g.pitch, ic),   lvl<NC>(pc + c - a.g.pitch, ic),
+                         lvl<NC>(pc + c + a.g.plane, ic),   lvl<NC>(pc + c - a.g.plane, ic)};
+    const float vc = lvl<NC>(pc + c, ic), vo = lvl<NC>(po + c, io);
     const int grp = (int)(info & 31u);
-    const int ix_buf = ring_index(g, a.lrs.K);
-    float v;
-    if (grp < 6) {
-        v = lrs_face<KT>(a.lrs, e, b, grp, (int)((info >> 5) & 255u), nb, fldg(pc + c, ic), fldg(po + c, io),
-                         ix_buf);
-    } else {
-        const float pint = (REF && grp == 25) ? fld(pn + c, 1.0f) : 0.0f;
-        v = lrs_point<REF, KT>(a.lrs, e, b, info, nb, fldg(pc + c, ic), fldg(po + c, io), pint, ix_buf);
-    }
-    fst(pn + c, v, s_new);
+    if (grp < 6) return lrs_face<KT>(a.lrs, e, b, grp, (int)((info >> 5) & 255u), nb, vc, vo, I.ix);
+    // the corner the reference leaves at its interior value (REF, group 25)
+    const float pint = (REF && grp == 25)
+                           ? slf_update(a.lambda2, a.cint, nb[0], nb[1], nb[2], nb[3], nb[4], nb[5], vc, vo)
+                           : 0.0f;
+    return lrs_point<REF, KT>(a.lrs, e, b, info, nb, vc, vo, pint, I.ix);
+}
+
+// The FP16 scales a boundary or PML update of member b uses (1 for FP32).
+struct LevelScales {
+    float s_new = 1.0f, i_new = 1.0f, ic = 1.0f, io = 1.0f;
+};
+template <typename T>
+__device__ __forceinline__ LevelScales level_scales(const StepArgs& a, int b, int s5) {
+    LevelScales r;
     if constexpr (sizeof(T) == 2) {
-        if (!f16_finite(v * s_new)) atomicOr(a.flag, 1);
+        const StepScales sc = step_scales(a.f16, b, s5);
+        r.s_new = sc.s_new;
+        r.i_new = sc.inv_new;
+        r.ic = sc.inv_cur;
+        r.io = sc.inv_old;
     }
+    return r;
+}
+
+// The same with the new value stored. Entries of source cells (kSrcEntry)
+// are left to src_rcv_role when `skip_src` is set.
+template <bool REF, int KT, typename T, bool NC = true>
+__device__ __forceinline__ void lrs_update(const StepArgs& a, const StepIdx& I, int b, int e, int64_t c,
+                                           uint32_t info, bool skip_src = false) {
+    if (skip_src && (info & kSrcEntry)) return;
+    const LevelScales sc = level_scales<T>(a, b, I.s5);
+    const float v = lrs_value<REF, KT, T, NC>(a, I, b, e, c, info, sc.ic, sc.io);
+    fst(level_ptr<T>(a, I.wn) + (size_t)b * a.g.vol + c, v, sc.s_new);
+    if constexpr (sizeof(T) == 2) {
+        if (!f16_finite(v * sc.s_new)) atomicOr(a.flag, 1);
+    }
+}
+
+// Source cells and receivers of one batch member inside the step's own
+// kernels (StepArgs::sr): thread t of `threads` takes source cells t, t +
+// threads, ...: the cell's update of this step (boundary entry, interior
+// value, or the untouched value of an outer face) followed by its sources in
+// insertion order (source.cl:32-40), each rounded to the storage type as a
+// store and load would. Receivers (mic.cl:32-41) are recorded one step late,
+// from p^n = the finished level g - 1, which no kernel of the step writes;
+// record = false at the first step of a chunk (the step before it was recorded
+// at that chunk's end). Not inlined: it would raise the register need of the
+// boundary kernel.
+template <bool REF, typename T, bool NC>
+__device__ __noinline__ void src_rcv_role(const StepArgs& a, const StepIdx I, int b, int t, int threads, bool record) {
+    const size_t base = (size_t)b * a.g.vol;
+    const long long g = I.g;
+    const LevelScales sc = level_scales<T>(a, b, I.s5);
+    const T* pc = level_ptr<T>(a, I.wc) + base;
+    const T* po = level_ptr<T>(a, I.wo) + base;
+    for (int k = t; k < a.sr.n; k += threads) {
+        const int64_t c = __ldg(a.sr.cell + k);
+        const int e = __ldg(a.sr.entry + k);
+        const int q0 = __ldg(a.sr.begin + k), q1 = __ldg(a.sr.begin + k + 1);
+        T* pn = level_ptr<T>(a, I.wn) + base + c;
+        float v;  // FP16: the stored value
+        if (e >= 0) {
+            v = lrs_value<REF, 0, T, NC>(a, I, b, e, c, __ldg(a.lrs.info + e), sc.ic, sc.io);
+            if constexpr (sizeof(T) == 2) {
+                if (!f16_finite(v * sc.s_new)) atomicOr(a.flag, 1);
+            }
+        } else if (e == kSrcInterior) {
+            const int64_t pitch = a.g.pitch, plane = a.g.plane;
+            if constexpr (sizeof(T) == 4) {
+                v = slf_update(a.lambda2, a.cint, pc[c + 1], pc[c - 1], pc[c + pitch], pc[c - pitch], pc[c + plane],
+                               pc[c - plane], pc[c], po[c]);
+            } else {
+                v = slf_update_scaled(
+                        a.lambda2, sc.s_new * sc.ic, sc.s_new * sc.io, __half2float(pc[c + 1]),
+                        __half2float(pc[c - 1]), __half2float(pc[c + pitch]), __half2float(pc[c - pitch]),
+                        __half2float(pc[c + plane]), __half2float(pc[c - plane]), __half2float(pc[c]),
+                        __half2float(po[c])) * sc.i_new;
+            }
+        } else {
+            v = fld(pn, sc.i_new);
+        }
+        auto stored = [&](float u) {  // what a store and load of u give
+            if constexpr (sizeof(T) == 4) return u;
+            else return __half2float(__float2half_rn(u * sc.s_new)) * sc.i_new;
+        };
+        v = stored(v);
+        for (int q = q0; q < q1; ++q) {
+            if (__ldg(a.sr.member + q) != b) continue;
+            v = stored(v + (g < __ldg(a.sr.len + q) ? a.src.data[__ldg(a.sr.off + q) + g] : 0.0f));
+        }
+        fst(pn, v, sc.s_new);
+    }
+    if (record) record_receivers<T>(a, b, g - 1, pc, sc.ic, 1.0f / sc.ic, t, threads);
 }
 
 template <bool REF, int KT, typename T>
 __global__ void __launch_bounds__(256, 5) k_lrs(const __grid_constant__ StepArgs a, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const TlMark tl(a, 1, g, blockIdx.y == 0);
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    // the first block column takes the sources and receivers: a chain of
+    // dependent loads that the other blocks hide (as the last one it added 9 us
+    // to the 512x384x320 step)
+    if (a.sr.on && blockIdx.x == 0) {
+        const TlMark tl6(a, 6, g, blockIdx.y == 0);
+        src_rcv_role<REF, T, true>(a, I, (int)blockIdx.y, (int)threadIdx.x, 256, j > 0);
+        return;
+    }
+    const int e = (blockIdx.x - (a.sr.on ? 1 : 0)) * blockDim.x + threadIdx.x;
     if (e >= a.lrs.n) return;
-    lrs_update<REF, KT, T>(a, (int)blockIdx.y, e, g);
+    lrs_update<REF, KT, T>(a, I, (int)blockIdx.y, e, __ldg(a.lrs.cell + e), __ldg(a.lrs.info + e), a.sr.on != 0);
+}
+
+// The receivers of the last step of a chunk whose steps ran with sr.on.
+template <typename T>
+__global__ void k_rcv_last(const __grid_constant__ StepArgs a, int j) {
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
+    float inv = 1.0f;
+    if constexpr (sizeof(T) == 2) inv = step_scales(a.f16, (int)blockIdx.x, I.s5).inv_new;
+    record_receivers<T>(a, (int)blockIdx.x, g, level_ptr<T>(a, I.wn) + (size_t)blockIdx.x * a.g.vol, inv,
+                        1.0f / inv, (int)threadIdx.x, (int)blockDim.x);
 }
 
 template <bool REF, typename T>
@@ -289,14 +407,11 @@ __device__ __forceinline__ void pml_aux(const StepArgs& a, unsigned axes, const 
     }
 }
 
-__device__ __forceinline__ int pml_level(const StepArgs& a, long long g) {
-    return (int)((g - a.pml.g0 + 1) & 1);
-}
-
 // REF pass 1: auxiliary fields of every cell 2..n-3, using the cell's own
 // new pressure and psi recomputed locally (nothing written that is read).
 __global__ void __launch_bounds__(256) k_pml_ref_aux(StepArgs a, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const TlMark tl(a, 3, g, blockIdx.z < (unsigned)(a.g.nz - 4));
     const int x = 2 + blockIdx.x * blockDim.x + threadIdx.x;
     const int y = 2 + blockIdx.y * blockDim.y + threadIdx.y;
@@ -311,10 +426,10 @@ __global__ void __launch_bounds__(256) k_pml_ref_aux(StepArgs a, int j) {
     if (z < W || z > a.g.nz - W - 1) axes |= 4u;
     if (!axes) return;
     const size_t base = (size_t)b * a.g.vol;
-    const float* pn = a.p[buf_new(g)] + base;
-    const float* pc = a.p[buf_cur(g)] + base;
-    const float* po = a.p[buf_old(g)] + base;
-    const int lv = pml_level(a, g);
+    const float* pn = a.p[I.wn] + base;
+    const float* pc = a.p[I.wc] + base;
+    const float* po = a.p[I.wo] + base;
+    const int lv = I.lv;
     const float* fx1 = a.pml.fi[0][lv ^ 1] + base;
     const float* fy1 = a.pml.fi[1][lv ^ 1] + base;
     const float* fz1 = a.pml.fi[2][lv ^ 1] + base;
@@ -329,7 +444,8 @@ __global__ void __launch_bounds__(256) k_pml_ref_aux(StepArgs a, int j) {
 
 // REF pass 2: pressure and psi of every cell 2..n-3 (pml.cl:182-207).
 __global__ void __launch_bounds__(256) k_pml_ref_p(StepArgs a, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const TlMark tl(a, 2, g, blockIdx.z < (unsigned)(a.g.nz - 4));
     const int x = 2 + blockIdx.x * blockDim.x + threadIdx.x;
     const int y = 2 + blockIdx.y * blockDim.y + threadIdx.y;
@@ -338,10 +454,10 @@ __global__ void __launch_bounds__(256) k_pml_ref_p(StepArgs a, int j) {
     const int z = 2 + blockIdx.z % zn;
     if (x > a.g.nx - 3 || y > a.g.ny - 3) return;
     const size_t base = (size_t)b * a.g.vol;
-    float* pn = a.p[buf_new(g)] + base;
-    const float* pc = a.p[buf_cur(g)] + base;
-    const float* po = a.p[buf_old(g)] + base;
-    const int lv = pml_level(a, g);
+    float* pn = a.p[I.wn] + base;
+    const float* pc = a.p[I.wc] + base;
+    const float* po = a.p[I.wo] + base;
+    const int lv = I.lv;
     const int64_t i = (int64_t)z * a.g.plane + (int64_t)y * a.g.pitch + x;
     float psi_new;
     const float v = pml_pressure(a, pc, po, a.pml.fi[0][lv ^ 1] + base, a.pml.fi[1][lv ^ 1] + base,
@@ -433,224 +549,241 @@ __device__ __forceinline__ void store4t(T* p, const float v[4], unsigned m, floa
     }
 }
 
+// Pressure of one PML cell (pml.cl:185-207): c, o = p^n, p^{n-1}, s6 the sum of
+// the six neighbours, d the divergence of the auxiliary fields, ks = (kx + ky +
+// kz) / (2 dt), ps and pmh the new and old psi; quot(a, b) = a / b.
+template <typename Q>
+__device__ __forceinline__ float pml_p_cell(const PmlDev& P, float s6, float c, float o, float kx, float ky, float kz,
+                                            float ks, float d, float ps, float pmh, Q quot) {
+    const float A = P.cc_dxdx * (s6 - 6.0f * c);
+    const float B = P.inv_dx * d;
+    const float C = kx * ky * kz * 0.5f * (ps + pmh);
+    const float D = P.inv_dt2 * (o - 2.0f * c);
+    const float E = (kx * ky + ky * kz + kz * kx) * c;
+    const float F = ks * o;
+    return quot(A + B - C - D - E + F, P.inv_dt2 + ks);
+}
+
+// Auxiliary field of one PML cell (pml.cl:231-262 with the derivative and ksi
+// index corrected): f1 its previous value, k the damping average along its
+// axis, k1 and k2 along the others in axis order, dp and dpsi the derivatives.
+template <typename Q>
+__device__ __forceinline__ float pml_aux_cell(const PmlDev& P, float f1, float k, float k1, float k2, float dp,
+                                              float dpsi, Q quot) {
+    return quot(-0.5f * k * f1 + (k1 + k2 - k) * dp + (k1 * k2) * dpsi + P.inv_dt * f1, P.inv_dt + k * 0.5f);
+}
+
+// The face average of four values in the order of pml.cl:74-122: x-faces take
+// (y, z), (y, z+1), (y+1, z), (y+1, z+1); y-faces (x, z), (x, z+1), (x+1, z),
+// (x+1, z+1); z-faces (x, y), (x, y+1), (x+1, y), (x+1, y+1).
+__device__ __forceinline__ float face4(float v0, float v1, float v2, float v3) {
+    return 0.25f * (((v0 + v1) + v2) + v3);
+}
+
+// Adds axis AX's term of the divergence of the auxiliary fields to d[0..3],
+// from the rows r00 (y, z), r01 (y, z+1), r10 (y+1, z), r11 (y+1, z+1), cells
+// x..x+4 (pml.cl:189-195; axes in x, y, z order).
+template <int AX>
+__device__ __forceinline__ void pml_div(const float r00[5], const float r01[5], const float r10[5],
+                                        const float r11[5], float d[4]) {
+    if constexpr (AX == 0) {
+        float av[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) av[q] = face4(r00[q], r01[q], r10[q], r11[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[q] = av[q + 1] - av[q];
+    } else {
+        // y: rows of y+1 against rows of y; z: rows of z+1 against rows of z
+        const float* u0 = AX == 1 ? r10 : r01;
+        const float* l1 = AX == 1 ? r01 : r10;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            d[q] = d[q] + face4(u0[q], r11[q], u0[q + 1], r11[q + 1]);
+            d[q] = d[q] - face4(r00[q], l1[q], r00[q + 1], l1[q + 1]);
+        }
+    }
+}
+
+// Difference of the face averages along AX of the rows as in pml_div.
+template <int AX>
+__device__ __forceinline__ void face_ends(const float r00[5], const float r01[5], const float r10[5],
+                                          const float r11[5], int q, float* hi, float* lo) {
+    if constexpr (AX == 0) {
+        *hi = face4(r00[q + 1], r01[q + 1], r10[q + 1], r11[q + 1]);
+        *lo = face4(r00[q], r01[q], r10[q], r11[q]);
+    } else if constexpr (AX == 1) {
+        *hi = face4(r10[q], r11[q], r10[q + 1], r11[q + 1]);
+        *lo = face4(r00[q], r01[q], r00[q + 1], r01[q + 1]);
+    } else {
+        *hi = face4(r01[q], r11[q], r01[q + 1], r11[q + 1]);
+        *lo = face4(r00[q], r10[q], r00[q + 1], r10[q + 1]);
+    }
+}
+
+// Values x..x+4 of a row; NC as in lvl.
+template <bool NC, typename T>
+__device__ __forceinline__ void row5n(const T* p, float r[5], float inv, bool fifth) {
+    if constexpr (NC) {
+        row5t(p, r, inv, fifth);
+    } else if constexpr (sizeof(T) == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        r[0] = v.x;
+        r[1] = v.y;
+        r[2] = v.z;
+        r[3] = v.w;
+        r[4] = fifth ? p[4] : 0.0f;
+    } else {
+        const uint2 w = *reinterpret_cast<const uint2*>(p);
+        const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
+        const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+        r[0] = lo.x * inv;
+        r[1] = lo.y * inv;
+        r[2] = hi.x * inv;
+        r[3] = hi.y * inv;
+        r[4] = fifth ? __half2float(p[4]) * inv : 0.0f;
+    }
+}
+
 // Pressure of the PML cells (pml.cl:185-207 restricted to the slab cells)
 // of one 4-cell unit x..x+3 of row (y, z). Fields outside the read axes are
 // identically zero there and are not loaded; PSI: psi is kept (PML faces on
-// all three axes). s_new, ic, io: FP16 scales of the new level and inverse
-// scales of p^n and p^{n-1} (1 for FP32 storage).
-template <bool PSI, typename T>
-__device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int y, int z, long long g,
-                                           float s_new, float ic, float io) {
-    // The mask gates only the stores and the flag: the loads below issue
-    // without waiting for it (every unit of a box lies in planes and rows
-    // 2..n-3, so x-1 .. x+4, y+-1 and z+-1 stay inside the level and field
-    // arrays even for a unit with no PML cell, whose results are dropped).
+// all three axes). sc: the member's FP16 scales (1 for FP32 storage).
+template <bool PSI, typename T, bool NC = true>
+__device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int y, int z, const StepIdx& I,
+                                           const LevelScales& sc) {
+    // The mask gates only the stores, the flag and the numerators: the loads
+    // below issue without waiting for it (every unit of a box lies in planes
+    // and rows 2..n-3, so x-1 .. x+4, y+-1 and z+-1 stay inside the level and
+    // field arrays even for a unit with no PML cell, whose results are dropped).
     const unsigned m = pml_mask4(a, x, y, z);
     const PmlDev& P = a.pml;
     const size_t base = (size_t)b * a.g.vol;
-    const int64_t pitch = a.g.pitch, plane = a.g.plane;
-    const int64_t i = (int64_t)z * plane + (int64_t)y * pitch + x;
-    const T* pc = level_ptr<T>(a, buf_cur(g)) + base;
-    const T* po = level_ptr<T>(a, buf_old(g)) + base;
-    T* pn = level_ptr<T>(a, buf_new(g)) + base;
-    const int lv = pml_level(a, g);
+    const int pitch = (int)a.g.pitch, plane = (int)a.g.plane;
+    const int i = z * plane + y * pitch + x;  // a member has fewer than 2^31 cells
+    const T* pc = level_ptr<T>(a, I.wc) + base;
+    const T* po = level_ptr<T>(a, I.wo) + base;
+    const float ic = sc.ic;
     // x+4 is read only where it lies in the row (the unit's last cell can be
     // a PML cell only then)
-    const bool hi = x + 4 < a.g.pitch;
+    const bool hi = x + 4 < pitch;
     float c[5], ym4[5], yp4[5], zm4[5], zp4[5], o[5];
-    row5t(pc + i, c, ic, hi);
-    const float xm = x >= 1 ? fldg(pc + i - 1, ic) : 0.0f;
-    row5t(pc + i - pitch, ym4, ic, false);
-    row5t(pc + i + pitch, yp4, ic, false);
-    row5t(pc + i - plane, zm4, ic, false);
-    row5t(pc + i + plane, zp4, ic, false);
-    row5t(po + i, o, io, false);
+    row5n<NC>(pc + i, c, ic, hi);
+    const float xm = x >= 1 ? lvl<NC>(pc + i - 1, ic) : 0.0f;
+    row5n<NC>(pc + (i - pitch), ym4, ic, false);
+    row5n<NC>(pc + (i + pitch), yp4, ic, false);
+    row5n<NC>(pc + (i - plane), zm4, ic, false);
+    row5n<NC>(pc + (i + plane), zp4, ic, false);
+    row5n<NC>(po + i, o, sc.io, false);
     const float4 kx4 = __ldg(reinterpret_cast<const float4*>(P.ksi[0] + x));
-    const float kxv[4] = {kx4.x, kx4.y, kx4.z, kx4.w};
+    const float kx[4] = {kx4.x, kx4.y, kx4.z, kx4.w};
     const float ky = __ldg(P.ksi[1] + y), kz = __ldg(P.ksi[2] + z);
     const unsigned ra = slab_axes(a, x, x + 4, y, y + 1, z, z + 1);
     float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (ra & 1u) {
-        const float* f = P.fi[0][lv ^ 1] + base + i;
-        float r00[5], r01[5], r10[5], r11[5], av[5];
-        row5(f, r00, hi);
-        row5(f + plane, r01, hi);
-        row5(f + pitch, r10, hi);
-        row5(f + pitch + plane, r11, hi);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) av[q] = 0.25f * (((r00[q] + r01[q]) + r10[q]) + r11[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) d[q] = av[q + 1] - av[q];
-    }
-    if (ra & 2u) {
-        const float* f = P.fi[1][lv ^ 1] + base + i;
+    auto field = [&](int ax, auto add) {
+        const float* f = P.fi[ax][I.lv ^ 1] + base;
         float r00[5], r01[5], r10[5], r11[5];
-        row5(f, r00, hi);
-        row5(f + plane, r01, hi);
-        row5(f + pitch, r10, hi);
-        row5(f + pitch + plane, r11, hi);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float a1 = 0.25f * (((r10[q] + r11[q]) + r10[q + 1]) + r11[q + 1]);
-            const float a0 = 0.25f * (((r00[q] + r01[q]) + r00[q + 1]) + r01[q + 1]);
-            d[q] = d[q] + a1;
-            d[q] = d[q] - a0;
-        }
-    }
-    if (ra & 4u) {
-        const float* f = P.fi[2][lv ^ 1] + base + i;
-        float r00[5], r01[5], r10[5], r11[5];
-        row5(f, r00, hi);
-        row5(f + plane, r01, hi);
-        row5(f + pitch, r10, hi);
-        row5(f + pitch + plane, r11, hi);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float a1 = 0.25f * (((r01[q] + r11[q]) + r01[q + 1]) + r11[q + 1]);
-            const float a0 = 0.25f * (((r00[q] + r10[q]) + r00[q + 1]) + r10[q + 1]);
-            d[q] = d[q] + a1;
-            d[q] = d[q] - a0;
-        }
-    }
+        row5n<NC>(f + i, r00, 1.0f, hi);
+        row5n<NC>(f + (i + plane), r01, 1.0f, hi);
+        row5n<NC>(f + (i + pitch), r10, 1.0f, hi);
+        row5n<NC>(f + (i + pitch + plane), r11, 1.0f, hi);
+        add(r00, r01, r10, r11);
+    };
+    if (ra & 1u) field(0, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<0>(q, r, s, t, d); });
+    if (ra & 2u) field(1, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<1>(q, r, s, t, d); });
+    if (ra & 4u) field(2, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<2>(q, r, s, t, d); });
     float ps[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pmh[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (PSI) {
-        const float4 h = *reinterpret_cast<const float4*>(P.psi[lv ^ 1] + base + i);
+        const float4 h = *reinterpret_cast<const float4*>(P.psi[I.lv ^ 1] + base + i);
         pmh[0] = h.x;
         pmh[1] = h.y;
         pmh[2] = h.z;
         pmh[3] = h.w;
 #pragma unroll
         for (int q = 0; q < 4; ++q) ps[q] = P.dt * c[q] + pmh[q];
-        store4(P.psi[lv] + base + i, ps, m);
+        store4(P.psi[I.lv] + base + i, ps, m);
     }
-    float v[4];
     // ks depends on kx only within the row: one division when the four agree
-    float ksq[4];
-    if (kxv[0] == kxv[1] && kxv[1] == kxv[2] && kxv[2] == kxv[3]) {
-        const float k0 = (kxv[0] + ky + kz) / P.two_dt;
-        ksq[0] = ksq[1] = ksq[2] = ksq[3] = k0;
+    float v[4], ks[4];
+    if (kx[0] == kx[1] && kx[1] == kx[2] && kx[2] == kx[3]) {
+        ks[0] = ks[1] = ks[2] = ks[3] = (kx[0] + ky + kz) / P.two_dt;
     } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) ksq[q] = (kxv[q] + ky + kz) / P.two_dt;
+        for (int q = 0; q < 4; ++q) ks[q] = (kx[q] + ky + kz) / P.two_dt;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const float xmq = q == 0 ? xm : c[q - 1];
-        float s6 = c[q + 1] + xmq;
+        float s6 = c[q + 1] + (q == 0 ? xm : c[q - 1]);
         s6 = s6 + yp4[q];
         s6 = s6 + ym4[q];
         s6 = s6 + zp4[q];
         s6 = s6 + zm4[q];
-        const float kx = kxv[q];
-        const float ks = ksq[q];
-        const float A = P.cc_dxdx * (s6 - 6.0f * c[q]);
-        const float B = P.inv_dx * d[q];
-        const float C = kx * ky * kz * 0.5f * (ps[q] + pmh[q]);
-        const float D = P.inv_dt2 * (o[q] - 2.0f * c[q]);
-        const float E = (kx * ky + ky * kz + kz * kx) * c[q];
-        const float F = ks * o[q];
-        const float num = A + B - C - D - E + F;
-        v[q] = num / (P.inv_dt2 + ks);
+        v[q] = pml_p_cell(P, s6, c[q], o[q], kx[q], ky, kz, ks[q], d[q], ps[q], pmh[q],
+                          [](float n, float den) { return n / den; });
         if constexpr (sizeof(T) == 4) {
             if ((m >> q) & 1u) watch(a.flag, v[q]);
         } else {
-            if (((m >> q) & 1u) && !f16_finite(v[q] * s_new)) atomicOr(a.flag, 1);
+            if (((m >> q) & 1u) && !f16_finite(v[q] * sc.s_new)) atomicOr(a.flag, 1);
         }
     }
-    store4t(pn + i, v, m, s_new);
+    store4t(level_ptr<T>(a, I.wn) + base + i, v, m, sc.s_new);
 }
 
-// Auxiliary field AX of the PML cells of one 4-cell unit (pml.cl:231-262
-// with the derivative and ksi index corrected). The derivatives of the new
-// and previous pressure along every axis come from the same four rows
-// (y, y+1) x (z, z+1), x..x+4. in_, ic: FP16 inverse scales of the new
-// level and of p^n (1 for FP32 storage).
-template <int AX, bool PSI, typename T>
-__device__ __forceinline__ void pml_aux_unit(const StepArgs& a, int b, int x, int y, int z, long long g,
-                                             float in_, float ic) {
+// Auxiliary field AX of the PML cells of one 4-cell unit. The derivatives of
+// the new and previous pressure along every axis come from the same four rows
+// (y, y+1) x (z, z+1), x..x+4.
+template <int AX, bool PSI, typename T, bool NC = true>
+__device__ __forceinline__ void pml_aux_unit(const StepArgs& a, int b, int x, int y, int z, const StepIdx& I,
+                                             const LevelScales& sc) {
     // loads issue without waiting for the mask, as in pml_p_unit
     const unsigned m = pml_mask4(a, x, y, z);
     const PmlDev& P = a.pml;
     const size_t base = (size_t)b * a.g.vol;
-    const int64_t pitch = a.g.pitch, plane = a.g.plane;
-    const int64_t i = (int64_t)z * plane + (int64_t)y * pitch + x;
-    const T* pn = level_ptr<T>(a, buf_new(g)) + base + i;
-    const T* pc = level_ptr<T>(a, buf_cur(g)) + base + i;
-    const int lv = pml_level(a, g);
-    const bool hi = x + 4 < a.g.pitch;  // x+4 is read only where it lies in the row
+    const int pitch = (int)a.g.pitch, plane = (int)a.g.plane;
+    const int i = z * plane + y * pitch + x;
+    const T* pn = level_ptr<T>(a, I.wn) + base;
+    const T* pc = level_ptr<T>(a, I.wc) + base;
+    const bool hi = x + 4 < pitch;  // x+4 is read only where it lies in the row
     float n00[5], n01[5], n10[5], n11[5], m00[5], m01[5], m10[5], m11[5];
-    row5t(pn, n00, in_, hi);
-    row5t(pn + plane, n01, in_, hi);
-    row5t(pn + pitch, n10, in_, hi);
-    row5t(pn + pitch + plane, n11, in_, hi);
-    row5t(pc, m00, ic, hi);
-    row5t(pc + plane, m01, ic, hi);
-    row5t(pc + pitch, m10, ic, hi);
-    row5t(pc + pitch + plane, m11, ic, hi);
+    row5n<NC>(pn + i, n00, sc.i_new, hi);
+    row5n<NC>(pn + (i + plane), n01, sc.i_new, hi);
+    row5n<NC>(pn + (i + pitch), n10, sc.i_new, hi);
+    row5n<NC>(pn + (i + pitch + plane), n11, sc.i_new, hi);
+    row5n<NC>(pc + i, m00, sc.ic, hi);
+    row5n<NC>(pc + (i + plane), m01, sc.ic, hi);
+    row5n<NC>(pc + (i + pitch), m10, sc.ic, hi);
+    row5n<NC>(pc + (i + pitch + plane), m11, sc.ic, hi);
     float s00[5] = {0}, s01[5] = {0}, s10[5] = {0}, s11[5] = {0};
     if (PSI) {
-        const float* ps = P.psi[lv] + base + i;
-        row5(ps, s00, hi);
-        row5(ps + plane, s01, hi);
-        row5(ps + pitch, s10, hi);
-        row5(ps + pitch + plane, s11, hi);
+        const float* ps = P.psi[I.lv] + base;
+        row5n<NC>(ps + i, s00, 1.0f, hi);
+        row5n<NC>(ps + (i + plane), s01, 1.0f, hi);
+        row5n<NC>(ps + (i + pitch), s10, 1.0f, hi);
+        row5n<NC>(ps + (i + pitch + plane), s11, 1.0f, hi);
     }
     float kxs[5];
     row5(P.ksi[0] + x, kxs, hi);
     const float kay = 0.5f * (__ldg(P.ksi[1] + y) + __ldg(P.ksi[1] + y + 1));
     const float kaz = 0.5f * (__ldg(P.ksi[2] + z) + __ldg(P.ksi[2] + z + 1));
-    const float4 f14 = *reinterpret_cast<const float4*>(P.fi[AX][lv ^ 1] + base + i);
+    const float4 f14 = *reinterpret_cast<const float4*>(P.fi[AX][I.lv ^ 1] + base + i);
     const float f1v[4] = {f14.x, f14.y, f14.z, f14.w};
     float out[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const float kax = 0.5f * (kxs[q] + kxs[q + 1]);
-        const float f1 = f1v[q];
-        if (AX == 0) {
-            const float an1 = 0.25f * (((n00[q + 1] + n01[q + 1]) + n10[q + 1]) + n11[q + 1]);
-            const float an0 = 0.25f * (((n00[q] + n01[q]) + n10[q]) + n11[q]);
-            const float am1 = 0.25f * (((m00[q + 1] + m01[q + 1]) + m10[q + 1]) + m11[q + 1]);
-            const float am0 = 0.25f * (((m00[q] + m01[q]) + m10[q]) + m11[q]);
-            const float dxp = P.half_inv_dx * (an1 - an0 + am1 - am0);
-            float dxpsi = 0.0f;
-            if (PSI) {
-                const float as1 = 0.25f * (((s00[q + 1] + s01[q + 1]) + s10[q + 1]) + s11[q + 1]);
-                const float as0 = 0.25f * (((s00[q] + s01[q]) + s10[q]) + s11[q]);
-                dxpsi = P.inv_dx * (as1 - as0);
-            }
-            out[q] = (-0.5f * kax * f1 + (kay + kaz - kax) * dxp + (kay * kaz) * dxpsi + P.inv_dt * f1) /
-                     (P.inv_dt + kax * 0.5f);
-        } else if (AX == 1) {
-            const float an1 = 0.25f * (((n10[q] + n11[q]) + n10[q + 1]) + n11[q + 1]);
-            const float an0 = 0.25f * (((n00[q] + n01[q]) + n00[q + 1]) + n01[q + 1]);
-            const float am1 = 0.25f * (((m10[q] + m11[q]) + m10[q + 1]) + m11[q + 1]);
-            const float am0 = 0.25f * (((m00[q] + m01[q]) + m00[q + 1]) + m01[q + 1]);
-            const float dyp = P.half_inv_dx * (an1 - an0 + am1 - am0);
-            float dypsi = 0.0f;
-            if (PSI) {
-                const float as1 = 0.25f * (((s10[q] + s11[q]) + s10[q + 1]) + s11[q + 1]);
-                const float as0 = 0.25f * (((s00[q] + s01[q]) + s00[q + 1]) + s01[q + 1]);
-                dypsi = P.inv_dx * (as1 - as0);
-            }
-            out[q] = (-0.5f * kay * f1 + (kax + kaz - kay) * dyp + (kax * kaz) * dypsi + P.inv_dt * f1) /
-                     (P.inv_dt + kay * 0.5f);
-        } else {
-            const float an1 = 0.25f * (((n01[q] + n11[q]) + n01[q + 1]) + n11[q + 1]);
-            const float an0 = 0.25f * (((n00[q] + n10[q]) + n00[q + 1]) + n10[q + 1]);
-            const float am1 = 0.25f * (((m01[q] + m11[q]) + m01[q + 1]) + m11[q + 1]);
-            const float am0 = 0.25f * (((m00[q] + m10[q]) + m00[q + 1]) + m10[q + 1]);
-            const float dzp = P.half_inv_dx * (an1 - an0 + am1 - am0);
-            float dzpsi = 0.0f;
-            if (PSI) {
-                const float as1 = 0.25f * (((s01[q] + s11[q]) + s01[q + 1]) + s11[q + 1]);
-                const float as0 = 0.25f * (((s00[q] + s10[q]) + s00[q + 1]) + s10[q + 1]);
-                dzpsi = P.inv_dx * (as1 - as0);
-            }
-            out[q] = (-0.5f * kaz * f1 + (kax + kay - kaz) * dzp + (kax * kay) * dzpsi + P.inv_dt * f1) /
-                     (P.inv_dt + kaz * 0.5f);
+        float nh, nl, mh, ml;
+        face_ends<AX>(n00, n01, n10, n11, q, &nh, &nl);
+        face_ends<AX>(m00, m01, m10, m11, q, &mh, &ml);
+        const float dp = P.half_inv_dx * (nh - nl + mh - ml);
+        float dpsi = 0.0f;
+        if (PSI) {
+            float sh, sl;
+            face_ends<AX>(s00, s01, s10, s11, q, &sh, &sl);
+            dpsi = P.inv_dx * (sh - sl);
         }
+        out[q] = pml_aux_cell(P, f1v[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), AX == 0 ? kay : kax,
+                              AX == 2 ? kay : kaz, dp, dpsi, [](float n, float den) { return n / den; });
     }
-    store4(P.fi[AX][lv] + base + i, out, m);
+    store4(P.fi[AX][I.lv] + base + i, out, m);
 }
 
 // One launch over several PML boxes: a flat grid whose blocks are dealt to
@@ -700,19 +833,14 @@ __device__ __forceinline__ BoxThread box_thread(const BoxLaunch& L) {
 template <bool PSI, typename T>
 __global__ void __launch_bounds__(256, 3) k_pml_p_all(const __grid_constant__ StepArgs a,
                                                       const __grid_constant__ BoxLaunch L, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const BoxThread t = box_thread(L);
     const TlMark tl(a, 2, g, t.b == 0);
     if (!t.ok) return;
-    float s_new = 1.0f, ic = 1.0f, io = 1.0f;
-    if constexpr (sizeof(T) == 2) {
-        const StepScales sc = step_scales(a.f16, t.b, g);
-        s_new = sc.s_new;
-        ic = sc.inv_cur;
-        io = sc.inv_old;
-    }
+    const LevelScales sc = level_scales<T>(a, t.b, I.s5);
 #pragma unroll 1
-    for (int z = t.z0; z < t.z1; ++z) pml_p_unit<PSI, T>(a, t.b, t.x, t.y, z, g, s_new, ic, io);
+    for (int z = t.z0; z < t.z1; ++z) pml_p_unit<PSI, T>(a, t.b, t.x, t.y, z, I, sc);
 }
 
 // The auxiliary fields of every (axis, slab box) pair in one launch: the
@@ -721,28 +849,26 @@ __global__ void __launch_bounds__(256, 3) k_pml_p_all(const __grid_constant__ St
 template <bool PSI, typename T>
 __global__ void __launch_bounds__(256, 3) k_pml_aux_all(const __grid_constant__ StepArgs a,
                                                         const __grid_constant__ BoxLaunch L, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const BoxThread t = box_thread(L);
     const int ax = L.axis[t.k];
     const TlMark tl(a, 3 + ax, g, t.b == 0);
     if (!t.ok) return;
-    float in_ = 1.0f, ic = 1.0f;
-    if constexpr (sizeof(T) == 2) {
-        const StepScales sc = step_scales(a.f16, t.b, g);
-        in_ = sc.inv_new;
-        ic = sc.inv_cur;
-    }
+    const LevelScales sc = level_scales<T>(a, t.b, I.s5);
     if (ax == 0) {
 #pragma unroll 1
-        for (int z = t.z0; z < t.z1; ++z) pml_aux_unit<0, PSI, T>(a, t.b, t.x, t.y, z, g, in_, ic);
+        for (int z = t.z0; z < t.z1; ++z) pml_aux_unit<0, PSI, T>(a, t.b, t.x, t.y, z, I, sc);
     } else if (ax == 1) {
 #pragma unroll 1
-        for (int z = t.z0; z < t.z1; ++z) pml_aux_unit<1, PSI, T>(a, t.b, t.x, t.y, z, g, in_, ic);
+        for (int z = t.z0; z < t.z1; ++z) pml_aux_unit<1, PSI, T>(a, t.b, t.x, t.y, z, I, sc);
     } else {
 #pragma unroll 1
-        for (int z = t.z0; z < t.z1; ++z) pml_aux_unit<2, PSI, T>(a, t.b, t.x, t.y, z, g, in_, ic);
+        for (int z = t.z0; z < t.z1; ++z) pml_aux_unit<2, PSI, T>(a, t.b, t.x, t.y, z, I, sc);
     }
 }
+
+#include "roles.cuh"
 
 // Eight binary16 values (one 16-byte word) as FP32 numbers.
 __device__ __forceinline__ void cvt8(const uint4 w, float v[8]) {
@@ -769,7 +895,7 @@ __device__ __forceinline__ void cvt8(const uint4 w, float v[8]) {
 // cells; the order of the work items does not change any result.
 constexpr int kTailWarps = 4;
 
-__device__ __forceinline__ void stream_tail(const StepArgs& a, const FusedDev& f, int j, long long g) {
+__device__ __forceinline__ void stream_tail(const StepArgs& a, const FusedDev& f, int j, const StepIdx& I) {
     const int lane = threadIdx.x & 31;
     const long long B = a.batch;
     const long long n_lrs = (long long)a.lrs.n * B;
@@ -785,12 +911,14 @@ __device__ __forceinline__ void stream_tail(const StepArgs& a, const FusedDev& f
         const long long u = (long long)base + lane;
         if (u < n_lrs) {
             const int b = (int)(u / a.lrs.n), e = (int)(u - (long long)b * a.lrs.n);
+            const int64_t c = __ldg(a.lrs.cell + e);
+            const uint32_t info = __ldg(a.lrs.info + e);
             switch (K) {
-                case 1: lrs_update<false, 1, float>(a, b, e, g); break;
-                case 2: lrs_update<false, 2, float>(a, b, e, g); break;
-                case 3: lrs_update<false, 3, float>(a, b, e, g); break;
-                case 4: lrs_update<false, 4, float>(a, b, e, g); break;
-                default: lrs_update<false, 0, float>(a, b, e, g); break;
+                case 1: lrs_update<false, 1, float>(a, I, b, e, c, info); break;
+                case 2: lrs_update<false, 2, float>(a, I, b, e, c, info); break;
+                case 3: lrs_update<false, 3, float>(a, I, b, e, c, info); break;
+                case 4: lrs_update<false, 4, float>(a, I, b, e, c, info); break;
+                default: lrs_update<false, 0, float>(a, I, b, e, c, info); break;
             }
         } else if (u < total) {
             const PmlDev& P = a.pml;
@@ -804,8 +932,8 @@ __device__ __forceinline__ void stream_tail(const StepArgs& a, const FusedDev& f
             const int ux = (int)(r % bx.units);
             r /= bx.units;
             const int yy = (int)(r % bx.height), zz = (int)(r / bx.height);
-            if (psi) pml_p_unit<true, float>(a, b, bx.x0 + 4 * ux, bx.y0 + yy, bx.z0 + zz, g, 1.0f, 1.0f, 1.0f);
-            else pml_p_unit<false, float>(a, b, bx.x0 + 4 * ux, bx.y0 + yy, bx.z0 + zz, g, 1.0f, 1.0f, 1.0f);
+            if (psi) pml_p_unit<true, float>(a, b, bx.x0 + 4 * ux, bx.y0 + yy, bx.z0 + zz, I, LevelScales());
+            else pml_p_unit<false, float>(a, b, bx.x0 + 4 * ux, bx.y0 + yy, bx.z0 + zz, I, LevelScales());
         }
     }
 }
@@ -814,7 +942,8 @@ template <typename T, int S, bool TAIL = false>
 __global__ void __launch_bounds__(TAIL ? F_THREADS + 32 * kTailWarps : F_THREADS, 2)
     k_stream(const __grid_constant__ CUtensorMap tm_halo, const __grid_constant__ CUtensorMap tm_own,
              const __grid_constant__ StepArgs a, const __grid_constant__ FusedDev f, int j) {
-    const TlMark tl(a, 0, *a.d_step + j, true);
+    const StepIdx I = step_at(a, j);
+    const TlMark tl(a, 0, I.g, true);
     using TL = Tile<T, S>;
     constexpr int F_STAGES = TL::STAGES;
     extern __shared__ unsigned char smem_raw[];
@@ -831,13 +960,12 @@ __global__ void __launch_bounds__(TAIL ? F_THREADS + 32 * kTailWarps : F_THREADS
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    const long long g = *a.d_step + j;
     const int B = a.batch, nz = a.g.nz;
     const int n_items = f.items ? f.n_items : f.tiles_x * f.tiles_y * f.n_chunks * B;
-    const int wn = buf_new(g), wc = buf_cur(g), wo = buf_old(g);
+    const int wn = I.wn, wc = I.wc, wo = I.wo;
     if constexpr (TAIL && sizeof(T) == 4) {
         if (tid >= F_THREADS) {
-            stream_tail(a, f, j, g);
+            stream_tail(a, f, j, I);
             return;
         }
     }
@@ -849,7 +977,7 @@ __global__ void __launch_bounds__(TAIL ? F_THREADS + 32 * kTailWarps : F_THREADS
             if constexpr (sizeof(T) == 2) {
                 // level g's maximum is gathered by the next step
                 if (blockIdx.x == 0)
-                    for (int b = 0; b < B; ++b) a.f16.mx[(size_t)b * 5 + max_slot(g)] = 0u;
+                    for (int b = 0; b < B; ++b) a.f16.mx[(size_t)b * 5 + I.s5] = 0u;
             }
             uint32_t k = 0;
             bool ok = true;
@@ -975,7 +1103,7 @@ __global__ void __launch_bounds__(TAIL ? F_THREADS + 32 * kTailWarps : F_THREADS
             // only z+1, y+-1 and p^{n-1}. The update runs on stored values
             // of level g-1 (scale s_cur) and is rescaled once at the end.
             if (it.b != sc_b) {
-                const StepScales sc = step_scales(a.f16, it.b, g);
+                const StepScales sc = step_scales(a.f16, it.b, I.s5);
                 sc_rc = sc.s_new * sc.inv_cur;
                 sc_ro = sc.s_cur * sc.inv_old;
                 sc_ic = sc.inv_cur;
@@ -1089,7 +1217,7 @@ __global__ void __launch_bounds__(TAIL ? F_THREADS + 32 * kTailWarps : F_THREADS
             const uint32_t gmax = __reduce_max_sync(0xffffffffu, max(amax & 0xffffu, amax >> 16));
             if (lane == 0 && gmax) {
                 const float mv = __half2float(__ushort_as_half((unsigned short)gmax)) * sc_ic;
-                atomicMax(a.f16.mx + (size_t)it.b * 5 + max_slot(g - 1), __float_as_uint(mv));
+                atomicMax(a.f16.mx + (size_t)it.b * 5 + slot_back(I.s5, 1), __float_as_uint(mv));
             }
             // a stored binary16 infinity or NaN (magnitude bits >= 0x7c00)
             // in a grid-interior cell means the field left the range
@@ -1158,11 +1286,11 @@ static void launch_stream(int S, bool tail, int grid, cudaStream_t st, const CUt
 
 // Scale and inverse scale of level g for member b (1 for FP32 storage).
 template <typename T>
-__device__ __forceinline__ float2 new_level_scale(const StepArgs& a, int b, long long g) {
+__device__ __forceinline__ float2 new_level_scale(const StepArgs& a, int b, int s5) {
     if constexpr (sizeof(T) == 4) {
         return make_float2(1.0f, 1.0f);
     } else {
-        const int k = level_scale_exp(ld_slot(a.f16.mx + (size_t)b * 5 + max_slot(g - 2)), __ldg(a.f16.src_max + b));
+        const int k = level_scale_exp(ld_slot(a.f16.mx + (size_t)b * 5 + slot_back(s5, 2)), __ldg(a.f16.src_max + b));
         return make_float2(pow2_exact(k), pow2_exact(-k));
     }
 }
@@ -1171,11 +1299,12 @@ __device__ __forceinline__ float2 new_level_scale(const StepArgs& a, int b, long
 // Sources landing on one cell are added in insertion order.
 template <typename T>
 __global__ void k_src_rcv(StepArgs a, int j, int do_src, int do_rcv) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const TlMark tl(a, 6, g, blockIdx.x == 0);
     const int b = blockIdx.x;
-    T* pn = level_ptr<T>(a, buf_new(g)) + (size_t)b * a.g.vol;
-    const float2 sc = new_level_scale<T>(a, b, g);
+    T* pn = level_ptr<T>(a, I.wn) + (size_t)b * a.g.vol;
+    const float2 sc = new_level_scale<T>(a, b, I.s5);
     if (do_src && threadIdx.x == 0) {
         for (int s = a.src.begin[b]; s < a.src.begin[b + 1]; ++s) {
             const float v = (g < a.src.len[s]) ? a.src.data[a.src.off[s] + g] : 0.0f;
@@ -1208,11 +1337,12 @@ struct SrcRcvInline {
 template <typename T>
 __global__ void k_src_rcv_inline(const __grid_constant__ StepArgs a, const __grid_constant__ SrcRcvInline q,
                                  int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const TlMark tl(a, 6, g, blockIdx.x == 0);
     const int b = blockIdx.x;
-    T* pn = level_ptr<T>(a, buf_new(g)) + (size_t)b * a.g.vol;
-    const float2 sc = new_level_scale<T>(a, b, g);
+    T* pn = level_ptr<T>(a, I.wn) + (size_t)b * a.g.vol;
+    const float2 sc = new_level_scale<T>(a, b, I.s5);
     if (threadIdx.x == 0) {
         for (int s = 0; s < q.n_src; ++s) {
             if (q.src_batch[s] != b) continue;
@@ -1244,13 +1374,14 @@ struct CaptureDev {
 
 template <typename T>
 __global__ void k_capture(const __grid_constant__ StepArgs a, const CaptureDev c, int j) {
-    const long long g = *a.d_step + j;
+    const StepIdx I = step_at(a, j);
+    const long long g = I.g;
     const long long i = g - c.run0[0];
     if (i % c.every) return;
     const long long n = c.run0[1] + i / c.every;
     const int slot = (int)(n % c.max_frames);
-    const float2 sc = new_level_scale<T>(a, c.batch, g);
-    const T* p = level_ptr<T>(a, buf_new(g)) + (size_t)c.batch * a.g.vol;
+    const float2 sc = new_level_scale<T>(a, c.batch, I.s5);
+    const T* p = level_ptr<T>(a, I.wn) + (size_t)c.batch * a.g.vol;
     float* out = c.frames + (size_t)slot * c.rows * c.cols;
     const int total = c.rows * c.cols;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
@@ -1264,7 +1395,37 @@ __global__ void k_capture(const __grid_constant__ StepArgs a, const CaptureDev c
     if (blockIdx.x == 0 && threadIdx.x == 0) c.frame_step[slot] = g;
 }
 
-__global__ void k_advance(long long* d_step, int n) { *d_step += n; }
+// Advances the step counter by n and fills the table of the next chunk's
+// steps. One block of kChunkSteps threads.
+__global__ void k_advance(long long* d_step, int n, StepIdx* idx, int K, long long pml_g0) {
+    const long long g0 = *d_step + n, g = g0 + threadIdx.x;
+    __syncthreads();
+    if (threadIdx.x == 0) *d_step = g0;
+    idx[threadIdx.x] = StepIdx{g, buf_new(g), buf_cur(g), buf_old(g), ring_index(g, K), (int)((g - pml_g0 + 1) & 1),
+                               max_slot(g)};
+}
+
+// The boundary entries of the source cells: flags their packed info
+// (kSrcEntry) and fills `entry`; every other entry's flag is cleared.
+__global__ void k_mark_sources(const int32_t* __restrict__ cell, uint32_t* info, int n,
+                               const int32_t* __restrict__ src_cell, int n_src, int32_t* entry) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const int32_t c = cell[e];
+        uint32_t w = info[e] & ~kSrcEntry;
+        for (int k = 0; k < n_src; ++k)
+            if (__ldg(src_cell + k) == c) {
+                w |= kSrcEntry;
+                entry[k] = e;
+            }
+        info[e] = w;
+    }
+}
+
+// The cells of a mask of 1 bit per cell, set.
+__global__ void k_set_bits(const int32_t* __restrict__ cells, int n, uint32_t* bits) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) atomicOr(bits + (cells[k] >> 5), 1u << (cells[k] & 31));
+}
 
 // Solid cell of the model (cells outside the model or the grid are air).
 __device__ __forceinline__ bool cell_solid(const SolidBits& s, int x, int y, int z) {
@@ -1361,6 +1522,17 @@ struct Source {
     std::vector<float> sig;
 };
 
+// Source cells that the step's own kernels take (one block's table).
+constexpr int kMaxSrcCells = 256;
+// Cells (all members) up to which the resident kernel runs. Against replayed
+// launches it measured (us a step; FP32 without a PML, FP32 with six PML
+// faces, FP16 with two): 5.1 / 14.5 / 13.7 to 10.3 / 20.6 / 19.2 at 0.04 M
+// cells, 10.0 / 21.2 / 16.5 to 12.1 / 27.7 / 22.4 at 0.74 M, 15.0 / 28.7 / 19.4
+// to 15.3 / 43.5 / 28.2 at 1.85 M, 24.9 / 58.3 / 34.1 to 25.0 / 73.6 / 40.3 at
+// 5.0 M, and 42.2 / 79.8 / 45.7 to 33.8 / 90.8 / 48.2 at 8.2 M, where the
+// streaming kernel's TMA tiles beat the columns of plain loads.
+constexpr int64_t kResidentCells = 5 << 20;
+
 struct Engine::Impl {
     afd_params prm{};
     // geometry
@@ -1399,6 +1571,9 @@ struct Engine::Impl {
     DBuf<uint32_t> lrs_info;
     DBuf<float> lrs_in, lrs_out;
     DBuf<float> coef_a, coef_b;
+    DBuf<LrsMat> lrs_mat_dev;
+    // REF: simulation.hpp:368-369 passes lambda^2 as l (lrs_1.cl:58,78)
+    float lrs_l() const { return ref() ? lambda2() : prm.dt * prm.c / prm.dx; }
     DBuf<float> fi[3][2], psi[2];
     DBuf<float> ksi_dev[3];
     std::vector<PmlBox> pml_boxes;
@@ -1419,10 +1594,26 @@ struct Engine::Impl {
     DBuf<int64_t> src_off, src_len;
     DBuf<float> src_data;
     DBuf<int32_t> rcv_cell;
+    // sources and receivers taken by the step's kernels (SrcRcvDev)
+    DBuf<int32_t> sr_cell, sr_entry, sr_begin, sr_member;
+    DBuf<int64_t> sr_len, sr_off;
+    int32_t sr_n = 0;
+    bool sr_ok = false;  // the distinct source cells fit one block's table
+    DBuf<uint32_t> res_owned;
+    DBuf<ResidentGroup> res_groups;
+    DBuf<int32_t> res_order;
+    DBuf<unsigned int> res_bar;
+    ResidentDev res{};
+    int res_blocks = 0;
+    bool res_dirty = true;
     DBuf<float> rcv_out;
     int64_t rcv_cap = 0;
     int32_t rcv_n_dev = 0;
     DBuf<long long> d_step;
+    DBuf<StepIdx> step_table;  // [kChunkSteps]
+    void advance_table(int n) {
+        k_advance<<<1, kChunkSteps, 0, stream>>>(d_step.ptr, n, step_table.ptr, have_model ? model.ncoef : 1, pml_g0);
+    }
     // headless visualisation (afd_set_capture)
     int32_t cap_batch = 0, cap_axis = 1, cap_index = 0, cap_every = 0, cap_max = 0;
     bool cap_dirty = false;
@@ -1482,7 +1673,36 @@ struct Engine::Impl {
     int plan_id = 0;             // index of `plan` in tune_cands (graph cache key), 0 before tuning
     int64_t tune_gen = -1;       // model_gen the candidates were made for
     cudaEvent_t tev0 = nullptr, tev1 = nullptr;
-    bool tune_active() const { return use_fused() && prm.graphs && !prm.profile && !tuned; }
+    bool tune_active() const { return use_fused() && prm.graphs && !prm.profile && !tuned && !resident(); }
+    // The step's own kernels take the sources and receivers (src_rcv_role).
+    // Left out: launches without graphs, profile and slab runs (their order is
+    // per kernel), the forced beside and tail orders, REF with a PML, and
+    // sources where the auxiliary updates read the new pressure, which they
+    // must see before the injection.
+    bool sr_active() const {
+        if (!use_fused() || !prm.graphs || prm.profile || step_phase != 0 || slab_nz > 0 || !sr_ok) return false;
+        if (lists_beside() || tail_active()) return false;
+        return pml_width <= 0 || (!ref() && src_beside_aux);
+    }
+    bool pml_fixed() const { return !ref() && pml_width > 0 && pml_units > 0; }
+    // Grids whose levels stay in L2 run a whole chunk in the resident kernel,
+    // unless a plan is forced or a capture or timeline needs the step's own
+    // launches.
+    bool resident() const {
+        return sr_active() && !forced && cap_every <= 0 && tl_steps <= 0 && vol * prm.batch <= kResidentCells;
+    }
+    void build_resident();
+    template <typename T>
+    void launch_resident(int64_t n);
+    void upload_source_cells(const std::vector<int32_t>& cell, const std::vector<int64_t>& off,
+                             const std::vector<int64_t>& len, const std::vector<int32_t>& begin);
+    template <typename T>
+    void launch_pml_aux(int j, cudaStream_t st) {
+        if (args.pml.psi_on) k_pml_aux_all<true, T><<<pml_aux_blocks, 256, 0, st>>>(args, pml_aux_all, j);
+        else k_pml_aux_all<false, T><<<pml_aux_blocks, 256, 0, st>>>(args, pml_aux_all, j);
+        ++launches;
+    }
+    void launch_chunk_end(int64_t n);
     void apply_plan(int id) {
         plan = id == 0 ? Plan{0, 0, false, 0, false} : tune_cands[(size_t)id - 1];
         plan_id = id;
@@ -1495,7 +1715,7 @@ struct Engine::Impl {
     // gives the results of the serial order. Made once per model and grid
     // (the plan then restarts from the default).
     void ensure_candidates() {
-        if (use_fused() && tune_gen != model_gen) {
+        if (use_fused() && tune_gen != model_gen && !resident()) {
             make_candidates();
             apply_plan(forced ? 1 : 0);
         }
@@ -1667,7 +1887,10 @@ struct Engine::Impl {
     template <typename T>
     void launch_step_t(int j, bool profile);
     int64_t kernels_per_step() const;
-    void launch_step_count_only(int64_t n) { launches += kernels_per_step() * n + 1; }
+    void launch_step_count_only(int64_t n) {
+        launches += kernels_per_step() * n + 1;
+        if (args.sr.on && args.rcv.n > 0) ++launches;
+    }
     cudaGraphExec_t graph_for(int64_t n);
     void run_chunk(int64_t n);
     void setup_run(int64_t steps);
@@ -1735,8 +1958,26 @@ void Engine::Impl::init_device() {
     if (have_model) {
         coef_a.upload(model.a);
         coef_b.upload(model.b);
+        // the quotients of the boundary update per material, in its own
+        // operations (build_args passes the same l and l2)
+        const float l = lrs_l(), l2 = l * l;
+        std::vector<LrsMat> t((size_t)model.nmat);
+        for (int m = 0; m < model.nmat; ++m) {
+            const float a0 = model.a[(size_t)m * model.ncoef], b0 = model.b[(size_t)m * model.ncoef];
+            LrsMat& q = t[(size_t)m];
+            q.b0 = b0;
+            q.ratio = l * a0 / b0;
+            q.t1 = l2 / b0;
+            q.t3 = a0 / (l * b0);
+            q.t4 = 1.0f / a0;
+            q.rb = recip_of(b0);
+            q.rden = recip_of(1.0f + q.ratio);
+            q.pad = 0.0f;
+        }
+        lrs_mat_dev.upload(t);
     }
     maps_shape = -1;  // the tensor maps cover the new field buffers once build_fused encodes them
+    res_dirty = true;
     initialized = true;
     fused_dirty = true;
     owned_dirty = true;
@@ -1936,6 +2177,7 @@ void Engine::Impl::setup_pml() {
     pml_aux_all = BoxLaunch{};
     pml_p_blocks = pml_aux_blocks = 0;
     pml_units = 0;
+    res_dirty = true;
     n_pml_cells = 0;
     fused_dirty = true;
     pml_g0 = steps_done;
@@ -2078,8 +2320,192 @@ void Engine::Impl::upload_sources() {
     src_len.upload(len);
     if (data.empty()) data.push_back(0.0f);
     src_data.upload(data);
+    upload_source_cells(cell, off, len, begin);
     src_dirty = false;
     fused_dirty = true;
+}
+
+// The distinct source cells over all members with their sources in insertion
+// order, and the boundary entries that hold one.
+void Engine::Impl::upload_source_cells(const std::vector<int32_t>& cell, const std::vector<int64_t>& off,
+                                       const std::vector<int64_t>& len, const std::vector<int32_t>& begin) {
+    std::map<int32_t, std::vector<int>> at;  // cell -> sources, grouped by member, insertion order within one
+    for (size_t k = 0; k < cell.size(); ++k) at[cell[k]].push_back((int)k);
+    sr_ok = (int)at.size() <= kMaxSrcCells;
+    sr_n = sr_ok ? (int32_t)at.size() : 0;
+    std::vector<int32_t> c, e, b{0}, m;
+    std::vector<int64_t> l, o;
+    if (sr_ok)
+        for (const auto& kv : at) {
+            const int32_t x = (int32_t)(kv.first % pitch), y = (int32_t)(kv.first % plane / pitch),
+                          z = (int32_t)(kv.first / plane);
+            const bool inner = x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1;
+            c.push_back(kv.first);
+            e.push_back(inner ? kSrcInterior : kSrcOuter);
+            for (int k : kv.second) {
+                m.push_back((int32_t)(std::upper_bound(begin.begin(), begin.end(), k) - begin.begin()) - 1);
+                l.push_back(len[(size_t)k]);
+                o.push_back(off[(size_t)k]);
+            }
+            b.push_back((int32_t)m.size());
+        }
+    sr_cell.upload(c);
+    sr_entry.upload(e);
+    sr_begin.upload(b);
+    sr_member.upload(m);
+    sr_len.upload(l);
+    sr_off.upload(o);
+    if (lrs_info.n) {
+        k_mark_sources<<<(unsigned)std::min<size_t>((lrs_info.n + 255) / 256, 1184), 256, 0, stream>>>(
+            lrs_cell.ptr, lrs_info.ptr, (int)lrs_info.n, sr_cell.ptr, sr_n, sr_entry.ptr);
+        CK(cudaGetLastError());
+    }
+    res_dirty = true;
+}
+
+// The resident kernel's work: how the PML units, boundary entries and interior
+// columns of a step's first phase are dealt to its groups. Costs are per 256
+// of each, in units of one interior plane of 256 columns.
+void Engine::Impl::build_resident() {
+    const bool pml = pml_fixed();
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const int64_t all = (int64_t)sms * kResGroups - 1;  // one group keeps the sources and receivers
+    ResidentDev& R = res;
+    R = ResidentDev{};
+    R.nu = (nx - 2) / 4 + 1;
+    R.ncol = R.nu * (ny - 2);
+    const double c_plane = 1.0, c_item = 1.0, c_lrs = 3.0, c_pml = 4.0;
+    const int64_t lrs = (int64_t)lrs_cell.n * prm.batch, planes = nz - 2, units = pml ? pml_units * prm.batch : 0;
+    const double fixed = (lrs + 255) / 256 * c_lrs + (units + 255) / 256 * c_pml;
+    // columns of zc planes: about one item per thread of the remaining groups
+    const double cols = (double)R.ncol * prm.batch / 256.0;
+    int zc = 1;
+    while (zc < 16 && zc < planes &&
+           cols * ((planes + zc - 1) / zc) * (zc * c_plane + c_item) + fixed > all * (zc * c_plane + c_item))
+        ++zc;
+    R.zc = zc;
+    R.n_zc = (int32_t)((planes + zc - 1) / zc);
+    R.per_member = (int32_t)(((int64_t)R.ncol * R.n_zc + 31) / 32 * 32);
+    const int64_t items = (int64_t)R.per_member * prm.batch;
+    int64_t aux = 0;
+    for (int ax = 0; ax < 3 && pml; ++ax)
+        for (const PmlBox& bx : pml_axis_boxes[ax]) aux += (int64_t)bx.units * bx.height * bx.depth;
+    const int64_t top = (int64_t)1 << 31;
+    if (items >= top || lrs >= top || units >= top || aux * prm.batch >= top) throw Error(AFD_ERR_ARG, "grid too large");
+    R.by_nu.set((uint32_t)R.nu);
+    R.by_ncol.set((uint32_t)R.ncol);
+    R.by_member.set((uint32_t)R.per_member);
+    R.by_lrs.set((uint32_t)std::max<size_t>(lrs_cell.n, 1));
+    // PML boxes, units in x-y-z order within a box, members outermost
+    auto boxes = [](ResidentBoxes* B, const std::vector<std::pair<PmlBox, int>>& v) {
+        uint32_t first = 0;
+        for (const auto& e : v) {
+            ResidentBox& q = B->box[B->n++];
+            q.x0 = e.first.x0;
+            q.y0 = e.first.y0;
+            q.z0 = e.first.z0;
+            q.axis = e.second;
+            q.first = first;
+            q.by_units.set((uint32_t)e.first.units);
+            q.by_rows.set((uint32_t)e.first.height);
+            first += (uint32_t)((int64_t)e.first.units * e.first.height * e.first.depth);
+        }
+        B->total = first;
+        B->by_total.set(std::max<uint32_t>(first, 1));
+    };
+    if (pml) {
+        std::vector<std::pair<PmlBox, int>> pe, ae;
+        for (const PmlBox& bx : pml_boxes) pe.emplace_back(bx, 0);
+        for (int ax = 0; ax < 3; ++ax)
+            for (const PmlBox& bx : pml_axis_boxes[ax]) ae.emplace_back(bx, ax);
+        boxes(&R.press, pe);
+        boxes(&R.aux, ae);
+    }
+    const double item_cost = (zc * c_plane + c_item) / 256.0;
+    const double total = fixed + items * item_cost;
+    // a group's budget: an even share, but at least one pass over 256 items
+    const double budget = std::max(total / all * 1.02, item_cost * 256.0);
+    std::vector<ResidentGroup> g;
+    int64_t p = 0, l = 0, i = 0;
+    double left = 0.0;
+    while (p < units || l < lrs || i < items) {
+        ResidentGroup q{};
+        left += budget;  // what rounding left to the group before counts too
+        const bool last = (int64_t)g.size() + 1 == all;
+        // the next n of `rest`, in whole warps, that fit what is left of the budget
+        auto take = [&](int64_t& at, int64_t end, double cost, int32_t* b, int32_t* e) {
+            *b = (int32_t)at;
+            if (at < end && (last || left > 0.0)) {
+                const int64_t n = last ? end - at : std::min(end - at, (int64_t)std::ceil(left / cost * 8) * 32);
+                at += n;
+                left -= n / 256.0 * cost;
+            }
+            *e = (int32_t)at;
+        };
+        take(p, units, c_pml, &q.p0, &q.p1);
+        take(l, lrs, c_lrs, &q.l0, &q.l1);
+        take(i, items, item_cost * 256.0, &q.i0, &q.i1);
+        g.push_back(q);
+    }
+    // the second phase spreads its units over as many groups as are there
+    const int64_t need = std::max<int64_t>((int64_t)g.size(), std::min<int64_t>(all, (aux * prm.batch + 255) / 256));
+    res_blocks = (int)((need + 1 + kResGroups - 1) / kResGroups);
+    // group k of the list: block k mod blocks, so that heavy roles spread over the SMs
+    std::vector<ResidentGroup> placed((size_t)res_blocks * kResGroups, ResidentGroup{});
+    for (size_t k = 0; k < g.size(); ++k) placed[(k % res_blocks) * kResGroups + k / res_blocks] = g[k];
+    res_groups.upload(placed);
+    if (res_order.n != boundary.size()) {
+        std::vector<int32_t> order(boundary.size());
+        int64_t at[kNumGroups + 1] = {0};
+        for (const BoundaryPoint& q : boundary) ++at[q.group + 1];
+        for (int k = 0; k < kNumGroups; ++k) at[k + 1] += at[k];
+        for (size_t e = 0; e < boundary.size(); ++e) order[(size_t)at[boundary[e].group]++] = (int32_t)e;
+        res_order.upload(order);
+    }
+    if (!res_bar.ptr) res_bar.alloc(1);
+    // cells the interior role leaves to the others
+    const size_t words = (size_t)nz * ny * (pitch / 32);
+    res_owned.alloc(words, false);
+    or_masks_device(!ref() && pml_owned.n == words ? pml_owned.ptr : nullptr, lrs_bits.ptr, res_owned.ptr,
+                    (int64_t)words, stream);
+    if (sr_n) k_set_bits<<<(sr_n + 255) / 256, 256, 0, stream>>>(sr_cell.ptr, sr_n, res_owned.ptr);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(stream));
+    R.groups = res_groups.ptr;
+    R.order = res_order.ptr;
+    R.owned = res_owned.ptr;
+    R.bar = res_bar.ptr;
+    res_dirty = false;
+}
+
+template <typename T>
+void Engine::Impl::launch_resident(int64_t n) {
+    ResidentDev R = res;
+    R.steps = (int32_t)n;
+    const void* kern = nullptr;
+    if (pml_fixed())
+        kern = args.pml.psi_on ? (const void*)k_resident<false, 2, T> : (const void*)k_resident<false, 1, T>;
+    else if (ref())
+        kern = (const void*)k_resident<true, 0, float>;
+    else
+        kern = (const void*)k_resident<false, 0, T>;
+    CK(cudaMemsetAsync(res_bar.ptr, 0, sizeof(unsigned int), stream));
+    void* params[] = {&args, &R};
+    CK(cudaLaunchCooperativeKernel(kern, dim3((unsigned)res_blocks), dim3(kResGroups * kGroup), params, 0, stream));
+    ++launches;
+}
+
+// After the last step of a chunk whose steps ran with args.sr.on: the
+// receivers of that step.
+void Engine::Impl::launch_chunk_end(int64_t n) {
+    if (!args.sr.on) return;
+    const int j = (int)n - 1;
+    if (args.rcv.n > 0) {
+        if (f16()) k_rcv_last<__half><<<(unsigned)prm.batch, 256, 0, stream>>>(args, j);
+        else k_rcv_last<float><<<(unsigned)prm.batch, 256, 0, stream>>>(args, j);
+        ++launches;
+    }
 }
 
 // CheckVariables (simulation.hpp:436-447): the receiver record grows to the
@@ -2141,7 +2567,7 @@ void Engine::Impl::build_args() {
     } else {
         for (int k = 0; k < 3; ++k) a.p[k] = fields.ptr + (size_t)k * vol * prm.batch;
     }
-    a.d_step = d_step.ptr;
+    a.idx = step_table.ptr;
     a.lambda2 = lambda2();
     a.cint = 2.0f * (1.0f - 3.0f * a.lambda2);
     a.lrs.n = (int32_t)lrs_cell.n;
@@ -2153,8 +2579,8 @@ void Engine::Impl::build_args() {
     a.lrs.st_out = lrs_out.ptr;
     a.lrs.ca = coef_a.ptr;
     a.lrs.cb = coef_b.ptr;
-    // REF: simulation.hpp:368-369 passes lambda^2 as l (lrs_1.cl:58,78)
-    a.lrs.l = ref() ? a.lambda2 : prm.dt * prm.c / prm.dx;
+    a.lrs.mat = lrs_mat_dev.ptr;
+    a.lrs.l = lrs_l();
     a.lrs.l2 = a.lrs.l * a.lrs.l;
     a.lrs.c2 = 2.0f * (1.0f - 3.0f * a.lrs.l2);
     PmlDev& P = a.pml;
@@ -2190,6 +2616,13 @@ void Engine::Impl::build_args() {
     a.src.off = src_off.ptr;
     a.src.len = src_len.ptr;
     a.src.data = src_data.ptr;
+    a.sr.n = sr_n;
+    a.sr.cell = sr_cell.ptr;
+    a.sr.entry = sr_entry.ptr;
+    a.sr.begin = sr_begin.ptr;
+    a.sr.member = sr_member.ptr;
+    a.sr.len = sr_len.ptr;
+    a.sr.off = sr_off.ptr;
     a.rcv.n = rcv_n_dev;
     a.rcv.cell = rcv_cell.ptr;
     a.rcv.out = rcv_out.ptr;
@@ -2275,8 +2708,9 @@ void Engine::Impl::launch_step_t(int j, bool profile) {
             ++launches;
         }
     }
+    const bool sr = a.sr.on != 0;
     auto lrs_launch = [&](cudaStream_t st) {
-        const dim3 grd((unsigned)((a.lrs.n + 255) / 256), (unsigned)prm.batch);
+        const dim3 grd((unsigned)((a.lrs.n + 255) / 256) + (sr ? 1u : 0u), (unsigned)prm.batch);
         if constexpr (sizeof(T) == 4) {
             if (ref()) launch_lrs<true, float>(a, j, grd, st);
             else launch_lrs<false, float>(a, j, grd, st);
@@ -2292,11 +2726,7 @@ void Engine::Impl::launch_step_t(int j, bool profile) {
         else k_pml_p_all<false, T><<<pml_p_blocks, 256, 0, st>>>(a, pml_p_all, j);
         ++launches;
     };
-    auto pml_aux_launch = [&](cudaStream_t st) {
-        if (psi) k_pml_aux_all<true, T><<<pml_aux_blocks, 256, 0, st>>>(a, pml_aux_all, j);
-        else k_pml_aux_all<false, T><<<pml_aux_blocks, 256, 0, st>>>(a, pml_aux_all, j);
-        ++launches;
-    };
+    auto pml_aux_launch = [&](cudaStream_t st) { launch_pml_aux<T>(j, st); };
     bool src_done = false;  // the source/receiver kernel already queued beside the auxiliary updates
     auto src_rcv_launch = [&](cudaStream_t st) {
         if (inline_ok) k_src_rcv_inline<T><<<(unsigned)prm.batch, 256, 0, st>>>(a, inl, j);
@@ -2304,7 +2734,17 @@ void Engine::Impl::launch_step_t(int j, bool profile) {
         ++launches;
     };
     const bool fixed_pml = !ref() && a.pml.width > 0 && a.pml.n_units > 0;
-    if (beside) {
+    if (sr) {
+        // The boundary kernel takes the sources and receivers along. FIXED PML:
+        // the pressure boxes run beside it (disjoint cells, finished levels
+        // only); the auxiliary updates follow.
+        std::vector<std::function<void(cudaStream_t)>> w;
+        if (a.lrs.n > 0 || a.sr.n > 0 || a.rcv.n > 0) w.push_back(lrs_launch);
+        if (fixed_pml) w.push_back(pml_p_launch);
+        run_side_by_side(w);
+        if (fixed_pml) pml_aux_launch(stream);
+        src_done = true;
+    } else if (beside) {
         // FIXED scheme in graphs: the streaming kernel skips the cells of
         // the boundary and PML kernels, which run beside it (they read only
         // levels n and n-1, filter state and the old auxiliary fields); the
@@ -2384,11 +2824,13 @@ cudaGraphExec_t Engine::Impl::graph_for(int64_t n) {
     if (it != graphs.end()) return it->second;
     cudaGraph_t graph;
     const int64_t saved = launches;
+    args.sr.on = sr_active() ? 1 : 0;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     if (use_fused()) CK(cudaMemsetAsync(f_work.ptr, 0, (size_t)n * sizeof(int), stream));
     if (tail_active()) CK(cudaMemsetAsync(f_tail.ptr, 0, (size_t)n * sizeof(unsigned long long), stream));
     for (int64_t j = 0; j < n; ++j) launch_step((int)j, false);
-    k_advance<<<1, 1, 0, stream>>>(d_step.ptr, (int)n);
+    launch_chunk_end(n);
+    advance_table((int)n);
     CK(cudaStreamEndCapture(stream, &graph));
     launches = saved;
     cudaGraphExec_t exec;
@@ -2400,7 +2842,14 @@ cudaGraphExec_t Engine::Impl::graph_for(int64_t n) {
 
 void Engine::Impl::run_chunk(int64_t n) {
     const bool profile = prm.profile != 0;
-    if (prm.graphs && !profile) {
+    args.sr.on = sr_active() ? 1 : 0;
+    if (resident()) {
+        if (f16()) launch_resident<__half>(n);
+        else launch_resident<float>(n);
+        launch_chunk_end(n);
+        advance_table((int)n);
+        ++launches;
+    } else if (prm.graphs && !profile) {
         cudaGraphExec_t g = graph_for(n);
         CK(cudaGraphLaunch(g, stream));
         // the graph holds n steps of kernels plus the step-counter advance
@@ -2409,7 +2858,7 @@ void Engine::Impl::run_chunk(int64_t n) {
         if (use_fused()) CK(cudaMemsetAsync(f_work.ptr, 0, (size_t)n * sizeof(int), stream));
         if (tail_active()) CK(cudaMemsetAsync(f_tail.ptr, 0, (size_t)n * sizeof(unsigned long long), stream));
         for (int64_t j = 0; j < n; ++j) launch_step((int)j, profile);
-        k_advance<<<1, 1, 0, stream>>>(d_step.ptr, (int)n);
+        advance_table((int)n);
         ++launches;
     }
     CK(cudaGetLastError());
@@ -2432,6 +2881,8 @@ int64_t Engine::Impl::kernels_per_step() const {
     const StepArgs& a = args;
     int64_t k = 1;
     const bool tail = tail_active();
+    if (a.sr.on)
+        return 1 + (a.lrs.n > 0 || a.sr.n > 0 || a.rcv.n > 0 ? 1 : 0) + (pml_fixed() ? 2 : 0) + (cap_every > 0 ? 1 : 0);
     if (a.lrs.n > 0 && !tail) ++k;
     if (a.pml.width > 0) {
         if (ref()) k += (nx > 4 && ny > 4 && nz > 4) ? 2 : 0;
@@ -2467,6 +2918,7 @@ Engine::Engine(const afd_params& p) : d_(new Impl) {
     CK(cudaEventCreate(&D.ev0));
     CK(cudaEventCreate(&D.ev1));
     D.d_step.alloc(1);
+    D.step_table.alloc(kChunkSteps);
     D.d_flag.alloc(1);
     D.d_energy.alloc(1);
     CK(cudaMemcpyToSymbol(c_group_mask, kGroupMask, sizeof(kGroupMask)));
@@ -2546,7 +2998,7 @@ void Engine::step(int32_t phase) {
     }
     D.step_phase = 0;
     if (phase == 2) {
-        k_advance<<<1, 1, 0, D.stream>>>(D.d_step.ptr, 1);
+        D.advance_table(1);
         ++D.launches;
     }
     CK(cudaGetLastError());
@@ -2838,6 +3290,8 @@ void Engine::Impl::setup_run(int64_t steps) {
         CK(cudaStreamSynchronize(stream));
     }
     build_args();
+    advance_table(0);  // the table follows the filter length and the PML's first step
+    if (res_dirty && resident()) build_resident();
 }
 
 // Chunks of a run: step 0 alone, then up to 200 steps (the progress
@@ -2858,7 +3312,7 @@ static std::vector<int64_t> run_chunks(int64_t steps) {
 void Engine::prepare(int64_t steps) {
     Impl& D = *d_;
     D.setup_run(steps);
-    if (!D.prm.graphs || D.prm.profile) return;
+    if (!D.prm.graphs || D.prm.profile || D.resident()) return;
     D.ensure_candidates();
     std::vector<int64_t> lens = run_chunks(steps);
     std::sort(lens.begin(), lens.end());
@@ -3204,7 +3658,8 @@ void Engine::get_info(afd_info* info) {
     info->stream_beside = D.lists_beside() ? 1 : 0;
     info->stream_per_sm = D.stream_per_sm;
     info->stream_tail = D.tail_active() ? 1 : 0;
-    info->tuned = D.tuned ? 1 : 0;
+    // a grid that runs in the resident kernel has nothing left to choose
+    info->tuned = D.tuned || (D.initialized && D.resident()) ? 1 : 0;
 }
 
 int Engine::kernel_stats(int32_t idx, char* name, int64_t cap, int64_t* launches, double* ms) {
