@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "device.cuh"
+#include "sync.cuh"
 
 namespace afd {
 
@@ -24,7 +25,6 @@ constexpr int FT_X = 64;                 // default tile width in x (cells, FP32
 constexpr int FT_Y = 16;                 // default tile height in y
 constexpr int F_CONSUMERS = 256;
 constexpr int F_THREADS = F_CONSUMERS + 32;
-constexpr unsigned long long kWaitLimitNs = 2000000000ull;   // 2 s
 
 // Tile shapes of the streaming kernel (a plan parameter the autotuner
 // varies): S = 0: 64 x 16, 1: 128 x 8, 2: 32 x 32 cells for FP32 storage;
@@ -101,11 +101,6 @@ __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
         : "r"(smem_addr(bar)), "r"(parity)
         : "memory");
     return done != 0;
-}
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
 }
 // Bounded wait: false after kWaitLimitNs without the phase completing.
 // The clock is read once per 16 polls, so waiting warps issue few

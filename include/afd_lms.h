@@ -7,7 +7,7 @@
  * identification.py:36,54): `epochs` passes of sample-serial LMS with step
  * size mu over the first min(nx, nd) samples, the delay line cleared at the
  * start of each pass and the weights kept, all in FP64. The GPU evaluates
- * the same recursion in blocks of 128 samples (exact up to the order of
+ * the same recursion in blocks of 512 samples (exact up to the order of
  * floating-point additions).
  */
 #ifndef AFD_LMS_H
