@@ -9,21 +9,22 @@
 // both orientations for the GEMMs; activations and their gradients in BF16.
 //
 // GEMM: C[M][N] = A[M][K] * B[N][K]^T, both operands K-major BF16, K in
-// steps of 64 through a ring of TMA stages. Warp 0 (one thread) streams
-// tiles, warp 1 allocates TMEM and one of its threads issues tcgen05.mma
-// (K = 16 per instruction) and commits stage releases, warps 2-5 read the
-// accumulator with tcgen05.ld and run the epilogue. Two forms:
-//   k_gemm_p  N a multiple of 256: persistent, one CTA per SM looping over
-//             128 x 256 output tiles, 4-stage ring of 48 KB, two 256-column
-//             TMEM accumulators so that the epilogue of one tile overlaps
-//             the MMAs of the next;
-//   k_gemm_pair  M and N multiples of 256: the same, by CTA pairs (clusters
-//             of two): 256 x 256 tiles, each CTA loading 128 rows of A and
-//             128 rows of B per k-step (32 KB, 6-stage ring) and the even CTA
-//             issuing tcgen05.mma.cta_group::2 M 256 N 256 over both CTAs'
-//             shared memory, so a CTA pulls a third less from L2 per FLOP;
-//   k_gemm    otherwise: one 128 x 128 tile per CTA, 3-stage ring, two CTAs
-//             per SM.
+// steps of 64 through a ring of TMA stages. Warp 0 streams tiles, warp 1
+// allocates TMEM, issues tcgen05.mma (K = 16 per instruction) and commits stage
+// releases, warps 2-5 read the accumulator with tcgen05.ld and run the
+// epilogue. Four forms, chosen by gemm_cost:
+//   k_gemm_p  persistent, one CTA per SM looping over 128 x 256 output
+//             tiles, 4-stage ring of 48 KB, two 256-column TMEM accumulators so
+//             that the epilogue of one tile overlaps the MMAs of the next;
+//   k_gemm_pair  the same by CTA pairs (clusters of two): 256 x 256 tiles, each
+//             CTA loading 128 rows of A and 128 rows of B per k-step (32 KB,
+//             6-stage ring) and the even CTA issuing tcgen05.mma.cta_group::2 M
+//             256 N 256 over both CTAs' shared memory, so a CTA pulls a third
+//             less from L2 per FLOP;
+//   k_gemm    one 128 x 128 tile per CTA, 3-stage ring, two CTAs per SM;
+//   k_gemm_tile  one 128 x {32, 64, 128} tile per CTA with a deep ring, of one
+//             or several GEMMs in a launch, K split over a cluster where even
+//             32-column tiles are too few.
 // Every wait is bounded; on expiry the kernel records it in the error flag,
 // drains and frees TMEM.
 #include <algorithm>
@@ -64,7 +65,7 @@ constexpr int GEMM_THREADS = 192;
 constexpr size_t GEMM_SMEM = 1024 + (size_t)NST * STAGE_BYTES + 256;
 // persistent form
 constexpr int PTN = 256, PNST = 4;
-constexpr int PSTAGE = A_BYTES + 2 * B_BYTES;  // A 128 x 64, B 256 x 64 (two 128-row TMA boxes)
+constexpr int PSTAGE = A_BYTES + 2 * B_BYTES;  // A 128 x 64, B 256 x 64
 constexpr size_t PGEMM_SMEM = 1024 + (size_t)PNST * PSTAGE + 256;
 // pair form
 constexpr int QNST = 6;
@@ -166,18 +167,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             int issued = 0;
             for (int kt = 0; kt < KT; ++kt) {
                 const int s = kt % NST;
-                if (kt >= NST && !tc::bar_wait(&empty[s], ((kt / NST) - 1) & 1)) {
+                if (kt >= NST && !tc::bar_wait_warp(&empty[s], ((kt / NST) - 1) & 1)) {
                     atomicOr(g.flag, 1);
                     break;
                 }
                 unsigned char* st = sm + s * STAGE_BYTES;
-                tc::bar_expect_tx(&full[s], STAGE_BYTES);
-                tc::tma_2d(st, &ta, kt * TK, m0, &full[s]);
-                tc::tma_2d(st + A_BYTES, &tb, kt * TK, n0, &full[s]);
+                if (tc::elect()) {
+                    tc::bar_expect_tx(&full[s], STAGE_BYTES);
+                    tc::tma_3d(st, &ta, m0, kt, &full[s]);
+                    tc::tma_3d(st + A_BYTES, &tb, n0, kt, &full[s]);
+                }
+                __syncwarp();
                 ++issued;
             }
             // the copies still in flight complete before the block leaves
@@ -187,23 +191,25 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = tc::bf16_f32_idesc(TM, TN);
+            const uint64_t d0 = tc::sw128_kmajor_desc(tc::smem_u32(sm));
             for (int kt = 0; kt < KT; ++kt) {
                 const int s = kt % NST;
-                if (!tc::bar_wait(&full[s], (kt / NST) & 1)) {
+                if (!tc::bar_wait_warp(&full[s], (kt / NST) & 1)) {
                     atomicOr(g.flag, 1);
                     break;
                 }
-                tc::fence_after();
-                const uint32_t a0 = tc::smem_u32(sm + s * STAGE_BYTES), b0 = a0 + A_BYTES;
+                const uint64_t da = d0 + (uint64_t)(s * (STAGE_BYTES / 16)), db = da + A_BYTES / 16;
+                if (tc::elect()) {
 #pragma unroll
-                for (int ks = 0; ks < TK / 16; ++ks)  // 16 BF16 = 32 bytes along K inside the swizzled row
-                    tc::umma_bf16(tmem, tc::sw128_kmajor_desc(a0 + ks * 32), tc::sw128_kmajor_desc(b0 + ks * 32),
-                                  idesc, (kt | ks) != 0);
-                tc::umma_commit(&empty[s]);  // stage free once these MMAs have read it
+                    for (int ks = 0; ks < TK / 16; ++ks)  // 16 BF16 = 32 bytes along K inside the swizzled row
+                        tc::umma_bf16(tmem, da + 2 * ks, db + 2 * ks, idesc, (kt | ks) != 0);
+                    tc::umma_commit(&empty[s]);  // stage free once these MMAs have read it
+                }
+                __syncwarp();
             }
-            tc::umma_commit(done);  // accumulator complete (or the issued part of it)
+            if (tc::elect()) tc::umma_commit(done);  // accumulator complete (or the issued part of it)
         }
     } else {
         // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 = tile rows
@@ -280,7 +286,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             uint32_t u = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -288,16 +294,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 tile_of(t, tiles_m, tiles_n, TM, m0, n0);
                 for (int kt = 0; kt < KT; ++kt, ++u) {
                     const uint32_t s = u % PNST;
-                    if (u >= (uint32_t)PNST && !tc::bar_wait(&empty[s], ((u / PNST) - 1) & 1)) {
+                    if (u >= (uint32_t)PNST && !tc::bar_wait_warp(&empty[s], ((u / PNST) - 1) & 1)) {
                         atomicOr(g.flag, 1);
                         ok = false;
                         break;
                     }
                     unsigned char* st = sm + s * PSTAGE;
-                    tc::bar_expect_tx(&full[s], PSTAGE);
-                    tc::tma_2d(st, &ta, kt * TK, m0, &full[s]);
-                    tc::tma_2d(st + A_BYTES, &tb, kt * TK, n0, &full[s]);
-                    tc::tma_2d(st + A_BYTES + B_BYTES, &tb, kt * TK, n0 + 128, &full[s]);
+                    if (tc::elect()) {
+                        tc::bar_expect_tx(&full[s], PSTAGE);
+                        tc::tma_3d(st, &ta, m0, kt, &full[s]);
+                        tc::tma_3d(st + A_BYTES, &tb, n0, kt, &full[s]);
+                    }
+                    __syncwarp();
                 }
             }
             // the copies still in flight complete before the block leaves
@@ -307,14 +315,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             const uint32_t idesc = tc::bf16_f32_idesc(TM, PTN);
+            const uint64_t d0 = tc::sw128_kmajor_desc(tc::smem_u32(sm));
             uint32_t u = 0;
             int it = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
                 const int ab = it & 1;
-                if (it >= 2 && !tc::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+                if (it >= 2 && !tc::bar_wait_warp(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
                     atomicOr(g.flag, 1);
                     break;
                 }
@@ -322,23 +331,25 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                 const uint32_t d = tmem + (uint32_t)(ab * PTN);
                 for (int kt = 0; kt < KT; ++kt, ++u) {
                     const uint32_t s = u % PNST;
-                    if (!tc::bar_wait(&full[s], (u / PNST) & 1)) {
+                    if (!tc::bar_wait_warp(&full[s], (u / PNST) & 1)) {
                         atomicOr(g.flag, 1);
                         ok = false;
                         break;
                     }
-                    tc::fence_after();
-                    const uint32_t a0 = tc::smem_u32(sm + s * PSTAGE), b0 = a0 + A_BYTES;
+                    const uint64_t da = d0 + (uint64_t)(s * (PSTAGE / 16)), db = da + A_BYTES / 16;
+                    if (tc::elect()) {
 #pragma unroll
-                    for (int ks = 0; ks < TK / 16; ++ks)
-                        tc::umma_bf16(d, tc::sw128_kmajor_desc(a0 + ks * 32), tc::sw128_kmajor_desc(b0 + ks * 32),
-                                      idesc, (kt | ks) != 0);
-                    tc::umma_commit(&empty[s]);
+                        for (int ks = 0; ks < TK / 16; ++ks)
+                            tc::umma_bf16(d, da + 2 * ks, db + 2 * ks, idesc, (kt | ks) != 0);
+                        tc::umma_commit(&empty[s]);
+                    }
+                    __syncwarp();
                 }
-                if (ok) tc::umma_commit(&acc_full[ab]);
+                if (ok && tc::elect()) tc::umma_commit(&acc_full[ab]);
+                __syncwarp();
             }
             // every MMA issued has completed once this arrives
-            tc::umma_commit(drain);
+            if (tc::elect()) tc::umma_commit(drain);
             tc::bar_wait(drain, 0);
         }
     } else {
@@ -420,7 +431,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     const uint32_t tmem = *tslot;
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
             uint32_t u = 0;
             bool ok = true;
             for (int t = pair; t < tiles && ok; t += pairs) {
@@ -429,16 +440,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                 const int am = m0 + (int)rank * TM, bn = n0 + (int)rank * TN;
                 for (int kt = 0; kt < KT; ++kt, ++u) {
                     const uint32_t s = u % QNST;
-                    if (u >= (uint32_t)QNST && !tc::bar_wait(&empty[s], ((u / QNST) - 1) & 1)) {
+                    if (u >= (uint32_t)QNST && !tc::bar_wait_warp(&empty[s], ((u / QNST) - 1) & 1)) {
                         atomicOr(g.flag, 1);
                         ok = false;
                         break;
                     }
-                    if (rank == 0) tc::bar_expect_tx(&full[s], 2 * QSTAGE);
-                    const uint32_t fb = tc::mapa(tc::smem_u32(&full[s]), 0);
                     unsigned char* st = sm + s * QSTAGE;
-                    tc::tma_2d_pair(st, &ta, kt * TK, am, fb);
-                    tc::tma_2d_pair(st + A_BYTES, &tb, kt * TK, bn, fb);
+                    if (tc::elect()) {
+                        if (rank == 0) tc::bar_expect_tx(&full[s], 2 * QSTAGE);
+                        const uint32_t fb = tc::mapa(tc::smem_u32(&full[s]), 0);
+                        tc::tma_3d_pair(st, &ta, am, kt, fb);
+                        tc::tma_3d_pair(st + A_BYTES, &tb, bn, kt, fb);
+                    }
+                    __syncwarp();
                 }
             }
             // rank 0 sees the pair's copies complete; rank 1's land on the
@@ -450,14 +464,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                 }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = tc::bf16_f32_idesc(2 * TM, PTN);
+            const uint64_t d0 = tc::sw128_kmajor_desc(tc::smem_u32(sm));
             uint32_t u = 0;
             int it = 0;
             bool ok = true;
             for (int t = pair; t < tiles && ok; t += pairs, ++it) {
                 const int ab = it & 1;
-                if (it >= 2 && !tc::bar_wait(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
+                if (it >= 2 && !tc::bar_wait_warp(&acc_empty[ab], ((it >> 1) - 1) & 1)) {
                     atomicOr(g.flag, 1);
                     break;
                 }
@@ -465,22 +480,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
                 const uint32_t d = tmem + (uint32_t)(ab * PTN);
                 for (int kt = 0; kt < KT; ++kt, ++u) {
                     const uint32_t s = u % QNST;
-                    if (!tc::bar_wait(&full[s], (u / QNST) & 1)) {
+                    if (!tc::bar_wait_warp(&full[s], (u / QNST) & 1)) {
                         atomicOr(g.flag, 1);
                         ok = false;
                         break;
                     }
-                    tc::fence_after();
-                    const uint32_t a0 = tc::smem_u32(sm + s * QSTAGE), b0 = a0 + A_BYTES;
+                    const uint64_t da = d0 + (uint64_t)(s * (QSTAGE / 16)), db = da + A_BYTES / 16;
+                    if (tc::elect()) {
 #pragma unroll
-                    for (int ks = 0; ks < TK / 16; ++ks)
-                        tc::umma_bf16_pair(d, tc::sw128_kmajor_desc(a0 + ks * 32),
-                                           tc::sw128_kmajor_desc(b0 + ks * 32), idesc, (kt | ks) != 0);
-                    tc::umma_commit_pair(&empty[s], 3);
+                        for (int ks = 0; ks < TK / 16; ++ks)
+                            tc::umma_bf16_pair(d, da + 2 * ks, db + 2 * ks, idesc, (kt | ks) != 0);
+                        tc::umma_commit_pair(&empty[s], 3);
+                    }
+                    __syncwarp();
                 }
-                if (ok) tc::umma_commit_pair(&acc_full[ab], 3);
+                if (ok && tc::elect()) tc::umma_commit_pair(&acc_full[ab], 3);
+                __syncwarp();
             }
-            tc::umma_commit_pair(drain, 3);
+            if (tc::elect()) tc::umma_commit_pair(drain, 3);
         }
     } else {
         const int q = warp & 3;
@@ -519,78 +536,341 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
 }
 
-// ---- small kernels ---------------------------------------------------------
-// Fourier features: f[r][j] = sin(2 pi <x_r, B_j>) (j < n_freq) and the
-// cosine at j + n_freq; rows r >= n are zero.
-__global__ void k_fourier(const float* x, int n, int n_in, const float* Bf, int n_freq, int rows, bf16* f,
-                          bf16* ft) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y;
-    if (r >= rows) return;
-    float s = 0.0f, c = 0.0f;
-    if (r < n) {
-        float a = 0.0f;
-        for (int i = 0; i < n_in; ++i) a += x[(size_t)r * n_in + i] * Bf[(size_t)i * n_freq + j];
-        const float ph = 6.283185307179586f * a;
-        s = sinf(ph);
-        c = cosf(ph);
+// Tile form: one 128 x TN tile per CTA of one or several GEMMs of a launch,
+// for outputs too small to fill the chip with 256 x 256 tiles. A deep ring
+// (the loop over K is bound by the latency and rate of one SM's loads, not by
+// the MMAs). With a cluster of S CTAs the tile's K range is split over them:
+// each accumulates its share, writes it to its own shared memory, and CTA z
+// sums columns z TN / S .. in the order of the shares (EPI_F32 only).
+//
+// Issuing a stage costs its two warps about 300 clocks whatever its size, so a
+// stage holds two 64-column blocks, fetched by one TMA box per operand:
+// 128x2048x8192 as 32-column tiles fell from 43.2 us (one block a stage, the
+// loops in one lane) over 30.8 (elected lane) to 24.7. The five weight
+// gradients of the 512-wide network run in one launch of 120 tiles instead of
+// five of 16 us each with 4 to 32 CTAs.
+template <int TN_>
+struct Tile {
+    static constexpr int b_bytes = TN_ * TK * 2;
+    static constexpr int stage = 2 * (A_BYTES + b_bytes);  // two column blocks of A, then of B
+    static constexpr int stages = TN_ == 128 ? 3 : TN_ == 64 ? 4 : 5;
+    static constexpr size_t smem = 1024 + (size_t)stages * stage + 256;
+    static constexpr int part_ld = TN_ + 4;  // row stride of a share in shared memory (floats)
+};
+struct alignas(64) GemmItem {
+    CUtensorMap ta, tb;
+    GemmOut o;
+    int epi, first;  // first tile of this GEMM in the launch; several: EPI_F32
+};
+template <int NG>
+struct GemmGroup {
+    GemmItem g[NG];
+    int n;
+};
+template <int TN_, int NG>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tile(const __grid_constant__ GemmGroup<NG> gg) {
+    using S = Tile<TN_>;
+    constexpr int NS = S::stages;
+    extern __shared__ unsigned char raw[];
+    unsigned char* sm = (unsigned char*)(((uintptr_t)raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm + NS * S::stage);
+    uint64_t* empty = full + NS;
+    uint64_t* done = empty + NS;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int split = (int)gridDim.y, part = (int)blockIdx.y;
+    int at = 0;
+    if constexpr (NG > 1)
+        while (at + 1 < gg.n && (int)blockIdx.x >= gg.g[at + 1].first) ++at;
+    const GemmItem& G = gg.g[at];
+    const GemmOut& g = G.o;
+    const int tiles_m = g.M / TM, t = (int)blockIdx.x - G.first;
+    const int m0 = t % tiles_m * TM, n0 = t / tiles_m * TN_;
+    const int KT = (g.K / TK + 1) / 2;  // two column blocks a step; the last one's second may be zero fill
+    const int kb = (int)((int64_t)KT * part / split), ke = (int)((int64_t)KT * (part + 1) / split);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NS; ++i) {
+            tc::bar_init(&full[i], 1);
+            tc::bar_init(&empty[i], 1);
+        }
+        tc::bar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const int F = 2 * n_freq;
-    f[(size_t)r * F + j] = __float2bfloat16_rn(s);
-    f[(size_t)r * F + j + n_freq] = __float2bfloat16_rn(c);
-    ft[(size_t)j * rows + r] = __float2bfloat16_rn(s);
-    ft[(size_t)(j + n_freq) * rows + r] = __float2bfloat16_rn(c);
+    if (warp == 1) tc::tmem_alloc(tslot, TN_);
+    tc::fence_before();
+    __syncthreads();
+    tc::fence_after();
+    const uint32_t tmem = *tslot;
+    const int q = warp & 3;
+    bool ok = true;
+
+    if (warp == 0) {
+        {
+            int issued = 0;
+            for (int kt = kb; kt < ke; ++kt, ++issued) {
+                const int s = issued % NS;
+                if (issued >= NS && !tc::bar_wait_warp(&empty[s], ((issued / NS) - 1) & 1)) {
+                    atomicOr(g.flag, 1);
+                    break;
+                }
+                unsigned char* st = sm + s * S::stage;
+                if (tc::elect()) {
+                    tc::bar_expect_tx(&full[s], S::stage);
+                    tc::tma_3d(st, &G.ta, m0, 2 * kt, &full[s]);
+                    tc::tma_3d(st + 2 * A_BYTES, &G.tb, n0, 2 * kt, &full[s]);
+                }
+                __syncwarp();
+            }
+            // the copies still in flight complete before the block leaves
+            for (int s = 0; s < NS && s < issued; ++s) {
+                const int last = issued - 1 - ((issued - 1 - s) % NS);
+                tc::bar_wait(&full[s], (last / NS) & 1);
+            }
+        }
+    } else if (warp == 1) {
+        {
+            const uint32_t idesc = tc::bf16_f32_idesc(TM, TN_);
+            const uint64_t d0 = tc::sw128_kmajor_desc(tc::smem_u32(sm));
+            for (int u = 0; u < ke - kb; ++u) {
+                const int s = u % NS;
+                if (!tc::bar_wait_warp(&full[s], (u / NS) & 1)) {
+                    atomicOr(g.flag, 1);
+                    break;
+                }
+                const uint64_t da = d0 + (uint64_t)(s * (S::stage / 16)), db = da + 2 * A_BYTES / 16;
+                if (tc::elect()) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+#pragma unroll
+                        for (int ks = 0; ks < TK / 16; ++ks)
+                            tc::umma_bf16(tmem, da + h * (A_BYTES / 16) + 2 * ks, db + h * (S::b_bytes / 16) + 2 * ks,
+                                          idesc, (u | h | ks) != 0);
+                    tc::umma_commit(&empty[s]);
+                }
+                __syncwarp();
+            }
+            if (tc::elect()) tc::umma_commit(done);  // accumulator complete (or the issued part of it)
+        }
+    } else {
+        ok = __all_sync(0xffffffffu, tc::bar_wait(done, 0));
+        if (!ok && lane == 0) atomicOr(g.flag, 1);
+        tc::fence_after();
+        const int row = 32 * q + lane;
+        if (ok) {
+#pragma unroll 1
+            for (int c = 0; c < TN_ / 32; ++c) {
+                float v[32];
+                tc::tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * c), v);
+                if (split > 1) {
+                    // every MMA that read the ring has completed
+                    float4* p = reinterpret_cast<float4*>(sm) + (row * S::part_ld + 32 * c) / 4;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) p[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                } else if (NG > 1 || G.epi == EPI_F32) {
+                    epilogue32<EPI_F32>(g, v, m0 + row, n0 + 32 * c);
+                } else if (G.epi == EPI_RELU) {
+                    epilogue32<EPI_RELU>(g, v, m0 + row, n0 + 32 * c);
+                } else {
+                    epilogue32<EPI_MASK>(g, v, m0 + row, n0 + 32 * c);
+                }
+            }
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (split > 1) {
+        tc::cluster_sync();  // all shares written
+        if (warp >= 2) {
+            const int w = TN_ / split, row = 32 * q + lane, c0 = part * w;
+            const uint32_t mine = tc::smem_u32(sm) + (uint32_t)(row * S::part_ld + c0) * 4;
+            float* dst = g.c32 + (size_t)(m0 + row) * g.ldc + n0 + c0;
+#pragma unroll 1
+            for (int j = 0; j < w; j += 4) {
+                float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                for (int z = 0; z < split; ++z) {
+                    const float4 b = tc::ld_cluster(tc::mapa(mine + (uint32_t)j * 4, (uint32_t)z));
+                    if (z == 0) a = b;
+                    else a = make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+                }
+                *reinterpret_cast<float4*>(dst + j) = a;
+            }
+        }
+        __syncthreads();
+        tc::cluster_sync();  // no CTA leaves while its share is read
+    }
+    if (warp == 1) {
+        __syncwarp();
+        tc::fence_after();
+        tc::tmem_dealloc(tmem, TN_);
+    }
+}
+
+// ---- small kernels ---------------------------------------------------------
+// Tiles of 64 x 64 BF16 values on their way into a matrix and its transpose,
+// whose rows of 64 values leave as 128-byte runs. 256 threads.
+constexpr int SQ = 64;
+struct alignas(16) SquareTile {
+    bf16 v[SQ][SQ + 2];
+    // the transpose: row c0 + c of t[.][ld] from r0 on; after a barrier
+    __device__ __forceinline__ void store_transposed(bf16* t, size_t ld, int c0, int r0) const {
+        for (int k = threadIdx.x; k < SQ * SQ / 2; k += 256) {
+            const int c = k / (SQ / 2), r = k % (SQ / 2) * 2;
+            *reinterpret_cast<__nv_bfloat162*>(t + (size_t)(c0 + c) * ld + r0 + r) =
+                __nv_bfloat162(v[r][c], v[r + 1][c]);
+        }
+    }
+};
+
+// Fourier features: f[r][j] = sin(2 pi <x_r, B_j>) (j < n_freq) and the
+// cosine at j + n_freq; rows r >= n are zero. Block: 64 rows, 32 frequencies
+// (columns 0..31 of the tile the sines, 32..63 the cosines).
+__global__ void __launch_bounds__(256) k_fourier(const float* x, int n, int n_in, const float* Bf, int n_freq,
+                                                 int rows, bf16* f, bf16* ft) {
+    __shared__ SquareTile t;
+    const int r0 = blockIdx.x * SQ, j0 = blockIdx.y * 32, F = 2 * n_freq;
+    const int jj = threadIdx.x & 31;
+    for (int rr = threadIdx.x >> 5; rr < SQ; rr += 8) {
+        const int r = r0 + rr, j = j0 + jj;
+        float s = 0.0f, c = 0.0f;
+        if (r < n) {
+            float a = 0.0f;
+            for (int i = 0; i < n_in; ++i) a += x[(size_t)r * n_in + i] * Bf[(size_t)i * n_freq + j];
+            const float ph = 6.283185307179586f * a;
+            s = sinf(ph);
+            c = cosf(ph);
+        }
+        t.v[rr][jj] = __float2bfloat16_rn(s);
+        t.v[rr][32 + jj] = __float2bfloat16_rn(c);
+        f[(size_t)r * F + j] = t.v[rr][jj];
+        f[(size_t)r * F + j + n_freq] = t.v[rr][32 + jj];
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < SQ * SQ / 2; k += 256) {
+        const int c = k / (SQ / 2), r = k % (SQ / 2) * 2;
+        const int row = c < 32 ? j0 + c : n_freq + j0 + c - 32;
+        *reinterpret_cast<__nv_bfloat162*>(ft + (size_t)row * rows + r0 + r) = __nv_bfloat162(t.v[r][c], t.v[r + 1][c]);
+    }
 }
 
 // Loss gradient of the mean squared error over n valid rows:
 // d = 2 (pred - y) / (n * n_out); rows >= n get zero. Loss partial sums per
-// warp (FP32; the loss value is for reporting).
-__global__ void k_mse_grad(const float* pred, const float* y, int n, int n_out, int rows, float scale, bf16* d,
-                           bf16* dt, float* loss_acc) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y;
-    if (col >= n_out) return;
-    float e = 0.0f;
-    if (r < n) e = pred[(size_t)r * n_out + col] - y[(size_t)r * n_out + col];
-    const bf16 v = __float2bfloat16_rn(scale * e);
-    d[(size_t)r * n_out + col] = v;
-    dt[(size_t)col * rows + r] = v;
-    float sq = e * e;
+// block (FP32; the loss value is for reporting). Block: 64 x 64 values.
+__global__ void __launch_bounds__(256) k_mse_grad(const float* pred, const float* y, int n, int n_out, int rows,
+                                                  float scale, bf16* d, bf16* dt, float* loss_acc) {
+    __shared__ SquareTile t;
+    __shared__ float part[8];
+    const int c0 = blockIdx.x * SQ, r0 = blockIdx.y * SQ;
+    const int c = threadIdx.x % 16 * 4;
+    float sq = 0.0f;
+#pragma unroll
+    for (int rr = threadIdx.x / 16; rr < SQ; rr += 16) {
+        const int r = r0 + rr;
+        const size_t at = (size_t)r * n_out + c0 + c;
+        float e[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (r < n) {
+            const float4 p = *reinterpret_cast<const float4*>(pred + at), q = *reinterpret_cast<const float4*>(y + at);
+            e[0] = p.x - q.x;
+            e[1] = p.y - q.y;
+            e[2] = p.z - q.z;
+            e[3] = p.w - q.w;
+        }
+        bf16 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = __float2bfloat16_rn(scale * e[k]);
+            t.v[rr][c + k] = v[k];
+            sq += e[k] * e[k];
+        }
+        __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(d + at);
+        out[0] = __nv_bfloat162(v[0], v[1]);
+        out[1] = __nv_bfloat162(v[2], v[3]);
+    }
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
-    if ((threadIdx.x & 31) == 0 && sq != 0.0f) atomicAdd(loss_acc, sq);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    t.store_transposed(dt, (size_t)rows, c0, r0);
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) sq += part[k];
+        if (sq != 0.0f) atomicAdd(loss_acc, sq);
+    }
 }
 
-// Bias gradient: db[o] = sum_r d[r][o], from the transposed copy (rows of
-// dt contiguous), summed in order by one warp per output.
-__global__ void k_bias_grad(const bf16* dt, int outs, int rows, float* db) {
-    const int o = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+// What the bias gradients and the Adam update use of the layers.
+constexpr int kMaxLayers = 16;
+struct LayerDev {
+    int in, out, first;      // first: block of k_adam or warp of k_bias_grad
+    const bf16* gt;          // [out][rows]: gradient at the layer's output, transposed
+    float *w, *gw, *mw, *vw, *b, *gb, *mb, *vb;
+    bf16 *w16, *w16t;
+};
+struct Layers {
+    LayerDev l[kMaxLayers];
+    int n, rows, total;
+};
+
+// Bias gradients of all layers: db[o] = sum_r d[r][o], from the transposed
+// copy (rows contiguous), summed in order by one warp per output.
+__global__ void k_bias_grad(const __grid_constant__ Layers a) {
+    const int w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
-    if (o >= outs) return;
+    if (w >= a.total) return;
+    int k = 0, o = w;
+    while (o >= a.l[k].out) o -= a.l[k++].out;
+    const bf16* dt = a.l[k].gt + (size_t)o * a.rows;
     float s = 0.0f;
-    for (int r = lane; r < rows; r += 32) s += __bfloat162float(dt[(size_t)o * rows + r]);
-    for (int k = 16; k > 0; k >>= 1) s += __shfl_down_sync(0xffffffffu, s, k);
-    if (lane == 0) db[o] = s;
+#pragma unroll 8
+    for (int r = lane; r < a.rows; r += 32) s += __bfloat162float(dt[r]);
+    for (int i = 16; i > 0; i >>= 1) s += __shfl_down_sync(0xffffffffu, s, i);
+    if (lane == 0) a.l[k].gb[o] = s;
 }
 
 // Adam on FP32 master weights; refreshes the BF16 copies w16 ([out][in])
-// and w16t ([in][out]) of a weight matrix (w16 null for a bias vector).
-__global__ void k_adam(float* w, const float* gw, float* m, float* v, int64_t n, int in, float lr, float b1,
-                       float b2, float eps, float c1, float c2, bf16* w16, bf16* w16t, int outs) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gg = gw[i];
-        const float mm = b1 * m[i] + (1.0f - b1) * gg;
-        const float vv = b2 * v[i] + (1.0f - b2) * gg * gg;
-        m[i] = mm;
-        v[i] = vv;
-        const float wn = w[i] - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
-        w[i] = wn;
-        if (w16) {
-            const bf16 b = __float2bfloat16_rn(wn);
-            w16[i] = b;
-            const int o = (int)(i / in), c = (int)(i % in);
-            w16t[(size_t)c * outs + o] = b;
-        }
+// and w16t ([in][out]). All layers in one launch: a block takes a 64 x 64 tile
+// of a weight matrix, the blocks after a layer's tiles 256 biases each.
+struct AdamStep {
+    float lr, b1, b2, eps, c1, c2;
+    __device__ __forceinline__ float operator()(float w, float g, float* m, float* v) const {
+        const float mm = b1 * *m + (1.0f - b1) * g;
+        const float vv = b2 * *v + (1.0f - b2) * g * g;
+        *m = mm;
+        *v = vv;
+        return w - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
     }
+};
+__global__ void __launch_bounds__(256) k_adam(const __grid_constant__ Layers a, AdamStep step) {
+    __shared__ SquareTile t;
+    int k = 0;
+    while (k + 1 < a.n && (int)blockIdx.x >= a.l[k + 1].first) ++k;
+    const LayerDev& L = a.l[k];
+    const int tile = (int)blockIdx.x - L.first, tx = L.in / SQ, tiles = tx * (L.out / SQ);
+    if (tile >= tiles) {
+        const int i = (tile - tiles) * 256 + (int)threadIdx.x;
+        if (i < L.out) L.b[i] = step(L.b[i], L.gb[i], L.mb + i, L.vb + i);
+        return;
+    }
+    const int r0 = tile / tx * SQ, c0 = tile % tx * SQ, c = (int)threadIdx.x % 16 * 4;
+#pragma unroll
+    for (int rr = threadIdx.x / 16; rr < SQ; rr += 16) {
+        const size_t at = (size_t)(r0 + rr) * L.in + c0 + c;
+        float4 w = *reinterpret_cast<float4*>(L.w + at), m = *reinterpret_cast<float4*>(L.mw + at),
+               v = *reinterpret_cast<float4*>(L.vw + at);
+        const float4 g = *reinterpret_cast<const float4*>(L.gw + at);
+        w.x = step(w.x, g.x, &m.x, &v.x);
+        w.y = step(w.y, g.y, &m.y, &v.y);
+        w.z = step(w.z, g.z, &m.z, &v.z);
+        w.w = step(w.w, g.w, &m.w, &v.w);
+        *reinterpret_cast<float4*>(L.w + at) = w;
+        *reinterpret_cast<float4*>(L.mw + at) = m;
+        *reinterpret_cast<float4*>(L.vw + at) = v;
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(w.x, w.y), hi = __floats2bfloat162_rn(w.z, w.w);
+        __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(L.w16 + at);
+        out[0] = lo;
+        out[1] = hi;
+        *reinterpret_cast<__nv_bfloat162*>(&t.v[rr][c]) = lo;
+        *reinterpret_cast<__nv_bfloat162*>(&t.v[rr][c + 2]) = hi;
+    }
+    __syncthreads();
+    t.store_transposed(L.w16t, (size_t)L.out, c0, r0);
 }
 
 __global__ void k_f32_to_bf16_both(const float* w, int outs, int in, bf16* w16, bf16* w16t) {
@@ -642,24 +922,108 @@ static EncodeFn encoder() {
     return fn;
 }
 
-// K-major BF16 operand [rows][K] (row stride K): 64 x 128 boxes, 128-byte swizzle.
-static CUtensorMap operand_map(const bf16* base, int rows, int K) {
+// K-major BF16 operand [rows][K] (row stride K) as 64-element column blocks:
+// boxes of box_rows rows of `blocks` neighbouring blocks, 128-byte swizzle;
+// blocks past the last one read as zeros.
+static CUtensorMap operand_map(const bf16* base, int rows, int K, int box_rows, int blocks) {
     if (rows % 128 || K % 64 || ((uintptr_t)base & 15)) throw Err(AFD_ERR_ARG, "GEMM operand not tile-aligned");
     CUtensorMap m;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {TK, 128}, estr[2] = {1, 1};
-    CUresult r = encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr,
+    const cuuint64_t dims[3] = {TK, (cuuint64_t)rows, (cuuint64_t)(K / TK)};
+    const cuuint64_t strides[2] = {(cuuint64_t)K * 2, TK * 2};
+    const cuuint32_t box[3] = {TK, (cuuint32_t)box_rows, (cuuint32_t)blocks}, estr[3] = {1, 1, 1};
+    CUresult r = encoder()(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw Err(AFD_ERR_CUDA, "tensor map encoding failed");
     return m;
 }
 
+// How a GEMM is launched: kPair, kPersist, kDual (k_gemm), else the columns of
+// k_gemm_tile's tiles, with the CTAs that share a tile's K range.
+enum : int { kPair = 0, kPersist = 1, kDual = 2 };
+struct GemmPlan {
+    int form, split;
+};
+
+// The time of a form in us: start, waves of tiles, per wave its epilogue and
+// its steps over K, from measurements (M x N x K, us on the device):
+//                   pair  persist  dual  tile 128   64    32
+//    256x256x64     10.4    10.4    6.3      7.3   6.3   6.3
+//   1024x512x512    12.5    12.5    8.4      8.4   6.8   6.3
+//   1024x512x2048   20.6    18.6   14.5     12.4  10.4  10.4
+//   1024x2048x4096  29.2    28.8   20.6     19.5  29.4  51.4
+//   1920x2176x1024    -       -    16.5     20.6  26.8  39.0
+//   2048x2048x2048  20.7    20.6   20.7     24.7  37.0  55.4
+//   4096x4096x4096   105     120    125      139     -     -
+// The 256-column forms pay a start and an epilogue of their own (10 us even
+// for one tile) and fill the chip from 74 and 148 tiles on; below that the
+// smaller tiles reach more SMs. A split pays a cluster launch of 4 us:
+// 128x2048x8192 runs 26.8 as 64-column tiles, 14.5 split four ways and 45.2 as
+// persistent tiles.
+static double gemm_cost(int form, int split, int64_t tiles, int K, int sms) {
+    const int kt = K / TK;
+    if (form == kPair) return 8.0 + (double)((tiles + sms / 2 - 1) / (sms / 2)) * (3.0 + 0.34 * kt);
+    const int64_t waves = (tiles * split + sms - 1) / sms;
+    if (form == kPersist) return 7.0 + (double)waves * (3.0 + 0.4 * kt);
+    // two CTAs an SM: a second one beside the first costs what it takes alone
+    if (form == kDual) return 4.0 + (double)((waves + 1) / 2) * (3.3 + 0.225 * kt * (waves > 1 ? 2 : 1));
+    const double step = (form == 128 ? 0.38 : form == 64 ? 0.325 : 0.29) * (waves > 1 ? 1.25 : 1.0);
+    return 3.0 + (double)waves * (3.3 + 0.01 * form + step * ((kt / 2 + split) / split)) + (split > 1 ? 4.0 : 0.0);
+}
+
+static GemmPlan plan_gemm(int M, int N, int K, bool may_split, int sms) {
+    const int64_t mt = M / TM;
+    GemmPlan best{kDual, 1};
+    double cost = gemm_cost(kDual, 1, mt * (N / TN), K, sms);
+    auto consider = [&](int form, int split, int64_t tiles) {
+        const double c = gemm_cost(form, split, tiles, K, sms);
+        if (c < cost) {
+            cost = c;
+            best = GemmPlan{form, split};
+        }
+    };
+    if (M % (2 * TM) == 0 && N % PTN == 0 && sms >= 2) consider(kPair, 1, mt / 2 * (N / PTN));
+    if (N % PTN == 0) consider(kPersist, 1, mt * (N / PTN));
+    for (int tn : {128, 64, 32})
+        for (int split : {1, 2, 4, 8}) {
+            const int64_t tiles = mt * (N / tn);
+            // shares of at least two steps; all clusters resident at once (of
+            // eight CTAs only two fit a GPC, and not every one: 16 of them
+            // took two rounds)
+            if (split > 1 && (!may_split || K / TK < 4 * split || tiles * split > (split == 8 ? sms * 2 / 3 : sms - 16)))
+                continue;
+            consider(tn, split, tiles);
+        }
+    return best;
+}
+
+// Tile columns with which GEMMs of M x N = `sizes` and one K run in one
+// launch, or -1 where one by one is faster.
+static int plan_group(const std::vector<std::pair<int, int>>& sizes, int K, int sms) {
+    double alone = 0.0;
+    int best = -1;
+    for (const auto& z : sizes) {
+        const GemmPlan p = plan_gemm(z.first, z.second, K, false, sms);
+        const int th = p.form == kPair ? 2 * TM : TM, tw = p.form >= 32 ? p.form : p.form == kDual ? TN : PTN;
+        alone += gemm_cost(p.form, 1, (int64_t)(z.first / th) * (z.second / tw), K, sms);
+    }
+    for (int tn : {128, 64, 32}) {
+        int64_t tiles = 0;
+        for (const auto& z : sizes) tiles += (int64_t)(z.first / TM) * (z.second / tn);
+        const double c = gemm_cost(tn, 1, tiles, K, sms);
+        if (c < alone) {
+            alone = c;
+            best = tn;
+        }
+    }
+    return best;
+}
+
 struct Gemm {
     CUtensorMap ta, tb;
     GemmOut o;
     int epi;
+    GemmPlan plan;
 };
 
 // Shared-memory limits of the GEMM kernels and the SM count, per device
@@ -679,10 +1043,19 @@ static int set_smem_attr() {
     if (dev < 0 || dev >= 64) throw Err(AFD_ERR_ARG, "device ordinal out of range");
     DeviceGemm& d = devs[dev];
     if (d.ready) return d.sms;
-    const int s1 = (int)GEMM_SMEM, s2 = (int)PGEMM_SMEM, s3 = (int)QGEMM_SMEM;
-    MCK(cudaFuncSetAttribute((const void*)k_gemm<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
-    MCK(cudaFuncSetAttribute((const void*)k_gemm<EPI_RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
-    MCK(cudaFuncSetAttribute((const void*)k_gemm<EPI_MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, s1));
+    const int s2 = (int)PGEMM_SMEM, s3 = (int)QGEMM_SMEM;
+    auto tile_attr = [](auto kernel, size_t smem) {
+        MCK(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    };
+    tile_attr(k_gemm<EPI_F32>, GEMM_SMEM);
+    tile_attr(k_gemm<EPI_RELU>, GEMM_SMEM);
+    tile_attr(k_gemm<EPI_MASK>, GEMM_SMEM);
+    tile_attr(k_gemm_tile<128, 1>, Tile<128>::smem);
+    tile_attr(k_gemm_tile<64, 1>, Tile<64>::smem);
+    tile_attr(k_gemm_tile<32, 1>, Tile<32>::smem);
+    tile_attr(k_gemm_tile<128, kMaxLayers>, Tile<128>::smem);
+    tile_attr(k_gemm_tile<64, kMaxLayers>, Tile<64>::smem);
+    tile_attr(k_gemm_tile<32, kMaxLayers>, Tile<32>::smem);
     MCK(cudaFuncSetAttribute((const void*)k_gemm_p<EPI_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
     MCK(cudaFuncSetAttribute((const void*)k_gemm_p<EPI_RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
     MCK(cudaFuncSetAttribute((const void*)k_gemm_p<EPI_MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, s2));
@@ -694,9 +1067,47 @@ static int set_smem_attr() {
     return d.sms;
 }
 
+template <int TN_, int NG>
+static void launch_tiles(const GemmGroup<NG>& gg, int tiles, int split, cudaStream_t st) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)tiles, (unsigned)split);
+    c.blockDim = dim3(GEMM_THREADS);
+    c.dynamicSmemBytes = Tile<TN_>::smem;
+    c.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 1;
+    at.val.clusterDim.y = (unsigned)split;
+    at.val.clusterDim.z = 1;
+    c.attrs = &at;
+    c.numAttrs = split > 1 ? 1 : 0;
+    MCK(cudaLaunchKernelEx(&c, k_gemm_tile<TN_, NG>, gg));
+}
+
+// The GEMMs of `v` (n <= NG, all planned with the same tile columns) in one launch.
+template <int NG>
+static void launch_group(const Gemm* v, int n, cudaStream_t st) {
+    GemmGroup<NG> gg;
+    gg.n = n;
+    const int tn = v[0].plan.form;
+    int tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        gg.g[i].ta = v[i].ta;
+        gg.g[i].tb = v[i].tb;
+        gg.g[i].o = v[i].o;
+        gg.g[i].epi = v[i].epi;
+        gg.g[i].first = tiles;
+        tiles += (v[i].o.M / TM) * (v[i].o.N / tn);
+    }
+    const int split = NG == 1 ? v[0].plan.split : 1;
+    if (tn == 128) launch_tiles<128, NG>(gg, tiles, split, st);
+    else if (tn == 64) launch_tiles<64, NG>(gg, tiles, split, st);
+    else launch_tiles<32, NG>(gg, tiles, split, st);
+}
+
 static void launch(const Gemm& G, cudaStream_t st) {
     const int sms = set_smem_attr();
-    if (G.o.M % (2 * TM) == 0 && G.o.N % PTN == 0 && sms >= 2) {
+    if (G.plan.form == kPair) {
         const int tiles = (G.o.M / (2 * TM)) * (G.o.N / PTN);
         const unsigned grid = 2u * (unsigned)std::max(1, std::min(tiles, sms / 2));
         switch (G.epi) {
@@ -704,7 +1115,7 @@ static void launch(const Gemm& G, cudaStream_t st) {
             case EPI_RELU: k_gemm_pair<EPI_RELU><<<grid, GEMM_THREADS, QGEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
             default: k_gemm_pair<EPI_MASK><<<grid, GEMM_THREADS, QGEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
         }
-    } else if (G.o.N % PTN == 0) {
+    } else if (G.plan.form == kPersist) {
         const int tiles = (G.o.M / TM) * (G.o.N / PTN);
         const unsigned grid = (unsigned)std::max(1, std::min(tiles, sms));
         switch (G.epi) {
@@ -712,22 +1123,27 @@ static void launch(const Gemm& G, cudaStream_t st) {
             case EPI_RELU: k_gemm_p<EPI_RELU><<<grid, GEMM_THREADS, PGEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
             default: k_gemm_p<EPI_MASK><<<grid, GEMM_THREADS, PGEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
         }
-    } else {
+    } else if (G.plan.form == kDual) {
         const dim3 grid((unsigned)(G.o.N / TN), (unsigned)(G.o.M / TM));
         switch (G.epi) {
             case EPI_F32: k_gemm<EPI_F32><<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
             case EPI_RELU: k_gemm<EPI_RELU><<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
             default: k_gemm<EPI_MASK><<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
         }
+    } else {
+        launch_group<1>(&G, 1, st);
     }
     MCK(cudaGetLastError());
 }
 
-static Gemm make_gemm(int epi, const bf16* A, const bf16* B, int M, int N, int K, int* flag) {
+static Gemm make_gemm(int epi, const bf16* A, const bf16* B, int M, int N, int K, int* flag, bool may_split = false,
+                      int tile = -1) {
     if (M % TM || N % TN || K % TK || K <= 0) throw Err(AFD_ERR_ARG, "GEMM sizes must be multiples of 128 x 128 x 64");
     Gemm G;
-    G.ta = operand_map(A, M, K);
-    G.tb = operand_map(B, N, K);
+    G.plan = tile < 0 ? plan_gemm(M, N, K, may_split, set_smem_attr()) : GemmPlan{tile, 1};
+    const int form = G.plan.form, blocks = form >= 32 ? 2 : 1;
+    G.ta = operand_map(A, M, K, TM, blocks);
+    G.tb = operand_map(B, N, K, form >= 32 ? form : form == kPersist ? PTN : TN, blocks);
     std::memset(&G.o, 0, sizeof(G.o));
     G.o.M = M;
     G.o.N = N;
@@ -765,6 +1181,8 @@ struct afd_mlp {
     Dev<int> flag;
     int64_t step = 0;
     std::vector<Gemm> fwd, bwd_w, bwd_x;
+    bool group_w = false;           // the weight gradients in one launch
+    Layers bias_dev{}, adam_dev{};
 
     ~afd_mlp() {
         if (stream) cudaStreamSynchronize(stream);
@@ -845,6 +1263,11 @@ struct afd_mlp {
         pred.alloc((size_t)rows * p.n_out);
         loss.alloc(1);
         flag.alloc(1);
+        // one launch for the weight gradients where they would not fill the chip one by one
+        std::vector<std::pair<int, int>> sizes;
+        for (auto* ly : L) sizes.emplace_back(ly->out, ly->in);
+        const int form_w = plan_group(sizes, rows, set_smem_attr());
+        group_w = form_w >= 0;
         // the GEMMs of one training step, with their tensor maps
         for (int l = 0; l < p.n_layers; ++l) {
             Layer& ly = *L[(size_t)l];
@@ -862,7 +1285,7 @@ struct afd_mlp {
             }
             fwd.push_back(f);
             // dW = G^T (out x rows) * X^T (in x rows)^T
-            Gemm w = make_gemm(EPI_F32, GT[(size_t)l]->p, layer_input_t(l), ly.out, ly.in, rows, flag.p);
+            Gemm w = make_gemm(EPI_F32, GT[(size_t)l]->p, layer_input_t(l), ly.out, ly.in, rows, flag.p, false, form_w);
             w.o.c32 = ly.gw.p;
             w.o.ldc = ly.in;
             bwd_w.push_back(w);
@@ -877,6 +1300,22 @@ struct afd_mlp {
                 x.o.ldmask = ly.in;
                 bwd_x.push_back(x);
             }
+        }
+        Layers& t = bias_dev;
+        t.n = p.n_layers;
+        t.rows = rows;
+        for (int l = 0; l < p.n_layers; ++l) {
+            Layer& ly = *L[(size_t)l];
+            t.l[l] = LayerDev{ly.in, ly.out, 0, GT[(size_t)l]->p, ly.w.p, ly.gw.p, ly.mw.p, ly.vw.p, ly.b.p, ly.gb.p,
+                              ly.mb.p, ly.vb.p, ly.w16.p, ly.w16t.p};
+            t.total += ly.out;
+        }
+        adam_dev = t;
+        adam_dev.total = 0;
+        for (int l = 0; l < p.n_layers; ++l) {
+            LayerDev& d = adam_dev.l[l];
+            d.first = adam_dev.total;
+            adam_dev.total += (d.in / SQ) * (d.out / SQ) + (d.out + 255) / 256;
         }
     }
 
@@ -897,8 +1336,8 @@ struct afd_mlp {
     void features(const float* x_dev, int n) {
         if (n < 1 || n > rows) throw Err(AFD_ERR_ARG, "row count outside 1..batch");
         MCK(cudaMemcpyAsync(xin.p, x_dev, (size_t)n * prm.n_in * 4, cudaMemcpyDefault, stream));
-        const dim3 grd((unsigned)((rows + 127) / 128), (unsigned)prm.n_freq);
-        k_fourier<<<grd, 128, 0, stream>>>(xin.p, n, prm.n_in, fourier.p, prm.n_freq, rows, feat.p, featT.p);
+        const dim3 grd((unsigned)(rows / SQ), (unsigned)(prm.n_freq / 32));
+        k_fourier<<<grd, 256, 0, stream>>>(xin.p, n, prm.n_in, fourier.p, prm.n_freq, rows, feat.p, featT.p);
         MCK(cudaGetLastError());
     }
 
@@ -911,17 +1350,17 @@ struct afd_mlp {
         MCK(cudaMemsetAsync(loss.p, 0, 4, stream));
         const int nl = prm.n_layers;
         const float scale = 2.0f / ((float)n * (float)prm.n_out);
-        const dim3 grd((unsigned)((prm.n_out + 255) / 256), (unsigned)rows);
+        const dim3 grd((unsigned)(prm.n_out / SQ), (unsigned)(rows / SQ));
         k_mse_grad<<<grd, 256, 0, stream>>>(pred.p, yin.p, n, prm.n_out, rows, scale, G[(size_t)nl - 1]->p,
                                             GT[(size_t)nl - 1]->p, loss.p);
         MCK(cudaGetLastError());
         for (int l = nl - 1; l >= 0; --l) {
-            launch(bwd_w[(size_t)l], stream);
-            Layer& ly = *L[(size_t)l];
-            k_bias_grad<<<(unsigned)((ly.out + 7) / 8), 256, 0, stream>>>(GT[(size_t)l]->p, ly.out, rows, ly.gb.p);
-            MCK(cudaGetLastError());
+            if (!group_w) launch(bwd_w[(size_t)l], stream);
             if (l > 0) launch(bwd_x[(size_t)l - 1], stream);
         }
+        if (group_w) launch_group<kMaxLayers>(bwd_w.data(), nl, stream);
+        k_bias_grad<<<(unsigned)((bias_dev.total + 7) / 8), 256, 0, stream>>>(bias_dev);
+        MCK(cudaGetLastError());
     }
 
     void adam() {
@@ -929,15 +1368,8 @@ struct afd_mlp {
         const float b1 = prm.beta1, b2 = prm.beta2;
         const float c1 = 1.0f - (float)std::pow((double)b1, (double)step);
         const float c2 = 1.0f - (float)std::pow((double)b2, (double)step);
-        for (auto* lp : L) {
-            Layer& ly = *lp;
-            const int64_t nw = (int64_t)ly.in * ly.out;
-            k_adam<<<592, 256, 0, stream>>>(ly.w.p, ly.gw.p, ly.mw.p, ly.vw.p, nw, ly.in, prm.lr, b1, b2, prm.eps, c1,
-                                            c2, ly.w16.p, ly.w16t.p, ly.out);
-            k_adam<<<4, 256, 0, stream>>>(ly.b.p, ly.gb.p, ly.mb.p, ly.vb.p, ly.out, 1, prm.lr, b1, b2, prm.eps, c1, c2,
-                                          nullptr, nullptr, 1);
-            MCK(cudaGetLastError());
-        }
+        k_adam<<<(unsigned)adam_dev.total, 256, 0, stream>>>(adam_dev, AdamStep{prm.lr, b1, b2, prm.eps, c1, c2});
+        MCK(cudaGetLastError());
     }
 };
 
@@ -1099,7 +1531,7 @@ int afd_gemm_bf16_async(const void* a, const void* b, float* c, int32_t M, int32
                         int32_t* status) {
     try {
         if (!a || !b || !c || !status) throw Err(AFD_ERR_ARG, "null pointer");
-        Gemm g = make_gemm(EPI_F32, (const bf16*)a, (const bf16*)b, M, N, K, status);
+        Gemm g = make_gemm(EPI_F32, (const bf16*)a, (const bf16*)b, M, N, K, status, true);
         g.o.c32 = c;
         g.o.ldc = N;
         launch(g, (cudaStream_t)stream);
@@ -1119,23 +1551,26 @@ int afd_gemm_bf16(const void* a, const void* b, float* c, int32_t M, int32_t N, 
         int dev = 0;
         MCK(cudaGetDevice(&dev));
         if (dev < 0 || dev >= 64) throw Err(AFD_ERR_ARG, "device ordinal out of range");
-        static Dev<int> flags[64];  // the wait-expired flag of each device, kept for the process
-        Dev<int>& flag = flags[dev];
+        // the wait-expired flag of each device, kept for the process: host
+        // memory that the kernel writes only when a wait expires, so that a
+        // call needs neither a clearing launch nor a copy back
+        static int* flags[64];
         {
             std::lock_guard<std::mutex> lock(g_gemm_mu);
-            if (!flag.p) flag.alloc(1);
+            if (!flags[dev]) MCK(cudaHostAlloc((void**)&flags[dev], sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
         }
-        Gemm g = make_gemm(EPI_F32, (const bf16*)a, (const bf16*)b, M, N, K, flag.p);
+        volatile int* flag = flags[dev];
+        int* mapped = nullptr;
+        MCK(cudaHostGetDevicePointer((void**)&mapped, flags[dev], 0));
+        Gemm g = make_gemm(EPI_F32, (const bf16*)a, (const bf16*)b, M, N, K, mapped, true);
         g.o.c32 = c;
         g.o.ldc = N;
         cudaStream_t st = (cudaStream_t)stream;
         // one flag per device: concurrent calls on one device share it
-        MCK(cudaMemsetAsync(flag.p, 0, sizeof(int), st));
+        *flag = 0;
         launch(g, st);
-        int f = 0;
-        MCK(cudaMemcpyAsync(&f, flag.p, 4, cudaMemcpyDeviceToHost, st));
         MCK(cudaStreamSynchronize(st));
-        if (f) throw Err(AFD_ERR_CUDA, "GEMM pipeline wait timed out");
+        if (*flag) throw Err(AFD_ERR_CUDA, "GEMM pipeline wait timed out");
         return AFD_OK;
     } catch (const Err& e) {
         g_create_err = e.what();

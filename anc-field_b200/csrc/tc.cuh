@@ -1,6 +1,6 @@
 // Blackwell (sm_100a) tensor-core building blocks used by the surrogate's
 // GEMMs: TMEM allocation, UMMA shared-memory and instruction descriptors,
-// tcgen05.mma issue and commit, tcgen05.ld of the accumulator, 2-D TMA
+// tcgen05.mma issue and commit, tcgen05.ld of the accumulator, 3-D TMA
 // loads (no multicast) and bounded mbarrier waits.
 //
 // Operand tiles are K-major BF16 with 64 elements (128 bytes) per row,
@@ -60,12 +60,32 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity) {
     }
 }
 
-// 2-D tiled TMA load into shared memory, completing on an mbarrier.
-__device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* b) {
+// The same for a whole warp, which stays together: true for all lanes or for none.
+__device__ __forceinline__ bool bar_wait_warp(uint64_t* b, uint32_t parity) {
+    return __all_sync(0xffffffffu, bar_wait(b, parity));
+}
+
+// True in one lane of a converged warp, the same one every time. The warps that
+// issue copies and MMAs run their loops with all lanes and elect the issuing
+// one: with the loop itself inside `if (lane == 0)` a step of the ring took 580
+// clocks to issue against 300 this way.
+__device__ __forceinline__ bool elect() {
+    uint32_t p;
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(b))
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
+// 3-D tiled TMA load into shared memory (64 elements from x = 0, rows from y,
+// 64-element column blocks from z), completing on an mbarrier.
+__device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int y, int z, uint64_t* b) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(smem_u32(b))
         : "memory");
 }
 
@@ -166,17 +186,26 @@ __device__ __forceinline__ uint32_t mapa(uint32_t smem_addr, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
     return r;
 }
+// 16 bytes of another CTA's shared memory
+__device__ __forceinline__ float4 ld_cluster(uint32_t cluster_addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(cluster_addr)
+                 : "memory");
+    return v;
+}
 // arrive on an mbarrier of either CTA of the cluster
 __device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// 2-D TMA load into this CTA's shared memory whose completion is counted on
-// an mbarrier of either CTA of the pair (cluster address); no multicast.
-__device__ __forceinline__ void tma_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster) {
+// 3-D TMA load (as tma_3d) into this CTA's shared memory whose completion is
+// counted on an mbarrier of either CTA of the pair (cluster address); no multicast.
+__device__ __forceinline__ void tma_3d_pair(void* dst, const CUtensorMap* map, int y, int z, uint32_t bar_cluster) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-        "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar_cluster)
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(bar_cluster)
         : "memory");
 }
 // one warp of each CTA (the same warp)
