@@ -306,167 +306,6 @@ static void launch_lrs(const StepArgs& a, int j, dim3 grd, cudaStream_t st) {
 }
 
 // ---- PML -------------------------------------------------------------------
-// Face averages of pml.cl:74-122 (fi_*_avg, p_*_avg, psi_*_avg share one
-// pattern each): x-faces average over (y, y+1) x (z, z+1), y-faces over
-// (x, x+1) x (z, z+1), z-faces over (x, x+1) x (y, y+1). `own` replaces the
-// value of cell `self` when it is one of the four (the reference kernel's
-// own write becomes visible to its later reads, pml.cl:185-188).
-struct Avg {
-    const float* f;
-    int64_t self;
-    float own;
-    bool subst;
-    __device__ __forceinline__ float v(int64_t i) const { return (subst && i == self) ? own : f[i]; }
-    __device__ __forceinline__ float ax(int64_t i, int64_t pitch, int64_t plane) const {
-        return 0.25f * (((v(i) + v(i + plane)) + v(i + pitch)) + v(i + pitch + plane));
-    }
-    __device__ __forceinline__ float ay(int64_t i, int64_t pitch, int64_t plane) const {
-        return 0.25f * (((v(i) + v(i + plane)) + v(i + 1)) + v(i + 1 + plane));
-    }
-    __device__ __forceinline__ float az(int64_t i, int64_t pitch, int64_t plane) const {
-        return 0.25f * (((v(i) + v(i + pitch)) + v(i + 1)) + v(i + 1 + pitch));
-    }
-};
-
-// PML pressure update, pml.cl:185-207. Returns p^{n+1}; psi_new receives
-// psi^{n+1/2} = dt*p^n + psi^{n-1/2}.
-__device__ __forceinline__ float pml_pressure(const StepArgs& a, const float* pc, const float* po,
-                                              const float* fx1, const float* fy1, const float* fz1,
-                                              const float* psimh, int x, int y, int z, int64_t i,
-                                              float* psi_new) {
-    const PmlDev& P = a.pml;
-    const int64_t pitch = a.g.pitch, plane = a.g.plane;
-    const float kx = P.ksi[0][x], ky = P.ksi[1][y], kz = P.ksi[2][z];
-    const float pm1 = pc[i];
-    const float ps = P.dt * pm1 + psimh[i];
-    *psi_new = ps;
-    float s = pc[i + 1] + pc[i - 1];
-    s = s + pc[i + pitch];
-    s = s + pc[i - pitch];
-    s = s + pc[i + plane];
-    s = s + pc[i - plane];
-    s = s - 6.0f * pm1;
-    const float A = P.cc_dxdx * s;
-    const Avg FX{fx1, -1, 0.0f, false}, FY{fy1, -1, 0.0f, false}, FZ{fz1, -1, 0.0f, false};
-    float d = FX.ax(i + 1, pitch, plane) - FX.ax(i, pitch, plane);
-    d = d + FY.ay(i + pitch, pitch, plane);
-    d = d - FY.ay(i, pitch, plane);
-    d = d + FZ.az(i + plane, pitch, plane);
-    d = d - FZ.az(i, pitch, plane);
-    const float B = P.inv_dx * d;
-    const float C = kx * ky * kz * 0.5f * (ps + psimh[i]);
-    const float D = P.inv_dt2 * (po[i] - 2.0f * pm1);
-    const float E = (kx * ky + ky * kz + kz * kx) * pm1;
-    const float F = (kx + ky + kz) / P.two_dt * po[i];
-    const float num = A + B - C - D - E + F;
-    return num / (P.inv_dt2 + (kx + ky + kz) / P.two_dt);
-}
-
-// Auxiliary field updates of pml.cl:231-262 for one cell. REF: `p` reads
-// see the cell's own new pressure and the other cells' values before the
-// PML pass; the x-derivative's last term reads p (pml.cl:126) and fi_y's
-// psi coefficient reads ksi_x at y (pml.cl:247). FIXED: both corrected.
-template <bool REF>
-__device__ __forceinline__ void pml_aux(const StepArgs& a, unsigned axes, const float* pnew,
-                                        const float* pc, const float* psiph, float p_own,
-                                        float psi_own, const float* fx1, const float* fy1,
-                                        const float* fz1, float* fx, float* fy, float* fz, int x,
-                                        int y, int z, int64_t i) {
-    const PmlDev& P = a.pml;
-    const int64_t pitch = a.g.pitch, plane = a.g.plane;
-    const Avg Pn{pnew, i, p_own, REF}, Pm{pc, -1, 0.0f, false}, Ps{psiph, i, psi_own, REF};
-    const Avg& Plast = REF ? Pn : Pm;
-    const float kax = 0.5f * (P.ksi[0][x] + P.ksi[0][x + 1]);
-    const float kay = 0.5f * (P.ksi[1][y] + P.ksi[1][y + 1]);
-    const float kaz = 0.5f * (P.ksi[2][z] + P.ksi[2][z + 1]);
-    const bool psi = REF || P.psi_on;
-    if (axes & 1u) {
-        const float dxp = P.half_inv_dx * (Pn.ax(i + 1, pitch, plane) - Pn.ax(i, pitch, plane) +
-                                           Pm.ax(i + 1, pitch, plane) - Plast.ax(i, pitch, plane));
-        const float dxpsi = psi ? P.inv_dx * (Ps.ax(i + 1, pitch, plane) - Ps.ax(i, pitch, plane)) : 0.0f;
-        const float f1 = fx1[i];
-        fx[i] = (-0.5f * kax * f1 + (kay + kaz - kax) * dxp + (kay * kaz) * dxpsi + P.inv_dt * f1) /
-                (P.inv_dt + kax * 0.5f);
-    }
-    if (axes & 2u) {
-        const float dyp = P.half_inv_dx * (Pn.ay(i + pitch, pitch, plane) - Pn.ay(i, pitch, plane) +
-                                           Pm.ay(i + pitch, pitch, plane) - Plast.ay(i, pitch, plane));
-        const float dypsi = psi ? P.inv_dx * (Ps.ay(i + pitch, pitch, plane) - Ps.ay(i, pitch, plane)) : 0.0f;
-        const float kx_coef = REF ? 0.5f * (P.ksi[0][y] + P.ksi[0][y + 1]) : kax;
-        const float f1 = fy1[i];
-        fy[i] = (-0.5f * kay * f1 + (kax + kaz - kay) * dyp + (kx_coef * kaz) * dypsi + P.inv_dt * f1) /
-                (P.inv_dt + kay * 0.5f);
-    }
-    if (axes & 4u) {
-        const float dzp = P.half_inv_dx * (Pn.az(i + plane, pitch, plane) - Pn.az(i, pitch, plane) +
-                                           Pm.az(i + plane, pitch, plane) - Plast.az(i, pitch, plane));
-        const float dzpsi = psi ? P.inv_dx * (Ps.az(i + plane, pitch, plane) - Ps.az(i, pitch, plane)) : 0.0f;
-        const float f1 = fz1[i];
-        fz[i] = (-0.5f * kaz * f1 + (kax + kay - kaz) * dzp + (kax * kay) * dzpsi + P.inv_dt * f1) /
-                (P.inv_dt + kaz * 0.5f);
-    }
-}
-
-// REF pass 1: auxiliary fields of every cell 2..n-3, using the cell's own
-// new pressure and psi recomputed locally (nothing written that is read).
-__global__ void __launch_bounds__(256) k_pml_ref_aux(StepArgs a, int j) {
-    const StepIdx I = step_at(a, j);
-    const long long g = I.g;
-    const TlMark tl(a, 3, g, blockIdx.z < (unsigned)(a.g.nz - 4));
-    const int x = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = 2 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int zn = a.g.nz - 4;
-    const int b = blockIdx.z / zn;
-    const int z = 2 + blockIdx.z % zn;
-    if (x > a.g.nx - 3 || y > a.g.ny - 3) return;
-    const int W = a.pml.width;
-    unsigned axes = 0;
-    if (x < W || x > a.g.nx - W - 1) axes |= 1u;
-    if (y < W || y > a.g.ny - W - 1) axes |= 2u;
-    if (z < W || z > a.g.nz - W - 1) axes |= 4u;
-    if (!axes) return;
-    const size_t base = (size_t)b * a.g.vol;
-    const float* pn = a.p[I.wn] + base;
-    const float* pc = a.p[I.wc] + base;
-    const float* po = a.p[I.wo] + base;
-    const int lv = I.lv;
-    const float* fx1 = a.pml.fi[0][lv ^ 1] + base;
-    const float* fy1 = a.pml.fi[1][lv ^ 1] + base;
-    const float* fz1 = a.pml.fi[2][lv ^ 1] + base;
-    const float* psiph = a.pml.psi[lv] + base;
-    const float* psimh = a.pml.psi[lv ^ 1] + base;
-    const int64_t i = (int64_t)z * a.g.plane + (int64_t)y * a.g.pitch + x;
-    float psi_new;
-    const float p_new = pml_pressure(a, pc, po, fx1, fy1, fz1, psimh, x, y, z, i, &psi_new);
-    pml_aux<true>(a, axes, pn, pc, psiph, p_new, psi_new, fx1, fy1, fz1, a.pml.fi[0][lv] + base,
-                  a.pml.fi[1][lv] + base, a.pml.fi[2][lv] + base, x, y, z, i);
-}
-
-// REF pass 2: pressure and psi of every cell 2..n-3 (pml.cl:182-207).
-__global__ void __launch_bounds__(256) k_pml_ref_p(StepArgs a, int j) {
-    const StepIdx I = step_at(a, j);
-    const long long g = I.g;
-    const TlMark tl(a, 2, g, blockIdx.z < (unsigned)(a.g.nz - 4));
-    const int x = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = 2 + blockIdx.y * blockDim.y + threadIdx.y;
-    const int zn = a.g.nz - 4;
-    const int b = blockIdx.z / zn;
-    const int z = 2 + blockIdx.z % zn;
-    if (x > a.g.nx - 3 || y > a.g.ny - 3) return;
-    const size_t base = (size_t)b * a.g.vol;
-    float* pn = a.p[I.wn] + base;
-    const float* pc = a.p[I.wc] + base;
-    const float* po = a.p[I.wo] + base;
-    const int lv = I.lv;
-    const int64_t i = (int64_t)z * a.g.plane + (int64_t)y * a.g.pitch + x;
-    float psi_new;
-    const float v = pml_pressure(a, pc, po, a.pml.fi[0][lv ^ 1] + base, a.pml.fi[1][lv ^ 1] + base,
-                                 a.pml.fi[2][lv ^ 1] + base, a.pml.psi[lv ^ 1] + base, x, y, z, i,
-                                 &psi_new);
-    a.pml.psi[lv][base + i] = psi_new;
-    pn[i] = v;
-}
-
 // ---- FIXED-mode PML over dense slab boxes ----------------------------------
 // Axes whose enabled slab meets the coordinate ranges (inclusive): for one
 // cell, the auxiliary fields it updates; for a cell's 2x2x2 cube, the fields
@@ -566,11 +405,12 @@ __device__ __forceinline__ float pml_p_cell(const PmlDev& P, float s6, float c, 
 
 // Auxiliary field of one PML cell (pml.cl:231-262 with the derivative and ksi
 // index corrected): f1 its previous value, k the damping average along its
-// axis, k1 and k2 along the others in axis order, dp and dpsi the derivatives.
+// axis, k1 and k2 along the others in axis order, k12 their product, dp and dpsi
+// the derivatives.
 template <typename Q>
 __device__ __forceinline__ float pml_aux_cell(const PmlDev& P, float f1, float k, float k1, float k2, float dp,
-                                              float dpsi, Q quot) {
-    return quot(-0.5f * k * f1 + (k1 + k2 - k) * dp + (k1 * k2) * dpsi + P.inv_dt * f1, P.inv_dt + k * 0.5f);
+                                              float k12, float dpsi, Q quot) {
+    return quot(-0.5f * k * f1 + (k1 + k2 - k) * dp + k12 * dpsi + P.inv_dt * f1, P.inv_dt + k * 0.5f);
 }
 
 // The face average of four values in the order of pml.cl:74-122: x-faces take
@@ -644,20 +484,15 @@ __device__ __forceinline__ void row5n(const T* p, float r[5], float inv, bool fi
     }
 }
 
-// Pressure of the PML cells (pml.cl:185-207 restricted to the slab cells)
-// of one 4-cell unit x..x+3 of row (y, z). Fields outside the read axes are
-// identically zero there and are not loaded; PSI: psi is kept (PML faces on
-// all three axes). sc: the member's FP16 scales (1 for FP32 storage).
-template <bool PSI, typename T, bool NC = true>
-__device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int y, int z, const StepIdx& I,
-                                           const LevelScales& sc) {
-    // The mask gates only the stores, the flag and the numerators: the loads
-    // below issue without waiting for it (every unit of a box lies in planes
-    // and rows 2..n-3, so x-1 .. x+4, y+-1 and z+-1 stay inside the level and
-    // field arrays even for a unit with no PML cell, whose results are dropped).
-    const unsigned m = pml_mask4(a, x, y, z);
+// PML pressure (pml.cl:185-207) of the cells x..x+3 of row (y, z) into v, not
+// stored, with their damping sums ks and the old and new psi (pmh, ps; PSI:
+// psi is kept). ra: axes whose auxiliary fields are read; elsewhere they are
+// identically zero. row0 receives p^n of x..x+4.
+template <bool PSI, typename T, bool NC>
+__device__ __forceinline__ void pml_p_calc(const StepArgs& a, size_t base, int x, int y, int z, const StepIdx& I,
+                                           const LevelScales& sc, unsigned ra, float v[4], float ps[4],
+                                           float row0[5]) {
     const PmlDev& P = a.pml;
-    const size_t base = (size_t)b * a.g.vol;
     const int pitch = (int)a.g.pitch, plane = (int)a.g.plane;
     const int i = z * plane + y * pitch + x;  // a member has fewer than 2^31 cells
     const T* pc = level_ptr<T>(a, I.wc) + base;
@@ -666,7 +501,8 @@ __device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int 
     // x+4 is read only where it lies in the row (the unit's last cell can be
     // a PML cell only then)
     const bool hi = x + 4 < pitch;
-    float c[5], ym4[5], yp4[5], zm4[5], zp4[5], o[5];
+    float* const c = row0;
+    float ym4[5], yp4[5], zm4[5], zp4[5], o[5];
     row5n<NC>(pc + i, c, ic, hi);
     const float xm = x >= 1 ? lvl<NC>(pc + i - 1, ic) : 0.0f;
     row5n<NC>(pc + (i - pitch), ym4, ic, false);
@@ -677,7 +513,6 @@ __device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int 
     const float4 kx4 = __ldg(reinterpret_cast<const float4*>(P.ksi[0] + x));
     const float kx[4] = {kx4.x, kx4.y, kx4.z, kx4.w};
     const float ky = __ldg(P.ksi[1] + y), kz = __ldg(P.ksi[2] + z);
-    const unsigned ra = slab_axes(a, x, x + 4, y, y + 1, z, z + 1);
     float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     auto field = [&](int ax, auto add) {
         const float* f = P.fi[ax][I.lv ^ 1] + base;
@@ -691,19 +526,18 @@ __device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int 
     if (ra & 1u) field(0, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<0>(q, r, s, t, d); });
     if (ra & 2u) field(1, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<1>(q, r, s, t, d); });
     if (ra & 4u) field(2, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<2>(q, r, s, t, d); });
-    float ps[4] = {0.0f, 0.0f, 0.0f, 0.0f}, pmh[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float pmh[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if (PSI) {
         const float4 h = *reinterpret_cast<const float4*>(P.psi[I.lv ^ 1] + base + i);
         pmh[0] = h.x;
         pmh[1] = h.y;
         pmh[2] = h.z;
         pmh[3] = h.w;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) ps[q] = P.dt * c[q] + pmh[q];
-        store4(P.psi[I.lv] + base + i, ps, m);
     }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ps[q] = PSI ? P.dt * c[q] + pmh[q] : 0.0f;
     // ks depends on kx only within the row: one division when the four agree
-    float v[4], ks[4];
+    float ks[4];
     if (kx[0] == kx[1] && kx[1] == kx[2] && kx[2] == kx[3]) {
         ks[0] = ks[1] = ks[2] = ks[3] = (kx[0] + ky + kz) / P.two_dt;
     } else {
@@ -719,6 +553,28 @@ __device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int 
         s6 = s6 + zm4[q];
         v[q] = pml_p_cell(P, s6, c[q], o[q], kx[q], ky, kz, ks[q], d[q], ps[q], pmh[q],
                           [](float n, float den) { return n / den; });
+    }
+}
+
+// Pressure of the PML cells (pml.cl:185-207 restricted to the slab cells)
+// of one 4-cell unit x..x+3 of row (y, z). Fields outside the read axes are
+// identically zero there and are not loaded; PSI: psi is kept (PML faces on
+// all three axes). sc: the member's FP16 scales (1 for FP32 storage).
+template <bool PSI, typename T, bool NC = true>
+__device__ __forceinline__ void pml_p_unit(const StepArgs& a, int b, int x, int y, int z, const StepIdx& I,
+                                           const LevelScales& sc) {
+    // The mask gates only the stores, the flag and the numerators: the loads
+    // issue without waiting for it (every unit of a box lies in planes and
+    // rows 2..n-3, so x-1 .. x+4, y+-1 and z+-1 stay inside the level and
+    // field arrays even for a unit with no PML cell, whose results are dropped).
+    const unsigned m = pml_mask4(a, x, y, z);
+    const size_t base = (size_t)b * a.g.vol;
+    const int i = z * (int)a.g.plane + y * (int)a.g.pitch + x;
+    float v[4], ps[4], c[5];
+    pml_p_calc<PSI, T, NC>(a, base, x, y, z, I, sc, slab_axes(a, x, x + 4, y, y + 1, z, z + 1), v, ps, c);
+    if (PSI) store4(a.pml.psi[I.lv] + base + i, ps, m);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
         if constexpr (sizeof(T) == 4) {
             if ((m >> q) & 1u) watch(a.flag, v[q]);
         } else {
@@ -780,10 +636,135 @@ __device__ __forceinline__ void pml_aux_unit(const StepArgs& a, int b, int x, in
             face_ends<AX>(s00, s01, s10, s11, q, &sh, &sl);
             dpsi = P.inv_dx * (sh - sl);
         }
-        out[q] = pml_aux_cell(P, f1v[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), AX == 0 ? kay : kax,
-                              AX == 2 ? kay : kaz, dp, dpsi, [](float n, float den) { return n / den; });
+        const float k1 = AX == 0 ? kay : kax, k2 = AX == 2 ? kay : kaz;
+        out[q] = pml_aux_cell(P, f1v[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), k1, k2, dp, k1 * k2, dpsi,
+                              [](float n, float den) { return n / den; });
     }
     store4(P.fi[AX][I.lv] + base + i, out, m);
+}
+
+// ---- REF-mode PML ------------------------------------------------------------
+// The reference's PML kernel works on every cell 2..n-3 and reads its
+// neighbours' pressure before they have their PML update, its own after
+// (pml.cl:185-188): first the auxiliary fields, with the cell's own new
+// pressure and psi formed locally, then pressure and psi. Units of four cells
+// as in FIXED mode: the kernels are bound by load instructions (every array of
+// a grid stays in L2), of which a thread per cell issued 60.
+//
+// Unit u of plane z of the launch: cells x..x+3, valid ones as the mask m.
+__device__ __forceinline__ bool ref_unit(const StepArgs& a, int* b, int* x, int* y, int* z, unsigned* m) {
+    const unsigned nu = (unsigned)(a.g.nx + 1) / 4;  // units that hold a cell 2..nx-3
+    const unsigned u = blockIdx.x * blockDim.x + threadIdx.x, row = u / nu;
+    const int zn = a.g.nz - 4;
+    *b = (int)blockIdx.y / zn;
+    *z = 2 + (int)blockIdx.y % zn;
+    *y = 2 + (int)row;
+    *x = 4 * (int)(u - row * nu);
+    if (*y > a.g.ny - 3) return false;
+    *m = 15u;
+    if (*x == 0) *m &= 12u;
+    if (*x + 3 > a.g.nx - 3) *m &= (1u << (a.g.nx - 2 - *x)) - 1u;
+    return true;
+}
+// axes whose slabs meet x0..x1, y0..y1, z0..z1
+__device__ __forceinline__ unsigned ref_axes(const StepArgs& a, int x0, int x1, int y0, int y1, int z0, int z1) {
+    const int W = a.pml.width;
+    return (x0 < W || x1 > a.g.nx - W - 1 ? 1u : 0u) | (y0 < W || y1 > a.g.ny - W - 1 ? 2u : 0u) |
+           (z0 < W || z1 > a.g.nz - W - 1 ? 4u : 0u);
+}
+
+// Auxiliary fields of pml.cl:231-262, with the reference's derivatives (their
+// last term reads p, pml.cl:126) and fi_y's psi coefficient (ksi_x at y,
+// pml.cl:247). The cell's own p and psi are the first of the four values of
+// its lower faces.
+__global__ void __launch_bounds__(256) k_pml_ref_aux(StepArgs a, int j) {
+    const StepIdx I = step_at(a, j);
+    const TlMark tl(a, 3, I.g, blockIdx.y < (unsigned)(a.g.nz - 4));
+    int b, x, y, z;
+    unsigned m;
+    if (!ref_unit(a, &b, &x, &y, &z, &m)) return;
+    const unsigned axes = ref_axes(a, x, x + 3, y, y, z, z);
+    if (!axes) return;
+    const PmlDev& P = a.pml;
+    const size_t base = (size_t)b * a.g.vol;
+    const int pitch = (int)a.g.pitch, plane = (int)a.g.plane, i = z * plane + y * pitch + x;
+    const bool hi = x + 4 < pitch;
+    const LevelScales sc = level_scales<float>(a, b, I.s5);
+    float own[4], ps[4], m00[5];
+    pml_p_calc<true, float, true>(a, base, x, y, z, I, sc, ref_axes(a, x, x + 4, y, y + 1, z, z + 1), own, ps, m00);
+    const float *pn = a.p[I.wn] + base, *pc = a.p[I.wc] + base, *sp = P.psi[I.lv] + base;
+    float n00[5], n01[5], n10[5], n11[5], m01[5], m10[5], m11[5], s00[5], s01[5], s10[5], s11[5];
+    row5(pn + i, n00, hi);
+    row5(pn + (i + plane), n01, hi);
+    row5(pn + (i + pitch), n10, hi);
+    row5(pn + (i + pitch + plane), n11, hi);
+    row5(pc + (i + plane), m01, hi);
+    row5(pc + (i + pitch), m10, hi);
+    row5(pc + (i + pitch + plane), m11, hi);
+    row5(sp + i, s00, hi);
+    row5(sp + (i + plane), s01, hi);
+    row5(sp + (i + pitch), s10, hi);
+    row5(sp + (i + pitch + plane), s11, hi);
+    float kxs[5];
+    row5(P.ksi[0] + x, kxs, hi);
+    const float kay = 0.5f * (__ldg(P.ksi[1] + y) + __ldg(P.ksi[1] + y + 1));
+    const float kaz = 0.5f * (__ldg(P.ksi[2] + z) + __ldg(P.ksi[2] + z + 1));
+    const float kxy = 0.5f * (__ldg(P.ksi[0] + y) + __ldg(P.ksi[0] + y + 1));
+    auto field = [&](auto axis, unsigned cells) {
+        constexpr int AX = decltype(axis)::value;
+        const float4 f14 = *reinterpret_cast<const float4*>(P.fi[AX][I.lv ^ 1] + base + i);
+        const float f1[4] = {f14.x, f14.y, f14.z, f14.w};
+        float out[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float nh, nl, mh, ml, sh, sl;
+            face_ends<AX>(n00, n01, n10, n11, q, &nh, &nl);
+            face_ends<AX>(m00, m01, m10, m11, q, &mh, &ml);
+            face_ends<AX>(s00, s01, s10, s11, q, &sh, &sl);
+            // the lower faces with the cell's own new values
+            if constexpr (AX == 0) {
+                nl = face4(own[q], n01[q], n10[q], n11[q]);
+                sl = face4(ps[q], s01[q], s10[q], s11[q]);
+            } else if constexpr (AX == 1) {
+                nl = face4(own[q], n01[q], n00[q + 1], n01[q + 1]);
+                sl = face4(ps[q], s01[q], s00[q + 1], s01[q + 1]);
+            } else {
+                nl = face4(own[q], n10[q], n00[q + 1], n10[q + 1]);
+                sl = face4(ps[q], s10[q], s00[q + 1], s10[q + 1]);
+            }
+            const float dp = P.half_inv_dx * (nh - nl + mh - nl), dpsi = P.inv_dx * (sh - sl);
+            const float kax = 0.5f * (kxs[q] + kxs[q + 1]);
+            const float k1 = AX == 0 ? kay : kax, k2 = AX == 2 ? kay : kaz;
+            out[q] = pml_aux_cell(P, f1[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), k1, k2, dp,
+                                  AX == 1 ? kxy * kaz : k1 * k2, dpsi, [](float n, float den) { return n / den; });
+        }
+        store4(P.fi[AX][I.lv] + base + i, out, cells);
+    };
+    if (axes & 1u) {
+        unsigned cells = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (x + q < P.width || x + q > a.g.nx - P.width - 1) cells |= 1u << q;
+        field(std::integral_constant<int, 0>{}, m & cells);
+    }
+    if (axes & 2u) field(std::integral_constant<int, 1>{}, m);
+    if (axes & 4u) field(std::integral_constant<int, 2>{}, m);
+}
+
+// Pressure and psi of every cell 2..n-3 (pml.cl:182-207).
+__global__ void __launch_bounds__(256) k_pml_ref_p(StepArgs a, int j) {
+    const StepIdx I = step_at(a, j);
+    const TlMark tl(a, 2, I.g, blockIdx.y < (unsigned)(a.g.nz - 4));
+    int b, x, y, z;
+    unsigned m;
+    if (!ref_unit(a, &b, &x, &y, &z, &m)) return;
+    const size_t base = (size_t)b * a.g.vol;
+    const int i = z * (int)a.g.plane + y * (int)a.g.pitch + x;
+    float v[4], ps[4], c[5];
+    pml_p_calc<true, float, true>(a, base, x, y, z, I, level_scales<float>(a, b, I.s5),
+                                  ref_axes(a, x, x + 4, y, y + 1, z, z + 1), v, ps, c);
+    store4(a.pml.psi[I.lv] + base + i, ps, m);
+    store4(a.p[I.wn] + base + i, v, m);
 }
 
 // One launch over several PML boxes: a flat grid whose blocks are dealt to
@@ -2782,13 +2763,13 @@ void Engine::Impl::launch_step_t(int j, bool profile) {
         if (a.pml.width > 0) {
             if (ref()) {
                 if (sizeof(T) == 4 && nx > 4 && ny > 4 && nz > 4) {
-                    const dim3 grd((unsigned)((nx - 4 + 63) / 64), (unsigned)((ny - 4 + 3) / 4),
-                                   (unsigned)((nz - 4) * prm.batch));
+                    const int64_t units = (int64_t)((nx + 1) / 4) * (ny - 4);
+                    const dim3 grd((unsigned)((units + 255) / 256), (unsigned)((nz - 4) * prm.batch));
                     begin(KK_PML_AUX);
-                    k_pml_ref_aux<<<grd, blk, 0, stream>>>(a, j);
+                    k_pml_ref_aux<<<grd, 256, 0, stream>>>(a, j);
                     end();
                     begin(KK_PML_P);
-                    k_pml_ref_p<<<grd, blk, 0, stream>>>(a, j);
+                    k_pml_ref_p<<<grd, 256, 0, stream>>>(a, j);
                     end();
                     launches += 2;
                 }
