@@ -2499,10 +2499,22 @@ void Engine::Impl::ensure_receivers(int64_t t_end) {
         check_cell(r.data(), nx, ny, nz, "receiver");
         cell.push_back((int32_t)(r[2] * plane + r[1] * pitch + r[0]));
     }
-    int64_t cap = std::max<int64_t>(t_end, 1);
-    cap = std::max(cap, rcv_cap);
+    // Room for later runs as well (64 MB and 8192 steps at most): a longer
+    // record moves, and with it go the captured graphs, whose capture and
+    // instantiation cost 2 to 9 ms, as much as 20 to 80 steps.
+    const int64_t rows = (int64_t)prm.batch * std::max(nr, 1);
+    int64_t cap = std::max(std::max<int64_t>(t_end, 1), rcv_cap);
+    const int64_t room = cap > rcv_cap ? std::min<int64_t>(8192, ((int64_t)64 << 20) / (4 * rows)) : 0;
     DBuf<float> fresh;
-    fresh.alloc((size_t)prm.batch * std::max(nr, 1) * cap);
+    if (room > 0) {
+        try {
+            fresh.alloc((size_t)rows * (cap + room));
+            cap += room;
+        } catch (const Error&) {  // not that much memory left: the steps of this run alone
+            cudaGetLastError();
+        }
+    }
+    if (!fresh.ptr) fresh.alloc((size_t)rows * cap);
     if (rcv_out.ptr && rcv_cap > 0 && steps_done > 0) {
         // copy the rows of the receivers that existed before
         for (int32_t b = 0; b < prm.batch; ++b)

@@ -93,3 +93,32 @@ def test_resident_routes(pkg, mode, storage, form):
         sim.close()
     assert np.abs(out[0][0]).max() > 0
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+# the record's spare room (8192 steps) used up exactly, passed by one, and with
+# a receiver added on the way; every run against one run of the same length.
+# capture: the steps' own launches in graphs that outlive the runs
+@pytest.mark.parametrize("capture", [0, 5000])
+@pytest.mark.parametrize("runs", [[1, 8192, 1, 200], [100, 8093, 300], [300, 7]])
+def test_record_grows_over_runs(pkg, capture, runs):
+    dims = (20, 14, 12)
+    vox, a, b = room(*dims, 2, 3)
+    n = sum(runs)
+    sig = np.random.default_rng(8).standard_normal(n).astype(np.float32)
+    out = []
+    for steps in (runs, [n]):
+        sim = pkg.Simulation(mode=1, dx=0.02, c=340.0, dt=3.125e-5)
+        sim.SetModel(pkg.Model.from_voxels(vox, a, b))
+        sim.AddSourceCell((5, 6, 7), sig)
+        sim.AddMicCell((9, 9, 9))
+        if capture:
+            sim.set_capture(2, 6, capture)
+        for k, r in enumerate(steps):
+            if k == len(steps) - 1 and len(steps) > 1:
+                sim.AddMicCell((3, 2, 2))
+            sim.Run(r)
+        out.append((np.array(sim.mics()), np.array(sim.field())))
+        sim.close()
+    (m0, f0), (m1, f1) = out
+    assert m0.shape == (2, n) and np.array_equal(m0[0], m1[0]) and np.array_equal(f0, f1)
+    assert not m0[1, :n - runs[-1]].any()
