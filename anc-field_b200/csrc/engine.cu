@@ -651,6 +651,12 @@ __device__ __forceinline__ void pml_aux_unit(const StepArgs& a, int b, int x, in
 // as in FIXED mode: the kernels are bound by load instructions (every array of
 // a grid stays in L2), of which a thread per cell issued 60.
 //
+// The cells 2..nx-3 of unit x..x+3 as a mask.
+__device__ __forceinline__ unsigned ref_cells(const StepArgs& a, int x) {
+    unsigned m = x == 0 ? 12u : 15u;
+    if (x + 3 > a.g.nx - 3) m &= (1u << (a.g.nx - 2 - x)) - 1u;
+    return m;
+}
 // Unit u of plane z of the launch: cells x..x+3, valid ones as the mask m.
 __device__ __forceinline__ bool ref_unit(const StepArgs& a, int* b, int* x, int* y, int* z, unsigned* m) {
     const unsigned nu = (unsigned)(a.g.nx + 1) / 4;  // units that hold a cell 2..nx-3
@@ -661,9 +667,7 @@ __device__ __forceinline__ bool ref_unit(const StepArgs& a, int* b, int* x, int*
     *y = 2 + (int)row;
     *x = 4 * (int)(u - row * nu);
     if (*y > a.g.ny - 3) return false;
-    *m = 15u;
-    if (*x == 0) *m &= 12u;
-    if (*x + 3 > a.g.nx - 3) *m &= (1u << (a.g.nx - 2 - *x)) - 1u;
+    *m = ref_cells(a, *x);
     return true;
 }
 // axes whose slabs meet x0..x1, y0..y1, z0..z1
@@ -671,84 +675,6 @@ __device__ __forceinline__ unsigned ref_axes(const StepArgs& a, int x0, int x1, 
     const int W = a.pml.width;
     return (x0 < W || x1 > a.g.nx - W - 1 ? 1u : 0u) | (y0 < W || y1 > a.g.ny - W - 1 ? 2u : 0u) |
            (z0 < W || z1 > a.g.nz - W - 1 ? 4u : 0u);
-}
-
-// Auxiliary fields of pml.cl:231-262, with the reference's derivatives (their
-// last term reads p, pml.cl:126) and fi_y's psi coefficient (ksi_x at y,
-// pml.cl:247). The cell's own p and psi are the first of the four values of
-// its lower faces.
-__global__ void __launch_bounds__(256) k_pml_ref_aux(StepArgs a, int j) {
-    const StepIdx I = step_at(a, j);
-    const TlMark tl(a, 3, I.g, blockIdx.y < (unsigned)(a.g.nz - 4));
-    int b, x, y, z;
-    unsigned m;
-    if (!ref_unit(a, &b, &x, &y, &z, &m)) return;
-    const unsigned axes = ref_axes(a, x, x + 3, y, y, z, z);
-    if (!axes) return;
-    const PmlDev& P = a.pml;
-    const size_t base = (size_t)b * a.g.vol;
-    const int pitch = (int)a.g.pitch, plane = (int)a.g.plane, i = z * plane + y * pitch + x;
-    const bool hi = x + 4 < pitch;
-    const LevelScales sc = level_scales<float>(a, b, I.s5);
-    float own[4], ps[4], m00[5];
-    pml_p_calc<true, float, true>(a, base, x, y, z, I, sc, ref_axes(a, x, x + 4, y, y + 1, z, z + 1), own, ps, m00);
-    const float *pn = a.p[I.wn] + base, *pc = a.p[I.wc] + base, *sp = P.psi[I.lv] + base;
-    float n00[5], n01[5], n10[5], n11[5], m01[5], m10[5], m11[5], s00[5], s01[5], s10[5], s11[5];
-    row5(pn + i, n00, hi);
-    row5(pn + (i + plane), n01, hi);
-    row5(pn + (i + pitch), n10, hi);
-    row5(pn + (i + pitch + plane), n11, hi);
-    row5(pc + (i + plane), m01, hi);
-    row5(pc + (i + pitch), m10, hi);
-    row5(pc + (i + pitch + plane), m11, hi);
-    row5(sp + i, s00, hi);
-    row5(sp + (i + plane), s01, hi);
-    row5(sp + (i + pitch), s10, hi);
-    row5(sp + (i + pitch + plane), s11, hi);
-    float kxs[5];
-    row5(P.ksi[0] + x, kxs, hi);
-    const float kay = 0.5f * (__ldg(P.ksi[1] + y) + __ldg(P.ksi[1] + y + 1));
-    const float kaz = 0.5f * (__ldg(P.ksi[2] + z) + __ldg(P.ksi[2] + z + 1));
-    const float kxy = 0.5f * (__ldg(P.ksi[0] + y) + __ldg(P.ksi[0] + y + 1));
-    auto field = [&](auto axis, unsigned cells) {
-        constexpr int AX = decltype(axis)::value;
-        const float4 f14 = *reinterpret_cast<const float4*>(P.fi[AX][I.lv ^ 1] + base + i);
-        const float f1[4] = {f14.x, f14.y, f14.z, f14.w};
-        float out[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            float nh, nl, mh, ml, sh, sl;
-            face_ends<AX>(n00, n01, n10, n11, q, &nh, &nl);
-            face_ends<AX>(m00, m01, m10, m11, q, &mh, &ml);
-            face_ends<AX>(s00, s01, s10, s11, q, &sh, &sl);
-            // the lower faces with the cell's own new values
-            if constexpr (AX == 0) {
-                nl = face4(own[q], n01[q], n10[q], n11[q]);
-                sl = face4(ps[q], s01[q], s10[q], s11[q]);
-            } else if constexpr (AX == 1) {
-                nl = face4(own[q], n01[q], n00[q + 1], n01[q + 1]);
-                sl = face4(ps[q], s01[q], s00[q + 1], s01[q + 1]);
-            } else {
-                nl = face4(own[q], n10[q], n00[q + 1], n10[q + 1]);
-                sl = face4(ps[q], s10[q], s00[q + 1], s10[q + 1]);
-            }
-            const float dp = P.half_inv_dx * (nh - nl + mh - nl), dpsi = P.inv_dx * (sh - sl);
-            const float kax = 0.5f * (kxs[q] + kxs[q + 1]);
-            const float k1 = AX == 0 ? kay : kax, k2 = AX == 2 ? kay : kaz;
-            out[q] = pml_aux_cell(P, f1[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), k1, k2, dp,
-                                  AX == 1 ? kxy * kaz : k1 * k2, dpsi, [](float n, float den) { return n / den; });
-        }
-        store4(P.fi[AX][I.lv] + base + i, out, cells);
-    };
-    if (axes & 1u) {
-        unsigned cells = 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (x + q < P.width || x + q > a.g.nx - P.width - 1) cells |= 1u << q;
-        field(std::integral_constant<int, 0>{}, m & cells);
-    }
-    if (axes & 2u) field(std::integral_constant<int, 1>{}, m);
-    if (axes & 4u) field(std::integral_constant<int, 2>{}, m);
 }
 
 // Pressure and psi of every cell 2..n-3 (pml.cl:182-207).
@@ -822,6 +748,87 @@ __global__ void __launch_bounds__(256, 3) k_pml_p_all(const __grid_constant__ St
     const LevelScales sc = level_scales<T>(a, t.b, I.s5);
 #pragma unroll 1
     for (int z = t.z0; z < t.z1; ++z) pml_p_unit<PSI, T>(a, t.b, t.x, t.y, z, I, sc);
+}
+
+// Auxiliary fields of pml.cl:231-262, with the reference's derivatives (their
+// last term reads p, pml.cl:126) and fi_y's psi coefficient (ksi_x at y,
+// pml.cl:247). The cell's own p and psi are the first of the four values of
+// its lower faces. The launch covers the slabs' units with boxes: as one flat
+// grid over all units, two thirds of the warps held a few slab units each and
+// the pass took 24 us at 160x120x100.
+__global__ void __launch_bounds__(256) k_pml_ref_aux(const __grid_constant__ StepArgs a,
+                                                     const __grid_constant__ BoxLaunch L, int j) {
+    const StepIdx I = step_at(a, j);
+    const BoxThread t = box_thread(L);
+    const TlMark tl(a, 3, I.g, t.b == 0);
+    if (!t.ok) return;
+    const int b = t.b, x = t.x, y = t.y, z = t.z0;
+    const unsigned m = ref_cells(a, x), axes = ref_axes(a, x, x + 3, y, y, z, z);
+    if (!axes) return;
+    const PmlDev& P = a.pml;
+    const size_t base = (size_t)b * a.g.vol;
+    const int pitch = (int)a.g.pitch, plane = (int)a.g.plane, i = z * plane + y * pitch + x;
+    const bool hi = x + 4 < pitch;
+    const LevelScales sc = level_scales<float>(a, b, I.s5);
+    float own[4], ps[4], m00[5];
+    pml_p_calc<true, float, true>(a, base, x, y, z, I, sc, ref_axes(a, x, x + 4, y, y + 1, z, z + 1), own, ps, m00);
+    const float *pn = a.p[I.wn] + base, *pc = a.p[I.wc] + base, *sp = P.psi[I.lv] + base;
+    float n00[5], n01[5], n10[5], n11[5], m01[5], m10[5], m11[5], s00[5], s01[5], s10[5], s11[5];
+    row5(pn + i, n00, hi);
+    row5(pn + (i + plane), n01, hi);
+    row5(pn + (i + pitch), n10, hi);
+    row5(pn + (i + pitch + plane), n11, hi);
+    row5(pc + (i + plane), m01, hi);
+    row5(pc + (i + pitch), m10, hi);
+    row5(pc + (i + pitch + plane), m11, hi);
+    row5(sp + i, s00, hi);
+    row5(sp + (i + plane), s01, hi);
+    row5(sp + (i + pitch), s10, hi);
+    row5(sp + (i + pitch + plane), s11, hi);
+    float kxs[5];
+    row5(P.ksi[0] + x, kxs, hi);
+    const float kay = 0.5f * (__ldg(P.ksi[1] + y) + __ldg(P.ksi[1] + y + 1));
+    const float kaz = 0.5f * (__ldg(P.ksi[2] + z) + __ldg(P.ksi[2] + z + 1));
+    const float kxy = 0.5f * (__ldg(P.ksi[0] + y) + __ldg(P.ksi[0] + y + 1));
+    auto field = [&](auto axis, unsigned cells) {
+        constexpr int AX = decltype(axis)::value;
+        const float4 f14 = *reinterpret_cast<const float4*>(P.fi[AX][I.lv ^ 1] + base + i);
+        const float f1[4] = {f14.x, f14.y, f14.z, f14.w};
+        float out[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float nh, nl, mh, ml, sh, sl;
+            face_ends<AX>(n00, n01, n10, n11, q, &nh, &nl);
+            face_ends<AX>(m00, m01, m10, m11, q, &mh, &ml);
+            face_ends<AX>(s00, s01, s10, s11, q, &sh, &sl);
+            // the lower faces with the cell's own new values
+            if constexpr (AX == 0) {
+                nl = face4(own[q], n01[q], n10[q], n11[q]);
+                sl = face4(ps[q], s01[q], s10[q], s11[q]);
+            } else if constexpr (AX == 1) {
+                nl = face4(own[q], n01[q], n00[q + 1], n01[q + 1]);
+                sl = face4(ps[q], s01[q], s00[q + 1], s01[q + 1]);
+            } else {
+                nl = face4(own[q], n10[q], n00[q + 1], n10[q + 1]);
+                sl = face4(ps[q], s10[q], s00[q + 1], s10[q + 1]);
+            }
+            const float dp = P.half_inv_dx * (nh - nl + mh - nl), dpsi = P.inv_dx * (sh - sl);
+            const float kax = 0.5f * (kxs[q] + kxs[q + 1]);
+            const float k1 = AX == 0 ? kay : kax, k2 = AX == 2 ? kay : kaz;
+            out[q] = pml_aux_cell(P, f1[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), k1, k2, dp,
+                                  AX == 1 ? kxy * kaz : k1 * k2, dpsi, [](float n, float den) { return n / den; });
+        }
+        store4(P.fi[AX][I.lv] + base + i, out, cells);
+    };
+    if (axes & 1u) {
+        unsigned cells = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (x + q < P.width || x + q > a.g.nx - P.width - 1) cells |= 1u << q;
+        field(std::integral_constant<int, 0>{}, m & cells);
+    }
+    if (axes & 2u) field(std::integral_constant<int, 1>{}, m);
+    if (axes & 4u) field(std::integral_constant<int, 2>{}, m);
 }
 
 // The auxiliary fields of every (axis, slab box) pair in one launch: the
@@ -2116,7 +2123,7 @@ void Engine::Impl::build_fused() {
 // min(units, 32) units across, zc planes per thread; *blocks receives the
 // grid size.
 static BoxLaunch make_box_launch(const std::vector<std::pair<PmlBox, int>>& entries, int batch, int zc,
-                                 int* blocks) {
+                                 int* blocks, int max_w = 32) {
     if ((int)entries.size() > kMaxLaunchBoxes) throw Error(AFD_ERR_ARG, "too many PML boxes for one launch");
     BoxLaunch L{};
     L.n = (int32_t)entries.size();
@@ -2124,7 +2131,7 @@ static BoxLaunch make_box_launch(const std::vector<std::pair<PmlBox, int>>& entr
     int64_t start = 0;
     for (size_t k = 0; k < entries.size(); ++k) {
         const PmlBox& bx = entries[k].first;
-        const int w = std::min(bx.units, 32), rows = 256 / w;
+        const int w = std::min(bx.units, max_w), rows = 256 / w;
         L.box[k] = bx;
         L.axis[k] = entries[k].second;
         L.w[k] = w;
@@ -2175,6 +2182,31 @@ void Engine::Impl::setup_pml() {
         std::vector<float> k((size_t)kmax, 0.0f);
         for (int32_t i = 0; i < dims[a] && i < (int32_t)ksi[a].size(); ++i) k[(size_t)i] = ksi[a][(size_t)i];
         ksi_dev[a].upload(k);
+    }
+    if (ref() && nx > 4 && ny > 4 && nz > 4) {
+        // REF: the units of the cells 2..n-3 that lie in a slab, z slabs first
+        const int W = pml_width, units = (nx + 1) / 4;
+        std::vector<std::pair<PmlBox, int>> e;
+        auto add = [&](int u0, int u1, int y0, int y1, int z0, int z1) {  // inclusive
+            if (u0 > u1 || y0 > y1 || z0 > z1) return;
+            e.emplace_back(PmlBox{4 * u0, u1 - u0 + 1, y0, y1 - y0 + 1, z0, z1 - z0 + 1, 0}, 0);
+        };
+        // last cell of the lower slab, first of the upper one (2..n-3, disjoint)
+        auto ends = [&](int n, int* lo, int* hi) {
+            *lo = std::min(std::max(W - 1, 1), n - 3);
+            *hi = std::min(std::max(n - W, *lo + 1), n - 2);
+        };
+        int ly, hy, lz, hz;
+        ends(ny, &ly, &hy);
+        ends(nz, &lz, &hz);
+        add(0, units - 1, 2, ny - 3, 2, lz);
+        add(0, units - 1, 2, ny - 3, hz, nz - 3);
+        add(0, units - 1, 2, ly, lz + 1, hz - 1);
+        add(0, units - 1, hy, ny - 3, lz + 1, hz - 1);
+        const int lu = W > 2 ? std::min((W - 1) / 4, units - 1) : -1, hu = std::max(std::max(nx - W, 0) / 4, lu + 1);
+        add(0, lu, ly + 1, hy - 1, lz + 1, hz - 1);
+        add(hu, units - 1, ly + 1, hy - 1, lz + 1, hz - 1);
+        pml_aux_all = make_box_launch(e, prm.batch, 1, &pml_aux_blocks, 256);
     }
     if (!ref()) {
         // FIXED: PML cells are the plain air cells (not solid, not boundary)
@@ -2778,7 +2810,7 @@ void Engine::Impl::launch_step_t(int j, bool profile) {
                     const int64_t units = (int64_t)((nx + 1) / 4) * (ny - 4);
                     const dim3 grd((unsigned)((units + 255) / 256), (unsigned)((nz - 4) * prm.batch));
                     begin(KK_PML_AUX);
-                    k_pml_ref_aux<<<grd, 256, 0, stream>>>(a, j);
+                    if (pml_aux_blocks > 0) k_pml_ref_aux<<<pml_aux_blocks, 256, 0, stream>>>(a, pml_aux_all, j);
                     end();
                     begin(KK_PML_P);
                     k_pml_ref_p<<<grd, 256, 0, stream>>>(a, j);
