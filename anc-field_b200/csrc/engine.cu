@@ -5,8 +5,11 @@
 // LRS groups, the PML kernel, source and mic. Here a step is
 //   fused:   the streaming interior kernel (k_stream, TMA z-marching), then
 //            the boundary list and, in FIXED mode, the PML pressure boxes
-//            (side by side inside a CUDA graph), the per-axis PML auxiliary
-//            updates and the source/receiver kernel;
+//            (side by side inside a CUDA graph) and the per-axis PML auxiliary
+//            updates; the boundary kernel takes the sources and receivers, or
+//            a kernel of their own follows;
+//   resident: all of a chunk's steps in one cooperative kernel, for grids
+//            that stay in L2 (roles.cuh);
 //   unfused: one-thread-per-cell interior kernel, boundary, PML and
 //            source/receiver kernels in turn.
 // REF mode with a PML runs the reference's PML order (k_pml_ref_*), because

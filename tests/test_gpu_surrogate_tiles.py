@@ -76,3 +76,22 @@ def test_training_step_of_all_layers(pkg, freq, hidden, layers, out, batch, n):
             assert rel(m.get(S.GRAD_WEIGHT, l), want[l][0]) < 2 * layers * 2.0 ** -8
             assert rel(m.get(S.GRAD_BIAS, l), want[l][1]) < 2 * layers * 2.0 ** -8
     m.close()
+
+
+def test_split_product_in_a_cuda_graph(pkg):
+    """The cluster launch of a split product captured and replayed: the bits
+    of the plain call."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a = torch.randn(128, 8192, device="cuda", generator=g).to(torch.bfloat16)
+    b = torch.randn(128, 8192, device="cuda", generator=g).to(torch.bfloat16)
+    c, want = torch.zeros(128, 128, device="cuda"), torch.zeros(128, 128, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pkg.surrogate.gemm_bf16(a, b, want, torch.cuda.current_stream().cuda_stream)
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        with torch.cuda.graph(graph, stream=s):
+            pkg.surrogate.gemm_bf16_async(a, b, c, status, s.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and torch.equal(c, want)
