@@ -588,6 +588,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tile(const __grid_cons
     const int m0 = t % tiles_m * TM, n0 = t / tiles_m * TN_;
     const int KT = (g.K / TK + 1) / 2;  // two column blocks a step; the last one's second may be zero fill
     const int kb = (int)((int64_t)KT * part / split), ke = (int)((int64_t)KT * (part + 1) / split);
+    tc::launch_dependents();
     if (threadIdx.x == 0) {
         for (int i = 0; i < NS; ++i) {
             tc::bar_init(&full[i], 1);
@@ -601,6 +602,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tile(const __grid_cons
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *tslot;
+    tc::wait_previous();
     const int q = warp & 3;
     bool ok = true;
 
@@ -722,14 +724,17 @@ struct alignas(16) SquareTile {
 };
 
 // Fourier features: f[r][j] = sin(2 pi <x_r, B_j>) (j < n_freq) and the
-// cosine at j + n_freq; rows r >= n are zero. Block: 64 rows, 32 frequencies
-// (columns 0..31 of the tile the sines, 32..63 the cosines).
+// cosine at j + n_freq; rows r >= n are zero. Block: 16 rows, 32 frequencies
+// (columns 0..31 of the tile the sines, 32..63 the cosines); with 64 rows a
+// block 64 blocks of 1024 rows took 9.5 us.
+constexpr int kFourierRows = 16;
 __global__ void __launch_bounds__(256) k_fourier(const float* x, int n, int n_in, const float* Bf, int n_freq,
                                                  int rows, bf16* f, bf16* ft) {
-    __shared__ SquareTile t;
-    const int r0 = blockIdx.x * SQ, j0 = blockIdx.y * 32, F = 2 * n_freq;
+    __shared__ alignas(16) bf16 t[kFourierRows][SQ + 2];
+    const int r0 = blockIdx.x * kFourierRows, j0 = blockIdx.y * 32, F = 2 * n_freq;
     const int jj = threadIdx.x & 31;
-    for (int rr = threadIdx.x >> 5; rr < SQ; rr += 8) {
+    tc::launch_dependents();
+    for (int rr = threadIdx.x >> 5; rr < kFourierRows; rr += 8) {
         const int r = r0 + rr, j = j0 + jj;
         float s = 0.0f, c = 0.0f;
         if (r < n) {
@@ -739,16 +744,16 @@ __global__ void __launch_bounds__(256) k_fourier(const float* x, int n, int n_in
             s = sinf(ph);
             c = cosf(ph);
         }
-        t.v[rr][jj] = __float2bfloat16_rn(s);
-        t.v[rr][32 + jj] = __float2bfloat16_rn(c);
-        f[(size_t)r * F + j] = t.v[rr][jj];
-        f[(size_t)r * F + j + n_freq] = t.v[rr][32 + jj];
+        t[rr][jj] = __float2bfloat16_rn(s);
+        t[rr][32 + jj] = __float2bfloat16_rn(c);
+        f[(size_t)r * F + j] = t[rr][jj];
+        f[(size_t)r * F + j + n_freq] = t[rr][32 + jj];
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < SQ * SQ / 2; k += 256) {
-        const int c = k / (SQ / 2), r = k % (SQ / 2) * 2;
+    for (int k = threadIdx.x; k < SQ * kFourierRows / 2; k += 256) {
+        const int c = k / (kFourierRows / 2), r = k % (kFourierRows / 2) * 2;
         const int row = c < 32 ? j0 + c : n_freq + j0 + c - 32;
-        *reinterpret_cast<__nv_bfloat162*>(ft + (size_t)row * rows + r0 + r) = __nv_bfloat162(t.v[r][c], t.v[r + 1][c]);
+        *reinterpret_cast<__nv_bfloat162*>(ft + (size_t)row * rows + r0 + r) = __nv_bfloat162(t[r][c], t[r + 1][c]);
     }
 }
 
@@ -761,6 +766,8 @@ __global__ void __launch_bounds__(256) k_mse_grad(const float* pred, const float
     __shared__ float part[8];
     const int c0 = blockIdx.x * SQ, r0 = blockIdx.y * SQ;
     const int c = threadIdx.x % 16 * 4;
+    tc::launch_dependents();
+    tc::wait_previous();
     float sq = 0.0f;
 #pragma unroll
     for (int rr = threadIdx.x / 16; rr < SQ; rr += 16) {
@@ -813,7 +820,9 @@ struct Layers {
 __global__ void k_bias_grad(const __grid_constant__ Layers a) {
     const int w = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
+    tc::launch_dependents();
     if (w >= a.total) return;
+    tc::wait_previous();
     int k = 0, o = w;
     while (o >= a.l[k].out) o -= a.l[k++].out;
     const bf16* dt = a.l[k].gt + (size_t)o * a.rows;
@@ -843,6 +852,7 @@ __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ Layers a, 
     while (k + 1 < a.n && (int)blockIdx.x >= a.l[k + 1].first) ++k;
     const LayerDev& L = a.l[k];
     const int tile = (int)blockIdx.x - L.first, tx = L.in / SQ, tiles = tx * (L.out / SQ);
+    tc::wait_previous();
     if (tile >= tiles) {
         const int i = (tile - tiles) * 256 + (int)threadIdx.x;
         if (i < L.out) L.b[i] = step(L.b[i], L.gb[i], L.mb + i, L.vb + i);
@@ -1067,26 +1077,42 @@ static int set_smem_attr() {
     return d.sms;
 }
 
-template <int TN_, int NG>
-static void launch_tiles(const GemmGroup<NG>& gg, int tiles, int split, cudaStream_t st) {
+// A launch that may start before the stream's previous kernel has ended, for
+// the network's kernels, which wait for it themselves (wait_previous): a
+// training step is a chain of kernels of 5 to 14 us (135 -> 100 us a step at
+// 1024 rows, 512 wide). split > 1: clusters of that
+// many CTAs along y. Calls of a single GEMM start after what the stream holds.
+template <typename... P, typename... A>
+static void launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, int split,
+                         bool early, const A&... args) {
     cudaLaunchConfig_t c{};
-    c.gridDim = dim3((unsigned)tiles, (unsigned)split);
-    c.blockDim = dim3(GEMM_THREADS);
-    c.dynamicSmemBytes = Tile<TN_>::smem;
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
     c.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 1;
-    at.val.clusterDim.y = (unsigned)split;
-    at.val.clusterDim.z = 1;
-    c.attrs = &at;
-    c.numAttrs = split > 1 ? 1 : 0;
-    MCK(cudaLaunchKernelEx(&c, k_gemm_tile<TN_, NG>, gg));
+    cudaLaunchAttribute at[2]{};
+    if (early) {
+        at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[c.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (split > 1) {
+        at[c.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[c.numAttrs].val.clusterDim.x = 1;
+        at[c.numAttrs].val.clusterDim.y = (unsigned)split;
+        at[c.numAttrs++].val.clusterDim.z = 1;
+    }
+    c.attrs = at;
+    MCK(cudaLaunchKernelEx(&c, kernel, args...));
+}
+template <int TN_, int NG>
+static void launch_tiles(const GemmGroup<NG>& gg, int tiles, int split, bool early, cudaStream_t st) {
+    launch_after(k_gemm_tile<TN_, NG>, dim3((unsigned)tiles, (unsigned)split), GEMM_THREADS, Tile<TN_>::smem, st, split,
+                 early, gg);
 }
 
 // The GEMMs of `v` (n <= NG, all planned with the same tile columns) in one launch.
 template <int NG>
-static void launch_group(const Gemm* v, int n, cudaStream_t st) {
+static void launch_group(const Gemm* v, int n, cudaStream_t st, bool early) {
     GemmGroup<NG> gg;
     gg.n = n;
     const int tn = v[0].plan.form;
@@ -1100,12 +1126,12 @@ static void launch_group(const Gemm* v, int n, cudaStream_t st) {
         tiles += (v[i].o.M / TM) * (v[i].o.N / tn);
     }
     const int split = NG == 1 ? v[0].plan.split : 1;
-    if (tn == 128) launch_tiles<128, NG>(gg, tiles, split, st);
-    else if (tn == 64) launch_tiles<64, NG>(gg, tiles, split, st);
-    else launch_tiles<32, NG>(gg, tiles, split, st);
+    if (tn == 128) launch_tiles<128, NG>(gg, tiles, split, early, st);
+    else if (tn == 64) launch_tiles<64, NG>(gg, tiles, split, early, st);
+    else launch_tiles<32, NG>(gg, tiles, split, early, st);
 }
 
-static void launch(const Gemm& G, cudaStream_t st) {
+static void launch(const Gemm& G, cudaStream_t st, bool early = false) {
     const int sms = set_smem_attr();
     if (G.plan.form == kPair) {
         const int tiles = (G.o.M / (2 * TM)) * (G.o.N / PTN);
@@ -1131,7 +1157,7 @@ static void launch(const Gemm& G, cudaStream_t st) {
             default: k_gemm<EPI_MASK><<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(G.ta, G.tb, G.o); break;
         }
     } else {
-        launch_group<1>(&G, 1, st);
+        launch_group<1>(&G, 1, st, early);
     }
     MCK(cudaGetLastError());
 }
@@ -1336,13 +1362,13 @@ struct afd_mlp {
     void features(const float* x_dev, int n) {
         if (n < 1 || n > rows) throw Err(AFD_ERR_ARG, "row count outside 1..batch");
         MCK(cudaMemcpyAsync(xin.p, x_dev, (size_t)n * prm.n_in * 4, cudaMemcpyDefault, stream));
-        const dim3 grd((unsigned)(rows / SQ), (unsigned)(prm.n_freq / 32));
+        const dim3 grd((unsigned)(rows / kFourierRows), (unsigned)(prm.n_freq / 32));
         k_fourier<<<grd, 256, 0, stream>>>(xin.p, n, prm.n_in, fourier.p, prm.n_freq, rows, feat.p, featT.p);
         MCK(cudaGetLastError());
     }
 
     void forward() {
-        for (auto& g : fwd) launch(g, stream);
+        for (auto& g : fwd) launch(g, stream, true);
     }
 
     void backward(const float* y_dev, int n) {
@@ -1351,16 +1377,14 @@ struct afd_mlp {
         const int nl = prm.n_layers;
         const float scale = 2.0f / ((float)n * (float)prm.n_out);
         const dim3 grd((unsigned)(prm.n_out / SQ), (unsigned)(rows / SQ));
-        k_mse_grad<<<grd, 256, 0, stream>>>(pred.p, yin.p, n, prm.n_out, rows, scale, G[(size_t)nl - 1]->p,
-                                            GT[(size_t)nl - 1]->p, loss.p);
-        MCK(cudaGetLastError());
+        launch_after(k_mse_grad, grd, 256, 0, stream, 1, true, (const float*)pred.p, (const float*)yin.p, n, (int)prm.n_out,
+                     rows, scale, G[(size_t)nl - 1]->p, GT[(size_t)nl - 1]->p, loss.p);
         for (int l = nl - 1; l >= 0; --l) {
-            if (!group_w) launch(bwd_w[(size_t)l], stream);
-            if (l > 0) launch(bwd_x[(size_t)l - 1], stream);
+            if (!group_w) launch(bwd_w[(size_t)l], stream, true);
+            if (l > 0) launch(bwd_x[(size_t)l - 1], stream, true);
         }
-        if (group_w) launch_group<kMaxLayers>(bwd_w.data(), nl, stream);
-        k_bias_grad<<<(unsigned)((bias_dev.total + 7) / 8), 256, 0, stream>>>(bias_dev);
-        MCK(cudaGetLastError());
+        if (group_w) launch_group<kMaxLayers>(bwd_w.data(), nl, stream, true);
+        launch_after(k_bias_grad, dim3((unsigned)((bias_dev.total + 7) / 8)), 256, 0, stream, 1, true, bias_dev);
     }
 
     void adam() {
@@ -1368,8 +1392,8 @@ struct afd_mlp {
         const float b1 = prm.beta1, b2 = prm.beta2;
         const float c1 = 1.0f - (float)std::pow((double)b1, (double)step);
         const float c2 = 1.0f - (float)std::pow((double)b2, (double)step);
-        k_adam<<<(unsigned)adam_dev.total, 256, 0, stream>>>(adam_dev, AdamStep{prm.lr, b1, b2, prm.eps, c1, c2});
-        MCK(cudaGetLastError());
+        launch_after(k_adam, dim3((unsigned)adam_dev.total), 256, 0, stream, 1, true, adam_dev,
+                     AdamStep{prm.lr, b1, b2, prm.eps, c1, c2});
     }
 };
 

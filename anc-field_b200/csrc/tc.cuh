@@ -79,6 +79,12 @@ __device__ __forceinline__ bool elect() {
     return p != 0;
 }
 
+// Programmatic dependent launch: lets the stream's next kernel start its own
+// set-up now, and waits for everything the stream's previous kernels wrote
+// (before any read or write of what they share).
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // 3-D tiled TMA load into shared memory (64 elements from x = 0, rows from y,
 // 64-element column blocks from z), completing on an mbarrier.
 __device__ __forceinline__ void tma_3d(void* dst, const CUtensorMap* map, int y, int z, uint64_t* b) {

@@ -95,3 +95,26 @@ def test_split_product_in_a_cuda_graph(pkg):
     graph.replay()
     torch.cuda.synchronize()
     assert int(status.item()) == 0 and torch.equal(c, want)
+
+
+# grouped and single weight gradients; the chain of early launches against
+# steps that end before the next begins: the same kernels, so the same bits
+@pytest.mark.parametrize("hidden,out,batch", [(128, 128, 128), (512, 2048, 1024), (1024, 4096, 1024)])
+def test_queued_steps_equal_single_steps(pkg, hidden, out, batch):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.rand(3 * batch, 10, device="cuda", generator=g)
+    y = 0.3 * torch.randn(3 * batch, out, device="cuda", generator=g)
+    torch.cuda.synchronize()
+    kept = []
+    for queued in (True, True, False):
+        m = pkg.surrogate.Mlp(n_in=10, n_freq=64, hidden=hidden, n_layers=4, n_out=out, batch=batch, seed=2)
+        for k in range(24):
+            at = k % 3 * batch
+            m.train_step(x[at:at + batch], y[at:at + batch], want_loss=False)
+            if not queued:
+                m.sync()
+        kept.append(m.weights())
+        m.close()
+    for other in kept[1:]:
+        assert all(np.array_equal(a, b) for p, q in zip(kept[0], other) for a, b in zip(p, q))
