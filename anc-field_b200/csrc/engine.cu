@@ -1515,14 +1515,15 @@ struct Source {
 
 // Source cells that the step's own kernels take (one block's table).
 constexpr int kMaxSrcCells = 256;
-// Cells (all members) up to which the resident kernel runs. Against replayed
-// launches it measured (us a step; FP32 without a PML, FP32 with six PML
-// faces, FP16 with two): 5.1 / 14.5 / 13.7 to 10.3 / 20.6 / 19.2 at 0.04 M
-// cells, 10.0 / 21.2 / 16.5 to 12.1 / 27.7 / 22.4 at 0.74 M, 15.0 / 28.7 / 19.4
-// to 15.3 / 43.5 / 28.2 at 1.85 M, 24.9 / 58.3 / 34.1 to 25.0 / 73.6 / 40.3 at
-// 5.0 M, and 42.2 / 79.8 / 45.7 to 33.8 / 90.8 / 48.2 at 8.2 M, where the
-// streaming kernel's TMA tiles beat the columns of plain loads.
-constexpr int64_t kResidentCells = 5 << 20;
+// Cells (all members, rows as padded) up to which the resident kernel runs.
+// Against replayed launches it measured (us a step; FP32 without a PML, FP32
+// with six PML faces, FP16 with two): 5.2 / 14.2 / 13.5 to 10.3 / 20.6 / 19.2 at
+// 0.06 M cells, 7.6 / 20.3 / 15.5 to 12.1 / 27.7 / 22.4 at 0.94 M, 13.8 / 27.0 /
+// 21.2 to 15.3 / 43.5 / 28.2 at 2.1 M, 24.9 / 58.3 / 34.1 to 25.0 / 73.6 / 40.3
+// at 5.6 M (26.1 in another form of the dealing), and 42.2 / 79.8 / 45.7 to 33.8
+// / 90.8 / 48.2 at 8.7 M, where the streaming kernel's TMA tiles beat the
+// columns of plain loads; with a PML, whose launches it saves, the lines cross later.
+constexpr int64_t kResidentCells = 5 << 20, kResidentCellsPml = 6 << 20;
 
 struct Engine::Impl {
     afd_params prm{};
@@ -1680,7 +1681,8 @@ struct Engine::Impl {
     // unless a plan is forced or a capture or timeline needs the step's own
     // launches.
     bool resident() const {
-        return sr_active() && !forced && cap_every <= 0 && tl_steps <= 0 && vol * prm.batch <= kResidentCells;
+        return sr_active() && !forced && cap_every <= 0 && tl_steps <= 0 &&
+               vol * prm.batch <= (pml_fixed() ? kResidentCellsPml : kResidentCells);
     }
     void build_resident();
     template <typename T>
@@ -2381,7 +2383,9 @@ void Engine::Impl::upload_source_cells(const std::vector<int32_t>& cell, const s
 
 // The resident kernel's work: how the PML units, boundary entries and interior
 // columns of a step's first phase are dealt to its groups. Costs are per 256
-// of each, in units of one interior plane of 256 columns.
+// of each, in units of one interior plane of 256 columns (boundary 3 and PML 4
+// gave 10.5 us a step instead of 7.6 at 100x92x80 and 16.1 instead of 15.0 at
+// 160x120x100 with a PML face; 5 and 5, 6 and 6 were slower there too).
 void Engine::Impl::build_resident() {
     const bool pml = pml_fixed();
     int sms = 0;
@@ -2391,7 +2395,7 @@ void Engine::Impl::build_resident() {
     R = ResidentDev{};
     R.nu = (nx - 2) / 4 + 1;
     R.ncol = R.nu * (ny - 2);
-    const double c_plane = 1.0, c_item = 1.0, c_lrs = 3.0, c_pml = 4.0;
+    const double c_plane = 1.0, c_item = 1.0, c_lrs = 4.0, c_pml = 6.0;
     const int64_t lrs = (int64_t)lrs_cell.n * prm.batch, planes = nz - 2, units = pml ? pml_units * prm.batch : 0;
     const double fixed = (lrs + 255) / 256 * c_lrs + (units + 255) / 256 * c_pml;
     // columns of zc planes: about one item per thread of the remaining groups

@@ -14,7 +14,7 @@
 // sources and receivers 3.0. So what does not change from step to step is kept
 // in registers across them (the first boundary entry of a thread, the rotating
 // indices) and the items are found without divisions. A step measured 4.9 us
-// for 28x22x18 (13.5 as launches), 15.7 for 160x120x100 with one PML face (20)
+// for 28x22x18 (13.5 as launches), 15.0 for 160x120x100 with one PML face (20)
 // and 48.8 for 204x157x131 with six (62).
 #pragma once
 
