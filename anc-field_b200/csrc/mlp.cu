@@ -236,17 +236,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2)
     }
 }
 
-// Output tile t of the persistent form: groups of 16 row panels, columns
-// outer inside a group, so that the ~148 tiles in flight share their A and
-// B panels in L2.
+// Output tile t of the persistent forms and of the tile form: groups of 16 row
+// panels, columns outer inside a group, so that the ~148 tiles in flight share
+// their A and B panels in L2 whichever operand is the long one (with the tile
+// form's tiles in plain column order every column of tiles read a tall A again:
+// 11008x640x10752 175 us, 148 this way; 10880x896x12288 305 and 262).
 constexpr int RASTER_M = 16;
-__device__ __forceinline__ void tile_of(int t, int tiles_m, int tiles_n, int tile_h, int& m0, int& n0) {
+__device__ __forceinline__ void tile_of(int t, int tiles_m, int tiles_n, int tile_h, int tile_w, int& m0, int& n0) {
     const int per_group = RASTER_M * tiles_n;
     const int first = (t / per_group) * RASTER_M;
     const int gm = min(tiles_m - first, RASTER_M);
     const int w = t % per_group;
     m0 = (first + w % gm) * tile_h;
-    n0 = (w / gm) * PTN;
+    n0 = (w / gm) * tile_w;
 }
 
 // Persistent form, one CTA per SM (194 KB of shared memory, all 512 TMEM
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             bool ok = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 int m0, n0;
-                tile_of(t, tiles_m, tiles_n, TM, m0, n0);
+                tile_of(t, tiles_m, tiles_n, TM, PTN, m0, n0);
                 for (int kt = 0; kt < KT; ++kt, ++u) {
                     const uint32_t s = u % PNST;
                     if (u >= (uint32_t)PNST && !tc::bar_wait_warp(&empty[s], ((u / PNST) - 1) & 1)) {
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             tc::fence_after();
             int m0, n0;
-            tile_of(t, tiles_m, tiles_n, TM, m0, n0);
+            tile_of(t, tiles_m, tiles_n, TM, PTN, m0, n0);
             const int row = m0 + 32 * q + lane;
 #pragma unroll 1
             for (int c = 0; c < PTN / 32; ++c) {
@@ -436,7 +438,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
             bool ok = true;
             for (int t = pair; t < tiles && ok; t += pairs) {
                 int m0, n0;
-                tile_of(t, tiles_m, tiles_n, 2 * TM, m0, n0);
+                tile_of(t, tiles_m, tiles_n, 2 * TM, PTN, m0, n0);
                 const int am = m0 + (int)rank * TM, bn = n0 + (int)rank * TN;
                 for (int kt = 0; kt < KT; ++kt, ++u) {
                     const uint32_t s = u % QNST;
@@ -511,7 +513,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
             }
             tc::fence_after();
             int m0, n0;
-            tile_of(t, tiles_m, tiles_n, 2 * TM, m0, n0);
+            tile_of(t, tiles_m, tiles_n, 2 * TM, PTN, m0, n0);
             const int row = m0 + (int)rank * TM + 32 * q + lane;
 #pragma unroll 1
             for (int c = 0; c < PTN / 32; ++c) {
@@ -584,8 +586,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm_tile(const __grid_cons
         while (at + 1 < gg.n && (int)blockIdx.x >= gg.g[at + 1].first) ++at;
     const GemmItem& G = gg.g[at];
     const GemmOut& g = G.o;
-    const int tiles_m = g.M / TM, t = (int)blockIdx.x - G.first;
-    const int m0 = t % tiles_m * TM, n0 = t / tiles_m * TN_;
+    int m0, n0;
+    tile_of((int)blockIdx.x - G.first, g.M / TM, g.N / TN_, TM, TN_, m0, n0);
     const int KT = (g.K / TK + 1) / 2;  // two column blocks a step; the last one's second may be zero fill
     const int kb = (int)((int64_t)KT * part / split), ke = (int)((int64_t)KT * (part + 1) / split);
     tc::launch_dependents();
