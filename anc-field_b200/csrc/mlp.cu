@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/afd_surrogate.h"
+#include "gemm_plan.hpp"
 #include "tc.cuh"
 
 namespace afd {
@@ -59,12 +60,12 @@ struct Err : std::runtime_error {
         if (e__ != cudaSuccess) throw Err(AFD_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e__)); \
     } while (0)
 
-constexpr int TM = 128, TN = 128, TK = 64, NST = 3;
+constexpr int NST = 3;
 constexpr int A_BYTES = TM * TK * 2, B_BYTES = TN * TK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int GEMM_THREADS = 192;
 constexpr size_t GEMM_SMEM = 1024 + (size_t)NST * STAGE_BYTES + 256;
 // persistent form
-constexpr int PTN = 256, PNST = 4;
+constexpr int PNST = 4;
 constexpr int PSTAGE = A_BYTES + 2 * B_BYTES;  // A 128 x 64, B 256 x 64
 constexpr size_t PGEMM_SMEM = 1024 + (size_t)PNST * PSTAGE + 256;
 // pair form
@@ -948,87 +949,6 @@ static CUtensorMap operand_map(const bf16* base, int rows, int K, int box_rows, 
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw Err(AFD_ERR_CUDA, "tensor map encoding failed");
     return m;
-}
-
-// How a GEMM is launched: kPair, kPersist, kDual (k_gemm), else the columns of
-// k_gemm_tile's tiles, with the CTAs that share a tile's K range.
-enum : int { kPair = 0, kPersist = 1, kDual = 2 };
-struct GemmPlan {
-    int form, split;
-};
-
-// The time of a form in us: start, waves of tiles, per wave its epilogue and
-// its steps over K, from measurements (M x N x K, us on the device):
-//                   pair  persist  dual  tile 128   64    32
-//    256x256x64     10.4    10.4    6.3      7.3   6.3   6.3
-//   1024x512x512    12.5    12.5    8.4      8.4   6.8   6.3
-//   1024x512x2048   20.6    18.6   14.5     12.4  10.4  10.4
-//   1024x2048x4096  29.2    28.8   20.6     19.5  29.4  51.4
-//   1920x2176x1024    -       -    16.5     20.6  26.8  39.0
-//   2048x2048x2048  20.7    20.6   20.7     24.7  37.0  55.4
-//   4096x4096x4096   105     120    125      139     -     -
-// The 256-column forms pay a start and an epilogue of their own (10 us even
-// for one tile) and fill the chip from 74 and 148 tiles on; below that the
-// smaller tiles reach more SMs. A split pays a cluster launch of 4 us:
-// 128x2048x8192 runs 26.8 as 64-column tiles, 14.5 split four ways and 45.2 as
-// persistent tiles.
-static double gemm_cost(int form, int split, int64_t tiles, int K, int sms) {
-    const int kt = K / TK;
-    if (form == kPair) return 8.0 + (double)((tiles + sms / 2 - 1) / (sms / 2)) * (3.0 + 0.34 * kt);
-    const int64_t waves = (tiles * split + sms - 1) / sms;
-    if (form == kPersist) return 7.0 + (double)waves * (3.0 + 0.4 * kt);
-    // two CTAs an SM: a second one beside the first costs what it takes alone
-    if (form == kDual) return 4.0 + (double)((waves + 1) / 2) * (3.3 + 0.225 * kt * (waves > 1 ? 2 : 1));
-    const double step = (form == 128 ? 0.38 : form == 64 ? 0.325 : 0.29) * (waves > 1 ? 1.25 : 1.0);
-    return 3.0 + (double)waves * (3.3 + 0.01 * form + step * ((kt / 2 + split) / split)) + (split > 1 ? 4.0 : 0.0);
-}
-
-static GemmPlan plan_gemm(int M, int N, int K, bool may_split, int sms) {
-    const int64_t mt = M / TM;
-    GemmPlan best{kDual, 1};
-    double cost = gemm_cost(kDual, 1, mt * (N / TN), K, sms);
-    auto consider = [&](int form, int split, int64_t tiles) {
-        const double c = gemm_cost(form, split, tiles, K, sms);
-        if (c < cost) {
-            cost = c;
-            best = GemmPlan{form, split};
-        }
-    };
-    if (M % (2 * TM) == 0 && N % PTN == 0 && sms >= 2) consider(kPair, 1, mt / 2 * (N / PTN));
-    if (N % PTN == 0) consider(kPersist, 1, mt * (N / PTN));
-    for (int tn : {128, 64, 32})
-        for (int split : {1, 2, 4, 8}) {
-            const int64_t tiles = mt * (N / tn);
-            // shares of at least two steps; all clusters resident at once (of
-            // eight CTAs only two fit a GPC, and not every one: 16 of them
-            // took two rounds)
-            if (split > 1 && (!may_split || K / TK < 4 * split || tiles * split > (split == 8 ? sms * 2 / 3 : sms - 16)))
-                continue;
-            consider(tn, split, tiles);
-        }
-    return best;
-}
-
-// Tile columns with which GEMMs of M x N = `sizes` and one K run in one
-// launch, or -1 where one by one is faster.
-static int plan_group(const std::vector<std::pair<int, int>>& sizes, int K, int sms) {
-    double alone = 0.0;
-    int best = -1;
-    for (const auto& z : sizes) {
-        const GemmPlan p = plan_gemm(z.first, z.second, K, false, sms);
-        const int th = p.form == kPair ? 2 * TM : TM, tw = p.form >= 32 ? p.form : p.form == kDual ? TN : PTN;
-        alone += gemm_cost(p.form, 1, (int64_t)(z.first / th) * (z.second / tw), K, sms);
-    }
-    for (int tn : {128, 64, 32}) {
-        int64_t tiles = 0;
-        for (const auto& z : sizes) tiles += (int64_t)(z.first / TM) * (z.second / tn);
-        const double c = gemm_cost(tn, 1, tiles, K, sms);
-        if (c < alone) {
-            alone = c;
-            best = tn;
-        }
-    }
-    return best;
 }
 
 struct Gemm {
