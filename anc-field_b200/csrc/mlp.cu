@@ -43,6 +43,7 @@
 #include "../../include/afd_surrogate.h"
 #include "gemm_plan.hpp"
 #include "tc.cuh"
+#include "wait_flags.hpp"
 
 namespace afd {
 namespace mlp {
@@ -1337,6 +1338,19 @@ int mguard(afd_mlp* m, F&& f) {
 
 thread_local std::string g_create_err;
 
+// The wait-expired words of the synchronous GEMM calls: host memory that a
+// kernel writes only when a wait expires, so that a call needs neither a
+// clearing launch nor a copy back. Never destroyed: a thread may outlive main.
+int* mapped_word() {
+    int* w = nullptr;
+    MCK(cudaHostAlloc((void**)&w, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    return w;
+}
+afd::WaitFlags& gemm_flags() {
+    static afd::WaitFlags* flags = new afd::WaitFlags(mapped_word);
+    return *flags;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1497,26 +1511,16 @@ int afd_gemm_bf16(const void* a, const void* b, float* c, int32_t M, int32_t N, 
         int dev = 0;
         MCK(cudaGetDevice(&dev));
         if (dev < 0 || dev >= 64) throw Err(AFD_ERR_ARG, "device ordinal out of range");
-        // the wait-expired flag of each device, kept for the process: host
-        // memory that the kernel writes only when a wait expires, so that a
-        // call needs neither a clearing launch nor a copy back
-        static int* flags[64];
-        {
-            std::lock_guard<std::mutex> lock(g_gemm_mu);
-            if (!flags[dev]) MCK(cudaHostAlloc((void**)&flags[dev], sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-        }
-        volatile int* flag = flags[dev];
+        afd::WaitFlags::Lease flag(gemm_flags());
         int* mapped = nullptr;
-        MCK(cudaHostGetDevicePointer((void**)&mapped, flags[dev], 0));
+        MCK(cudaHostGetDevicePointer((void**)&mapped, flag.word(), 0));
         Gemm g = make_gemm(EPI_F32, (const bf16*)a, (const bf16*)b, M, N, K, mapped, true);
         g.o.c32 = c;
         g.o.ldc = N;
         cudaStream_t st = (cudaStream_t)stream;
-        // one flag per device: concurrent calls on one device share it
-        *flag = 0;
         launch(g, st);
         MCK(cudaStreamSynchronize(st));
-        if (*flag) throw Err(AFD_ERR_CUDA, "GEMM pipeline wait timed out");
+        if (flag.raised()) throw Err(AFD_ERR_CUDA, "GEMM pipeline wait timed out");
         return AFD_OK;
     } catch (const Err& e) {
         g_create_err = e.what();
