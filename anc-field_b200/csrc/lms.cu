@@ -372,14 +372,19 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_lms_pass(const __grid_constant
         if (!grid_barrier(a.bar, raised, a.flag)) return;
         for (int h = cta; h < kRowSets; h += G) {
             if (h != cta) rows(h);
+            const int row = row_of(h);
             double v = 0.0;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v = fma(m[u], __ldcg(a.f + col + 128 * u), v);
+            for (int u = 0; u < 4; ++u) {
+                // a later sample takes no part, not even where its f is not finite
+                const double f = __ldcg(a.f + col + 128 * u);
+                v = fma(m[u], col + 128 * u <= row ? f : 0.0, v);
+            }
             for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
             if (lane == 0) quad[warp] = v;
             __syncthreads();
             if (lane == 0 && (warp & 3) == 0)
-                a.e[row_of(h)] = (quad[warp] + quad[warp + 1]) + (quad[warp + 2] + quad[warp + 3]);
+                a.e[row] = (quad[warp] + quad[warp + 1]) + (quad[warp + 2] + quad[warp + 3]);
             __syncthreads();
         }
         raised += G;
