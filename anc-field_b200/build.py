@@ -26,7 +26,7 @@ CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-I" + 
 
 CU_SOURCES = ["engine.cu", "filters.cu", "mlp.cu", "lms.cu", "geometry.cu", "selftest.cu"]
 CXX_SOURCES = ["model.cpp", "api.cpp"]
-HEADERS = ["device.cuh", "engine.hpp", "model.hpp", "filters.hpp", "fused.cuh", "gemm_plan.hpp", "roles.cuh", "sync.cuh", "tc.cuh", "geometry.hpp", "wait_flags.hpp"]
+HEADERS = ["device.cuh", "engine.hpp", "model.hpp", "filters.hpp", "fused.cuh", "gemm_plan.hpp", "lms_subst.cuh", "roles.cuh", "sync.cuh", "tc.cuh", "geometry.hpp", "wait_flags.hpp"]
 
 
 def _nvcc():

@@ -21,9 +21,11 @@
 //   k_lms_diag     inverses of the 32 x 32 diagonal blocks
 //   k_lms_inverse  the inverses, 32 columns a CTA, by block substitution
 // and what stays sequential is one cooperative kernel over the blocks, k_lms_pass:
-// weight update by the last block's errors, y0, and e = M (d - y0).
-// All arithmetic is FP64, as in the reference.
+// weight update by the last block's errors, y0, and e = M (d - y0). Where an
+// entry of an inverse is not finite, the call runs again by substitution
+// (lms_subst.cuh). All arithmetic is FP64, as in the reference.
 #include <algorithm>
+#include <cfloat>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -46,6 +48,8 @@ constexpr int kTri = 1024 * NB * (NB + 1) / 2;  // packed inverse: row block i k
 constexpr int P_THREADS = 512;  // k_lms_pass
 constexpr int P_WARPS = P_THREADS / 32;
 constexpr int kRowSets = B / 4;  // sets of 4 samples and 4 inverse rows dealt to the CTAs
+// bits of the error flag (grid_barrier raises 2)
+constexpr int kFlagInverse = 4;
 
 // r_l over the samples of block n0 + blockIdx.x, thread l (0 < l < B).
 // WRITE = 0: the sum of the increments into r[n][l]. WRITE = 1: from r[n][l]
@@ -118,11 +122,13 @@ __global__ void __launch_bounds__(32) k_lms_diag(const double* __restrict__ tri,
 
 // 32 columns of the inverse, panel j of block g: X_i = D_i (E_i - sum_{j<=k<i}
 // T_ik X_k) for i = j .. NB-1, X in shared memory, the T and D tiles
-// streamed through two buffers. The longest panels (j = 0) come first.
+// streamed through two buffers. The longest panels (j = 0) come first. Bit 2 of
+// `flag`: an entry is not finite.
 constexpr int I_THREADS = 256;
 constexpr size_t I_SMEM = (size_t)(B * 32 + 2 * 1024) * sizeof(double);
 __global__ void __launch_bounds__(I_THREADS) k_lms_inverse(const double* __restrict__ tri,
-                                                           const double* __restrict__ diag, int blocks, double* inv) {
+                                                           const double* __restrict__ diag, int blocks, double* inv,
+                                                           int* flag) {
     extern __shared__ double i_smem[];
     double* X = i_smem;         // [32 (i - j) + row][column]
     double* A = X + B * 32;     // [2][column][row]
@@ -142,6 +148,7 @@ __global__ void __launch_bounds__(I_THREADS) k_lms_inverse(const double* __restr
     };
     fetch(j, j);
     int buf = 0;
+    bool finite = true;
     for (int i = j; i < NB; ++i) {
         double s[2][2];
 #pragma unroll
@@ -183,10 +190,12 @@ __global__ void __launch_bounds__(I_THREADS) k_lms_inverse(const double* __restr
                     const double2 v = make_double2(d[u][0], d[u][1]);
                     *reinterpret_cast<double2*>(Xi + (r + u) * 32 + c) = v;
                     *reinterpret_cast<double2*>(out + u * 32 * (i + 1)) = v;
+                    finite &= fabs(v.x) <= DBL_MAX && fabs(v.y) <= DBL_MAX;
                 }
             }
         }
     }
+    if (__any_sync(0xffffffffu, !finite) && (tid & 31) == 0) atomicOr(flag, kFlagInverse);
 }
 
 struct PassArgs {
@@ -430,12 +439,9 @@ struct Block {
     cudaStream_t st = nullptr;
     ~Block() {
         if (p) cudaFreeAsync(p, st);
-        if (st) {
-            cudaStreamSynchronize(st);
-            cudaStreamDestroy(st);
-        }
     }
-    bool alloc(size_t bytes, cudaMemPool_t pool) {
+    bool alloc(size_t bytes, cudaMemPool_t pool, cudaStream_t stream) {
+        st = stream;
         if (cudaMallocFromPoolAsync((void**)&p, bytes, pool, st) == cudaSuccess) return true;
         cudaGetLastError();
         p = nullptr;
@@ -443,7 +449,45 @@ struct Block {
     }
 };
 
+// The call's own stream; everything on it has ended once it is gone.
+struct Stream {
+    cudaStream_t st = nullptr;
+    Stream() { LCK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)); }
+    ~Stream() {
+        cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
+    }
+};
+
 thread_local std::string g_err;
+
+#include "lms_subst.cuh"
+
+// The whole recursion by substitution: w, zero on entry, from device inputs.
+void substitute(const double* xs, int64_t o, const double* d, int64_t steps, int N, double mu, int epochs, double* w,
+                int device, cudaStream_t st) {
+    using namespace subst;
+    const int nchunk = (N + J - 1) / J;
+    Block mem;
+    if (!mem.alloc(((size_t)nchunk + 2) * subst::B * sizeof(double), device_pool(device), st))
+        throw Err(AFD_ERR_CUDA, "out of device memory");
+    double* const partial = reinterpret_cast<double*>(mem.p);
+    double* const r = partial + (size_t)nchunk * subst::B;
+    double* const e = r + subst::B;
+    LCK(cudaFuncSetAttribute((const void*)k_lms_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_SMEM));
+    LCK(cudaFuncSetAttribute((const void*)k_lms_y0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Y0_SMEM));
+    for (int ep = 0; ep < epochs; ++ep) {
+        LCK(cudaMemsetAsync(r, 0, subst::B * sizeof(double), st));
+        for (int64_t k0 = 0; k0 < steps; k0 += subst::B) {
+            const int nb = (int)std::min<int64_t>(subst::B, steps - k0);
+            k_lms_y0<<<dim3((unsigned)nchunk, (unsigned)((nb + SPC - 1) / SPC)), Y0_THREADS, Y0_SMEM, st>>>(
+                w, xs, o, N, k0, nb, partial);
+            k_lms_solve<<<1, subst::B, SOLVE_SMEM, st>>>(xs, o, N, k0, nb, partial, nchunk, d, mu, r, e);
+            k_lms_update<<<(N + UPD_THREADS - 1) / UPD_THREADS, UPD_THREADS, 0, st>>>(w, xs, o, N, k0, nb, e, mu);
+        }
+    }
+    LCK(cudaGetLastError());
+}
 
 void estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t taps, double mu, int32_t epochs,
               int32_t device, double* w_out) {
@@ -487,12 +531,14 @@ void estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t 
     // inverses again in every pass.
     int64_t seg = std::min<int64_t>(nblocks, 768), group = std::min<int64_t>(seg, 64);
     const size_t tri_n = (size_t)B * B + NB * 1024;
+    Stream stream;
     Block mem;
-    LCK(cudaStreamCreateWithFlags(&mem.st, cudaStreamNonBlocking));
-    cudaStream_t st = mem.st;
+    cudaStream_t st = stream.st;
     const size_t fixed = (size_t)grid * B + 2 * B + (size_t)nblocks * B * 2 + nxs + (size_t)Np;
     for (;;) {
-        if (mem.alloc((fixed + (size_t)seg * kTri + (size_t)group * tri_n + 1) * sizeof(double), device_pool(device))) break;
+        if (mem.alloc((fixed + (size_t)seg * kTri + (size_t)group * tri_n + 1) * sizeof(double), device_pool(device),
+                      st))
+            break;
         if (seg == 1) throw Err(AFD_ERR_CUDA, "out of device memory");
         seg = (seg + 1) / 2;
         group = std::min(group, seg);
@@ -526,7 +572,7 @@ void estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t 
             const int m = (int)std::min(group, n - g);
             k_lms_lags<1><<<m, B, 0, st>>>(xs, o, N, b0 + g, 2 * mu, r, tri);
             k_lms_diag<<<dim3(NB, m), 32, 0, st>>>(tri, diag);
-            k_lms_inverse<<<m * NB, I_THREADS, I_SMEM, st>>>(tri, diag, m, inv + (size_t)g * kTri);
+            k_lms_inverse<<<m * NB, I_THREADS, I_SMEM, st>>>(tri, diag, m, inv + (size_t)g * kTri, sync + 1);
         }
         LCK(cudaGetLastError());
     };
@@ -583,7 +629,12 @@ void estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t 
     LCK(cudaMemcpyAsync(&flag, a.flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     LCK(cudaMemcpyAsync(w_out, w, (size_t)N * sizeof(double), cudaMemcpyDeviceToHost, st));
     LCK(cudaStreamSynchronize(st));
-    if (flag) throw Err(AFD_ERR_CUDA, "a wait of the recursion kernel ran out");
+    if (flag & ~kFlagInverse) throw Err(AFD_ERR_CUDA, "a wait of the recursion kernel ran out");
+    if (!flag) return;
+    LCK(cudaMemsetAsync(w, 0, (size_t)Np * sizeof(double), st));
+    substitute(xs, o, dd, steps, N, mu, epochs, w, device, st);
+    LCK(cudaMemcpyAsync(w_out, w, (size_t)N * sizeof(double), cudaMemcpyDeviceToHost, st));
+    LCK(cudaStreamSynchronize(st));
 }
 
 }  // namespace lms
