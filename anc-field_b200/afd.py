@@ -38,7 +38,7 @@ EXPORTS = [
     "afd_set_pml_profile", "afd_add_source", "afd_add_source_cell", "afd_add_receiver",
     "afd_add_receiver_cell", "afd_run", "afd_prepare", "afd_get_receivers", "afd_update_source",
     "afd_get_receivers_range", "afd_get_field", "afd_get_plane", "afd_set_capture", "afd_get_frames",
-    "afd_set_timeline", "afd_get_timeline", "afd_wait_selftest",
+    "afd_set_timeline", "afd_get_timeline", "afd_wait_selftest", "afd_barrier_selftest",
     "afd_get_info", "afd_energy", "afd_set_stream", "afd_set_plan", "afd_set_slab", "afd_step_phase", "afd_halo",
     "afd_kernel_stats", "afd_last_error",
     "afd_destroy",
@@ -129,6 +129,7 @@ def library(path=LIB_PATH):
         "afd_get_frames": (C.c_int, [vp, P(f32), i64, P(i64), i64, P(i32)]),
         "afd_set_timeline": (C.c_int, [vp, i64, i32]),
         "afd_wait_selftest": (C.c_int, [i32, i32, i32, P(i32), P(i64)]),
+        "afd_barrier_selftest": (C.c_int, [i32, i32, P(i32), P(i64)]),
         "afd_get_timeline": (C.c_int, [vp, P(f64), i64, P(i32)]),
         "afd_get_info": (C.c_int, [vp, P(Info)]),
         "afd_energy": (C.c_int, [vp, i32, P(f64)]),
@@ -271,6 +272,15 @@ def wait_selftest(which, complete, device=0):
     s = library().afd_wait_selftest(device, which, 1 if complete else 0, C.byref(t), C.byref(ns))
     if s != OK:
         raise AfdError(s, "wait self-test failed")
+    return bool(t.value), ns.value / 1e9
+
+
+def barrier_selftest(complete, device=0):
+    """The same for the grid barrier: (gave up, seconds waited)."""
+    t, ns = C.c_int32(), C.c_int64()
+    s = library().afd_barrier_selftest(device, 1 if complete else 0, C.byref(t), C.byref(ns))
+    if s != OK:
+        raise AfdError(s, "barrier self-test failed")
     return bool(t.value), ns.value / 1e9
 
 

@@ -268,6 +268,12 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_lms_pass(const __grid_constant
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    auto barrier = [&]() {
+        raised += G;
+        if (grid_barrier(a.bar, raised, a.flag)) return true;
+        copies_landed();  // the next block's windows are on their way
+        return false;
+    };
     if (cta < a.tiles) prefetch(a.a, cta, 0);
     int buf = 0;
     for (int64_t n = a.a; n < end; ++n) {
@@ -361,8 +367,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_lms_pass(const __grid_constant
             for (int u = 0; u < 4; ++u) m[u] = col + 128 * u < 32 * (i + 1) ? __ldg(p + col + 128 * u) : 0.0;
         };
         if (cta < kRowSets) rows(cta);
-        raised += G;
-        if (!grid_barrier(a.bar, raised, a.flag)) return;
+        if (!barrier()) return;
         for (int h = cta; h < kRowSets; h += G) {
             double v = 0.0;
             for (int c = tid >> 2; c < np; c += P_THREADS / 4) v += __ldcg(a.partial + (size_t)c * B + 4 * h + (tid & 3));
@@ -377,8 +382,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_lms_pass(const __grid_constant
             }
             __syncthreads();
         }
-        raised += G;
-        if (!grid_barrier(a.bar, raised, a.flag)) return;
+        if (!barrier()) return;
         for (int h = cta; h < kRowSets; h += G) {
             if (h != cta) rows(h);
             const int row = row_of(h);
@@ -396,8 +400,7 @@ __global__ void __launch_bounds__(P_THREADS, 1) k_lms_pass(const __grid_constant
                 a.e[row] = (quad[warp] + quad[warp + 1]) + (quad[warp + 2] + quad[warp + 3]);
             __syncthreads();
         }
-        raised += G;
-        if (!grid_barrier(a.bar, raised, a.flag)) return;
+        if (!barrier()) return;
     }
 }
 

@@ -13,6 +13,10 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+// Every copy of this thread to shared memory (cp.async) has landed: before a
+// block leaves early.
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Grid barrier on a counter that every block raises once per step; bounded
 // like every wait. The fences make the step's stores visible to all blocks
 // and drop the SM's cached copies of what they replaced.

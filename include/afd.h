@@ -382,6 +382,13 @@ int afd_kernel_stats(afd_sim* s, int32_t idx, char* name, int64_t cap,
 int afd_wait_selftest(int32_t device, int32_t which, int32_t complete, int32_t* timed_out,
                       int64_t* waited_ns);
 
+/* The same for the grid barrier of the kernels that run many steps in one
+ * launch: one block raises it and waits, complete = 0 for a second block that
+ * does not exist. *timed_out receives 1 when the barrier gave up, told every
+ * thread of the block so and raised the error flag that those kernels' hosts
+ * read; the block's copies in flight have then landed. */
+int afd_barrier_selftest(int32_t device, int32_t complete, int32_t* timed_out, int64_t* waited_ns);
+
 const char* afd_last_error(const afd_sim* s);
 void afd_destroy(afd_sim* s);
 
