@@ -419,14 +419,16 @@ struct Err : std::runtime_error {
 // The pool keeps what calls gave back, kPoolKeep at most (an estimate needs
 // tens to hundreds of MB, and mapping and unmapping them took 5 to 60 ms a call
 // beside 16 ms of kernels); the rest returns to the device at the next
-// synchronization, and all that no call holds when another allocation needs it.
+// synchronization, and all that no call holds when another allocation of the
+// process needs it or the caller says so (release).
 constexpr uint64_t kPoolKeep = (uint64_t)1 << 30;
-cudaMemPool_t device_pool(int device) {
+cudaMemPool_t device_pool(int device, bool make = true) {
     static std::mutex mu;
     static std::map<int, cudaMemPool_t> pools;
     std::lock_guard<std::mutex> hold(mu);
     auto it = pools.find(device);
     if (it != pools.end()) return it->second;
+    if (!make) return nullptr;
     cudaMemPoolProps p{};
     p.allocType = cudaMemAllocationTypePinned;
     p.location.type = cudaMemLocationTypeDevice;
@@ -640,6 +642,28 @@ void estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t 
     LCK(cudaStreamSynchronize(st));
 }
 
+// Gives back what the device's pool keeps beyond the calls in progress.
+void release(int32_t device) {
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) throw Err(AFD_ERR_CUDA, "no CUDA device available");
+    if (device < 0 || device >= ndev) throw Err(AFD_ERR_ARG, "device ordinal out of range");
+    if (cudaMemPool_t pool = device_pool(device, false)) LCK(cudaMemPoolTrimTo(pool, 0));
+}
+
+template <typename F>
+int guard(F&& f) {
+    try {
+        f();
+        return AFD_OK;
+    } catch (const Err& e) {
+        g_err = e.what();
+        return e.code;
+    } catch (const std::exception& e) {
+        g_err = e.what();
+        return AFD_ERR_STATE;
+    }
+}
+
 }  // namespace lms
 }  // namespace afd
 
@@ -647,16 +671,11 @@ extern "C" {
 
 int afd_lms_estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t taps, double mu,
                      int32_t epochs, int32_t device, double* w) {
-    try {
-        afd::lms::estimate(x, nx, d, nd, taps, mu, epochs, device, w);
-        return AFD_OK;
-    } catch (const afd::lms::Err& e) {
-        afd::lms::g_err = e.what();
-        return e.code;
-    } catch (const std::exception& e) {
-        afd::lms::g_err = e.what();
-        return AFD_ERR_STATE;
-    }
+    return afd::lms::guard([&] { afd::lms::estimate(x, nx, d, nd, taps, mu, epochs, device, w); });
+}
+
+int afd_lms_release(int32_t device) {
+    return afd::lms::guard([&] { afd::lms::release(device); });
 }
 
 const char* afd_lms_last_error(void) { return afd::lms::g_err.c_str(); }

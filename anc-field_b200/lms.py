@@ -7,7 +7,7 @@ import numpy as np
 
 from . import afd
 
-EXPORTS = ["afd_lms_estimate", "afd_lms_last_error"]
+EXPORTS = ["afd_lms_estimate", "afd_lms_release", "afd_lms_last_error"]
 _bound = False
 
 
@@ -19,6 +19,8 @@ def _lib():
         L.afd_lms_estimate.restype = C.c_int
         L.afd_lms_estimate.argtypes = [P(C.c_double), C.c_int64, P(C.c_double), C.c_int64, C.c_int32, C.c_double,
                                        C.c_int32, C.c_int32, P(C.c_double)]
+        L.afd_lms_release.restype = C.c_int
+        L.afd_lms_release.argtypes = [C.c_int32]
         L.afd_lms_last_error.restype = C.c_char_p
         L.afd_lms_last_error.argtypes = []
         _bound = True
@@ -38,6 +40,14 @@ def estimate_ir(x, d, N, mu=1e-4, epochs=16, device=0):
     if st != afd.OK:
         raise afd.AfdError(st, L.afd_lms_last_error().decode())
     return w[:N]
+
+
+def release(device=0):
+    """Gives the device memory kept for later estimates back to the device."""
+    L = _lib()
+    st = L.afd_lms_release(int(device))
+    if st != afd.OK:
+        raise afd.AfdError(st, L.afd_lms_last_error().decode())
 
 
 def EstimateIr(input, output, N, mu=1e-4):  # noqa: N802 - the reference's name

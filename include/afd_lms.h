@@ -22,9 +22,15 @@ extern "C" {
 #endif
 
 /* w[taps] (host) = the estimate; x, d host arrays. The reference's default
- * is epochs = 16. Returns AFD_OK or AFD_ERR_*. */
+ * is epochs = 16. Returns AFD_OK or AFD_ERR_*. Calls may run on several threads.
+ * Device memory of a call (1.1 MB per 512 samples, about 1 GB at most beside the
+ * signals) stays with the library for the next one, 1 GB a device at most, until
+ * another allocation of this process needs it or afd_lms_release. */
 int afd_lms_estimate(const double* x, int64_t nx, const double* d, int64_t nd, int32_t taps, double mu,
                      int32_t epochs, int32_t device, double* w);
+/* Gives the device memory kept for later calls back to the device (for other
+ * processes, say); calls in progress keep theirs. */
+int afd_lms_release(int32_t device);
 const char* afd_lms_last_error(void);
 
 #ifdef __cplusplus
