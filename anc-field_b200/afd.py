@@ -67,7 +67,8 @@ class Info(C.Structure):
                 ("last_run_ms", C.c_double), ("kernel_launches", C.c_int64),
                 ("tile_x", C.c_int32), ("tile_y", C.c_int32), ("tile_z", C.c_int32),
                 ("stream_blocks", C.c_int32), ("tuned", C.c_int32), ("stream_beside", C.c_int32),
-                ("stream_per_sm", C.c_int32), ("stream_tail", C.c_int32), ("reserved", C.c_int32 * 4)]
+                ("stream_per_sm", C.c_int32), ("stream_tail", C.c_int32), ("resident", C.c_int32),
+                ("reserved", C.c_int32 * 3)]
 
 
 class Plan(C.Structure):

@@ -3690,8 +3690,9 @@ void Engine::get_info(afd_info* info) {
     info->stream_beside = D.lists_beside() ? 1 : 0;
     info->stream_per_sm = D.stream_per_sm;
     info->stream_tail = D.tail_active() ? 1 : 0;
+    info->resident = D.initialized && D.resident() ? 1 : 0;
     // a grid that runs in the resident kernel has nothing left to choose
-    info->tuned = D.tuned || (D.initialized && D.resident()) ? 1 : 0;
+    info->tuned = D.tuned || info->resident ? 1 : 0;
 }
 
 int Engine::kernel_stats(int32_t idx, char* name, int64_t cap, int64_t* launches, double* ms) {

@@ -290,11 +290,13 @@ typedef struct afd_info {
     int64_t kernel_launches;     /* kernels launched by the last afd_run */
     int32_t tile_x, tile_y, tile_z;  /* tile (cells) and z-chunk depth of the streaming kernel's plan */
     int32_t stream_blocks;       /* resident blocks of the streaming kernel's plan */
-    int32_t tuned;               /* 1 once the online autotuner has chosen the plan */
+    int32_t tuned;               /* 1 once the plan is final: chosen by the online autotuner, or resident = 1 */
     int32_t stream_beside;       /* 1: the plan runs the boundary and PML kernels beside the streaming kernel */
     int32_t stream_per_sm;       /* resident streaming blocks per SM of the plan */
     int32_t stream_tail;         /* 1: the plan does the boundary and PML pressure work in the streaming kernel */
-    int32_t reserved[4];
+    int32_t resident;            /* 1: with the present settings the steps of a chunk run in the resident kernel,
+                                    which has no streaming plan (small grids); 0: in launches of their own */
+    int32_t reserved[3];
 } afd_info;
 int afd_get_info(afd_sim* s, afd_info* info);
 
