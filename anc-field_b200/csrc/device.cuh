@@ -112,17 +112,18 @@ struct RcvDev {
 };
 
 // Source cells and receivers taken by the step's own kernels (on != 0; see
-// src_rcv_role): n distinct source cells over all members; entry = the
-// cell's boundary entry, kSrcInterior for another cell 1..n-2, kSrcOuter on
-// an outer face; sources begin[k] .. begin[k+1]-1 of cell k in insertion
-// order, with their member, signal length and offset.
+// src_pair): n pairs of a member and a cell in which it has sources, by member,
+// then by cell; pairs first[b] .. first[b+1]-1 are member b's. entry = the cell's
+// boundary entry, kSrcInterior for another cell 1..n-2, kSrcOuter on an outer
+// face; sources begin[k] .. begin[k+1]-1 of pair k in insertion order, with their
+// signal length and offset.
 struct SrcRcvDev {
     int32_t on, n;
-    const int32_t *cell, *entry, *begin, *member;
+    const int32_t *first, *member, *cell, *entry, *begin;
     const int64_t *len, *off;
 };
 constexpr int32_t kSrcInterior = -1, kSrcOuter = -2;
-// bit of an entry's packed info: a source lies in its cell
+// bit of an entry's packed info: a source of some member lies in its cell
 constexpr uint32_t kSrcEntry = 1u << 31;
 
 // FP16 field storage (AFD_STORE_FP16, FIXED scheme): the three levels as

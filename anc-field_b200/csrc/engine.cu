@@ -81,17 +81,21 @@ __device__ __forceinline__ void watch(int* flag, float v) {
     if (!(fabsf(v) < 1e30f)) atomicOr(flag, 1);
 }
 
-// Receivers of one member from level g at `p` (mic.cl:32-41), threads t, t +
-// threads, ...; inv and sc: the level's inverse scale and scale.
+// Receiver r of one member from level g at `p` (mic.cl:32-41); inv and sc: the
+// level's inverse scale and scale.
+template <typename T>
+__device__ __forceinline__ void record_receiver(const StepArgs& a, int b, int r, long long g, const T* p, float inv,
+                                                float sc) {
+    const float v = fld(p + __ldg(a.rcv.cell + r), inv);
+    a.rcv.out[((size_t)b * a.rcv.n + r) * a.rcv.cap + g] = v;
+    if constexpr (sizeof(T) == 4) watch(a.flag, v);
+    else if (!f16_finite(v * sc)) atomicOr(a.flag, 1);
+}
+// Its receivers t, t + threads, ...
 template <typename T>
 __device__ __forceinline__ void record_receivers(const StepArgs& a, int b, long long g, const T* p, float inv,
                                                  float sc, int t, int threads) {
-    for (int r = t; r < a.rcv.n; r += threads) {
-        const float v = fld(p + __ldg(a.rcv.cell + r), inv);
-        a.rcv.out[((size_t)b * a.rcv.n + r) * a.rcv.cap + g] = v;
-        if constexpr (sizeof(T) == 4) watch(a.flag, v);
-        else if (!f16_finite(v * sc)) atomicOr(a.flag, 1);
-    }
+    for (int r = t; r < a.rcv.n; r += threads) record_receiver<T>(a, b, r, g, p, inv, sc);
 }
 
 // leapfrog.cl:34-55 over 1 <= x,y,z <= n-2 of every batch member. FP16
@@ -197,12 +201,27 @@ __device__ __forceinline__ LevelScales level_scales(const StepArgs& a, int b, in
     return r;
 }
 
+// Whether member b has a source in cell c, one of the source cells. Not inlined:
+// few entries ask.
+__device__ __noinline__ bool has_source(const StepArgs& a, int b, int c) {
+    if (a.batch == 1) return true;
+    int lo = __ldg(a.sr.first + b), hi = __ldg(a.sr.first + b + 1);
+    while (lo < hi) {
+        const int m = (lo + hi) >> 1, v = __ldg(a.sr.cell + m);
+        if (v == c) return true;
+        if (v < c) lo = m + 1;
+        else hi = m;
+    }
+    return false;
+}
+
 // The same with the new value stored. Entries of source cells (kSrcEntry)
-// are left to src_rcv_role when `skip_src` is set.
+// are left to src_pair for the members that have a source there, when `skip_src`
+// is set.
 template <bool REF, int KT, typename T, bool NC = true>
 __device__ __forceinline__ void lrs_update(const StepArgs& a, const StepIdx& I, int b, int e, int64_t c,
                                            uint32_t info, bool skip_src = false) {
-    if (skip_src && (info & kSrcEntry)) return;
+    if (skip_src && (info & kSrcEntry) && has_source(a, b, (int)c)) return;
     const LevelScales sc = level_scales<T>(a, b, I.s5);
     const float v = lrs_value<REF, KT, T, NC>(a, I, b, e, c, info, sc.ic, sc.io);
     fst(level_ptr<T>(a, I.wn) + (size_t)b * a.g.vol + c, v, sc.s_new);
@@ -211,61 +230,61 @@ __device__ __forceinline__ void lrs_update(const StepArgs& a, const StepIdx& I, 
     }
 }
 
-// Source cells and receivers of one batch member inside the step's own
-// kernels (StepArgs::sr): thread t of `threads` takes source cells t, t +
-// threads, ...: the cell's update of this step (boundary entry, interior
-// value, or the untouched value of an outer face) followed by its sources in
-// insertion order (source.cl:32-40), each rounded to the storage type as a
-// store and load would. Receivers (mic.cl:32-41) are recorded one step late,
-// from p^n = the finished level g - 1, which no kernel of the step writes;
-// record = false at the first step of a chunk (the step before it was recorded
-// at that chunk's end). Not inlined: it would raise the register need of the
-// boundary kernel.
+// Source pair k, of member b, inside the step's own kernels (StepArgs::sr): the
+// cell's update of this step (boundary entry, interior value, or the untouched
+// value of an outer face) followed by the member's sources there in insertion
+// order (source.cl:32-40), each rounded to the storage type as a store and load
+// would. Not inlined: it would raise the register need of the boundary kernel.
 template <bool REF, typename T, bool NC>
-__device__ __noinline__ void src_rcv_role(const StepArgs& a, const StepIdx I, int b, int t, int threads, bool record) {
+__device__ __noinline__ void src_pair(const StepArgs& a, const StepIdx I, int b, int k) {
     const size_t base = (size_t)b * a.g.vol;
-    const long long g = I.g;
     const LevelScales sc = level_scales<T>(a, b, I.s5);
     const T* pc = level_ptr<T>(a, I.wc) + base;
     const T* po = level_ptr<T>(a, I.wo) + base;
-    for (int k = t; k < a.sr.n; k += threads) {
-        const int64_t c = __ldg(a.sr.cell + k);
-        const int e = __ldg(a.sr.entry + k);
-        const int q0 = __ldg(a.sr.begin + k), q1 = __ldg(a.sr.begin + k + 1);
-        T* pn = level_ptr<T>(a, I.wn) + base + c;
-        float v;  // FP16: the stored value
-        if (e >= 0) {
-            v = lrs_value<REF, 0, T, NC>(a, I, b, e, c, __ldg(a.lrs.info + e), sc.ic, sc.io);
-            if constexpr (sizeof(T) == 2) {
-                if (!f16_finite(v * sc.s_new)) atomicOr(a.flag, 1);
-            }
-        } else if (e == kSrcInterior) {
-            const int64_t pitch = a.g.pitch, plane = a.g.plane;
-            if constexpr (sizeof(T) == 4) {
-                v = slf_update(a.lambda2, a.cint, pc[c + 1], pc[c - 1], pc[c + pitch], pc[c - pitch], pc[c + plane],
-                               pc[c - plane], pc[c], po[c]);
-            } else {
-                v = slf_update_scaled(
-                        a.lambda2, sc.s_new * sc.ic, sc.s_new * sc.io, __half2float(pc[c + 1]),
-                        __half2float(pc[c - 1]), __half2float(pc[c + pitch]), __half2float(pc[c - pitch]),
-                        __half2float(pc[c + plane]), __half2float(pc[c - plane]), __half2float(pc[c]),
-                        __half2float(po[c])) * sc.i_new;
-            }
+    const int64_t c = __ldg(a.sr.cell + k);
+    const int e = __ldg(a.sr.entry + k);
+    const int q0 = __ldg(a.sr.begin + k), q1 = __ldg(a.sr.begin + k + 1);
+    T* pn = level_ptr<T>(a, I.wn) + base + c;
+    float v;  // FP16: the stored value
+    if (e >= 0) {
+        v = lrs_value<REF, 0, T, NC>(a, I, b, e, c, __ldg(a.lrs.info + e), sc.ic, sc.io);
+        if constexpr (sizeof(T) == 2) {
+            if (!f16_finite(v * sc.s_new)) atomicOr(a.flag, 1);
+        }
+    } else if (e == kSrcInterior) {
+        const int64_t pitch = a.g.pitch, plane = a.g.plane;
+        if constexpr (sizeof(T) == 4) {
+            v = slf_update(a.lambda2, a.cint, pc[c + 1], pc[c - 1], pc[c + pitch], pc[c - pitch], pc[c + plane],
+                           pc[c - plane], pc[c], po[c]);
         } else {
-            v = fld(pn, sc.i_new);
+            v = slf_update_scaled(
+                    a.lambda2, sc.s_new * sc.ic, sc.s_new * sc.io, __half2float(pc[c + 1]), __half2float(pc[c - 1]),
+                    __half2float(pc[c + pitch]), __half2float(pc[c - pitch]), __half2float(pc[c + plane]),
+                    __half2float(pc[c - plane]), __half2float(pc[c]), __half2float(po[c])) * sc.i_new;
         }
-        auto stored = [&](float u) {  // what a store and load of u give
-            if constexpr (sizeof(T) == 4) return u;
-            else return __half2float(__float2half_rn(u * sc.s_new)) * sc.i_new;
-        };
-        v = stored(v);
-        for (int q = q0; q < q1; ++q) {
-            if (__ldg(a.sr.member + q) != b) continue;
-            v = stored(v + (g < __ldg(a.sr.len + q) ? a.src.data[__ldg(a.sr.off + q) + g] : 0.0f));
-        }
-        fst(pn, v, sc.s_new);
+    } else {
+        v = fld(pn, sc.i_new);
     }
-    if (record) record_receivers<T>(a, b, g - 1, pc, sc.ic, 1.0f / sc.ic, t, threads);
+    auto stored = [&](float u) {  // what a store and load of u give
+        if constexpr (sizeof(T) == 4) return u;
+        else return __half2float(__float2half_rn(u * sc.s_new)) * sc.i_new;
+    };
+    v = stored(v);
+    for (int q = q0; q < q1; ++q)
+        v = stored(v + (I.g < __ldg(a.sr.len + q) ? a.src.data[__ldg(a.sr.off + q) + I.g] : 0.0f));
+    fst(pn, v, sc.s_new);
+}
+
+// Sources and receivers of member b, pairs and receivers t, t + threads, ....
+// Receivers (mic.cl:32-41) are recorded one step late, from p^n = the finished
+// level g - 1, which no kernel of the step writes; record = false at the first
+// step of a chunk (the step before it was recorded at that chunk's end).
+template <bool REF, typename T, bool NC>
+__device__ __noinline__ void src_rcv_role(const StepArgs& a, const StepIdx I, int b, int t, int threads, bool record) {
+    for (int k = __ldg(a.sr.first + b) + t; k < __ldg(a.sr.first + b + 1); k += threads) src_pair<REF, T, NC>(a, I, b, k);
+    if (!record) return;
+    const float ic = level_scales<T>(a, b, I.s5).ic;
+    record_receivers<T>(a, b, I.g - 1, level_ptr<T>(a, I.wc) + (size_t)b * a.g.vol, ic, 1.0f / ic, t, threads);
 }
 
 template <bool REF, int KT, typename T>
@@ -1412,10 +1431,12 @@ __global__ void k_mark_sources(const int32_t* __restrict__ cell, uint32_t* info,
     }
 }
 
-// The cells of a mask of 1 bit per cell, set.
-__global__ void k_set_bits(const int32_t* __restrict__ cells, int n, uint32_t* bits) {
+// The cells of a mask of 1 bit per cell, set; cell k in the mask of member[k],
+// `words` after the one before it (0: one mask for all).
+__global__ void k_set_bits(const int32_t* __restrict__ cells, const int32_t* __restrict__ member, int n,
+                           int64_t words, uint32_t* bits) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) atomicOr(bits + (cells[k] >> 5), 1u << (cells[k] & 31));
+    if (k < n) atomicOr(bits + member[k] * words + (cells[k] >> 5), 1u << (cells[k] & 31));
 }
 
 // Solid cell of the model (cells outside the model or the grid are air).
@@ -1587,9 +1608,10 @@ struct Engine::Impl {
     DBuf<float> src_data;
     DBuf<int32_t> rcv_cell;
     // sources and receivers taken by the step's kernels (SrcRcvDev)
-    DBuf<int32_t> sr_cell, sr_entry, sr_begin, sr_member;
+    DBuf<int32_t> sr_first, sr_member, sr_cell, sr_entry, sr_begin;
     DBuf<int64_t> sr_len, sr_off;
     int32_t sr_n = 0;
+    bool sr_same = true;  // every member has sources in the same cells
     bool sr_ok = false;  // the distinct source cells fit one block's table
     DBuf<uint32_t> res_owned;
     DBuf<ResidentGroup> res_groups;
@@ -1682,6 +1704,7 @@ struct Engine::Impl {
     // launches.
     bool resident() const {
         return sr_active() && !forced && cap_every <= 0 && tl_steps <= 0 &&
+               (int64_t)receivers.size() * prm.batch < (int64_t)1 << 30 &&
                vol * prm.batch <= (pml_fixed() ? kResidentCellsPml : kResidentCells);
     }
     void build_resident();
@@ -2343,41 +2366,61 @@ void Engine::Impl::upload_sources() {
     fused_dirty = true;
 }
 
-// The distinct source cells over all members with their sources in insertion
-// order, and the boundary entries that hold one.
+// The pairs of a member and a cell in which it has sources, with these in
+// insertion order, and the boundary entries that hold a source of some member.
 void Engine::Impl::upload_source_cells(const std::vector<int32_t>& cell, const std::vector<int64_t>& off,
                                        const std::vector<int64_t>& len, const std::vector<int32_t>& begin) {
-    std::map<int32_t, std::vector<int>> at;  // cell -> sources, grouped by member, insertion order within one
-    for (size_t k = 0; k < cell.size(); ++k) at[cell[k]].push_back((int)k);
-    sr_ok = (int)at.size() <= kMaxSrcCells;
-    sr_n = sr_ok ? (int32_t)at.size() : 0;
-    std::vector<int32_t> c, e, b{0}, m;
+    std::map<int32_t, int32_t> cells;  // every source cell, and its place in `distinct`
+    for (int32_t c : cell) cells.emplace(c, 0);
+    sr_ok = (int)cells.size() <= kMaxSrcCells;
+    if (!sr_ok) cells.clear();
+    std::vector<int32_t> distinct, where;
+    for (auto& kv : cells) {
+        kv.second = (int32_t)distinct.size();
+        const int32_t x = (int32_t)(kv.first % pitch), y = (int32_t)(kv.first % plane / pitch),
+                      z = (int32_t)(kv.first / plane);
+        const bool inner = x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1;
+        distinct.push_back(kv.first);
+        where.push_back(inner ? kSrcInterior : kSrcOuter);
+    }
+    if (lrs_info.n) {
+        DBuf<int32_t> d, w;
+        d.upload(distinct);
+        w.upload(where);
+        k_mark_sources<<<(unsigned)std::min<size_t>((lrs_info.n + 255) / 256, 1184), 256, 0, stream>>>(
+            lrs_cell.ptr, lrs_info.ptr, (int)lrs_info.n, d.ptr, (int)distinct.size(), w.ptr);
+        CK(cudaGetLastError());
+        if (!where.empty())
+            CK(cudaMemcpyAsync(where.data(), w.ptr, where.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        CK(cudaStreamSynchronize(stream));
+    }
+    std::vector<int32_t> first{0}, m, c, e, b{0};
     std::vector<int64_t> l, o;
-    if (sr_ok)
+    for (int32_t bm = 0; bm < prm.batch; ++bm) {
+        std::map<int32_t, std::vector<int32_t>> at;
+        if (sr_ok)
+            for (int32_t k = begin[(size_t)bm]; k < begin[(size_t)bm + 1]; ++k) at[cell[(size_t)k]].push_back(k);
         for (const auto& kv : at) {
-            const int32_t x = (int32_t)(kv.first % pitch), y = (int32_t)(kv.first % plane / pitch),
-                          z = (int32_t)(kv.first / plane);
-            const bool inner = x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1;
+            m.push_back(bm);
             c.push_back(kv.first);
-            e.push_back(inner ? kSrcInterior : kSrcOuter);
-            for (int k : kv.second) {
-                m.push_back((int32_t)(std::upper_bound(begin.begin(), begin.end(), k) - begin.begin()) - 1);
+            e.push_back(where[(size_t)cells[kv.first]]);
+            for (int32_t k : kv.second) {
                 l.push_back(len[(size_t)k]);
                 o.push_back(off[(size_t)k]);
             }
-            b.push_back((int32_t)m.size());
+            b.push_back((int32_t)l.size());
         }
+        first.push_back((int32_t)c.size());
+    }
+    sr_n = (int32_t)c.size();
+    sr_same = c.size() == distinct.size() * (size_t)prm.batch;
+    sr_first.upload(first);
+    sr_member.upload(m);
     sr_cell.upload(c);
     sr_entry.upload(e);
     sr_begin.upload(b);
-    sr_member.upload(m);
     sr_len.upload(l);
     sr_off.upload(o);
-    if (lrs_info.n) {
-        k_mark_sources<<<(unsigned)std::min<size_t>((lrs_info.n + 255) / 256, 1184), 256, 0, stream>>>(
-            lrs_cell.ptr, lrs_info.ptr, (int)lrs_info.n, sr_cell.ptr, sr_n, sr_entry.ptr);
-        CK(cudaGetLastError());
-    }
     res_dirty = true;
 }
 
@@ -2390,16 +2433,27 @@ void Engine::Impl::build_resident() {
     const bool pml = pml_fixed();
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    const int64_t all = (int64_t)sms * kResGroups - 1;  // one group keeps the sources and receivers
     ResidentDev& R = res;
     R = ResidentDev{};
     R.nu = (nx - 2) / 4 + 1;
     R.ncol = R.nu * (ny - 2);
-    const double c_plane = 1.0, c_item = 1.0, c_lrs = 4.0, c_pml = 6.0;
+    const double c_plane = 1.0, c_item = 1.0, c_lrs = 4.0, c_pml = 6.0, c_pair = 6.0, c_rcv = 2.0;
     const int64_t lrs = (int64_t)lrs_cell.n * prm.batch, planes = nz - 2, units = pml ? pml_units * prm.batch : 0;
     const double fixed = (lrs + 255) / 256 * c_lrs + (units + 255) / 256 * c_pml;
-    // columns of zc planes: about one item per thread of the remaining groups
+    // groups that take the sources and receivers alone: as many as leave each no
+    // more of them than another group's share, in whole passes of 256 (one group
+    // for all of them, every member walking all source cells, took 257 us a step
+    // for 256 members of 28x22x18 with a source each)
     const double cols = (double)R.ncol * prm.batch / 256.0;
+    const int64_t rcv = (int64_t)rcv_n_dev * prm.batch, sr_items = (sr_n + 31) / 32 * 32 + rcv;
+    const double sr_cost = sr_n / 256.0 * c_pair + rcv / 256.0 * c_rcv;
+    const double share = (fixed + cols * planes * c_plane + sr_cost) / ((double)sms * kResGroups);
+    const int64_t passes = std::max<int64_t>((sr_items + 255) / 256, 1);
+    R.sr_groups = (int32_t)std::min<int64_t>(
+        {std::max<int64_t>((int64_t)std::ceil(sr_cost / std::max(share, c_pair)), 1), passes, (int64_t)sms});
+    R.by_rcv.set((uint32_t)std::max(rcv_n_dev, 1));
+    const int64_t all = (int64_t)sms * kResGroups - R.sr_groups;
+    // columns of zc planes: about one item per thread of the remaining groups
     int zc = 1;
     while (zc < 16 && zc < planes &&
            cols * ((planes + zc - 1) / zc) * (zc * c_plane + c_item) + fixed > all * (zc * c_plane + c_item))
@@ -2470,8 +2524,9 @@ void Engine::Impl::build_resident() {
     }
     // the second phase spreads its units over as many groups as are there
     const int64_t need = std::max<int64_t>((int64_t)g.size(), std::min<int64_t>(all, (aux * prm.batch + 255) / 256));
-    res_blocks = (int)((need + 1 + kResGroups - 1) / kResGroups);
-    // group k of the list: block k mod blocks, so that heavy roles spread over the SMs
+    res_blocks = (int)((need + R.sr_groups + kResGroups - 1) / kResGroups);
+    // group k of the list: block k mod blocks, so that heavy roles spread over the
+    // SMs; the last sr_groups are those of the sources and receivers
     std::vector<ResidentGroup> placed((size_t)res_blocks * kResGroups, ResidentGroup{});
     for (size_t k = 0; k < g.size(); ++k) placed[(k % res_blocks) * kResGroups + k / res_blocks] = g[k];
     res_groups.upload(placed);
@@ -2485,11 +2540,17 @@ void Engine::Impl::build_resident() {
     }
     if (!res_bar.ptr) res_bar.alloc(1);
     // cells the interior role leaves to the others
-    const size_t words = (size_t)nz * ny * (pitch / 32);
-    res_owned.alloc(words, false);
+    // (of each member where their source cells differ)
+    const size_t words = (size_t)nz * ny * (pitch / 32), masks = sr_same ? 1 : (size_t)prm.batch;
+    R.owned_words = sr_same ? 0 : (int64_t)words;
+    res_owned.alloc(words * masks, false);
     or_masks_device(!ref() && pml_owned.n == words ? pml_owned.ptr : nullptr, lrs_bits.ptr, res_owned.ptr,
                     (int64_t)words, stream);
-    if (sr_n) k_set_bits<<<(sr_n + 255) / 256, 256, 0, stream>>>(sr_cell.ptr, sr_n, res_owned.ptr);
+    for (size_t have = 1; have < masks; have *= 2)
+        CK(cudaMemcpyAsync(res_owned.ptr + have * words, res_owned.ptr, std::min(have, masks - have) * words * sizeof(uint32_t),
+                           cudaMemcpyDeviceToDevice, stream));
+    if (sr_n)
+        k_set_bits<<<(sr_n + 255) / 256, 256, 0, stream>>>(sr_cell.ptr, sr_member.ptr, sr_n, R.owned_words, res_owned.ptr);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream));
     R.groups = res_groups.ptr;
@@ -2564,6 +2625,7 @@ void Engine::Impl::ensure_receivers(int64_t t_end) {
     std::swap(rcv_out.ptr, fresh.ptr);
     std::swap(rcv_out.n, fresh.n);
     rcv_cap = cap;
+    if (nr != rcv_n_dev) res_dirty = true;  // their share of the resident step
     rcv_n_dev = nr;
     rcv_cell.upload(cell);
     drop_graphs();
@@ -2649,10 +2711,11 @@ void Engine::Impl::build_args() {
     a.src.len = src_len.ptr;
     a.src.data = src_data.ptr;
     a.sr.n = sr_n;
+    a.sr.first = sr_first.ptr;
+    a.sr.member = sr_member.ptr;
     a.sr.cell = sr_cell.ptr;
     a.sr.entry = sr_entry.ptr;
     a.sr.begin = sr_begin.ptr;
-    a.sr.member = sr_member.ptr;
     a.sr.len = sr_len.ptr;
     a.sr.off = sr_off.ptr;
     a.rcv.n = rcv_n_dev;

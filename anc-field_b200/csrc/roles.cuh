@@ -4,9 +4,9 @@
 // All steps of a chunk in one cooperative launch, for grids whose levels stay
 // in L2: per step every group of 256 threads takes its share of PML pressure
 // units, boundary entries and interior columns (they write disjoint cells and
-// read only finished levels), one group the sources and receivers; a grid
-// barrier, the auxiliary PML units where there are any, and another barrier end
-// the step.
+// read only finished levels), one group or a few more the sources and receivers; a
+// grid barrier, the auxiliary PML units where there are any, and another barrier
+// end the step.
 //
 // Latency sets the pace: the chunk's 200 steps as graph nodes cost 10 us each
 // even for the smallest room (three to five dependent launches), while the
@@ -70,6 +70,9 @@ struct ResidentDev {
     ResidentBoxes press, aux;  // PML units of the pressure and of the auxiliary updates
     const int32_t* order;      // boundary entries by kind, so that few warps mix kinds
     const uint32_t* owned;     // cells of the other roles, pitch / 32 words per row
+    int64_t owned_words;       // words from a member's mask to the next one's, 0: one for all
+    int32_t sr_groups;         // groups of the sources and receivers
+    FastDiv by_rcv;
     unsigned int* bar;
     int32_t steps;
 };
@@ -135,7 +138,8 @@ __device__ __forceinline__ void interior_role(const StepArgs& a, const StepIdx& 
             const T* pc = pc0 + at;
             const T* po = po0 + at;
             T* pn = pn0 + at;
-            const uint32_t* ow = R.owned ? R.owned + ((int64_t)z0 * a.g.ny + y) * wpr + (x >> 5) : nullptr;
+            const uint32_t* ow =
+                R.owned ? R.owned + b * R.owned_words + ((int64_t)z0 * a.g.ny + y) * wpr + (x >> 5) : nullptr;
             unsigned in = 15u;  // cells of the unit inside 1..nx-2
             if (x == 0) in &= 14u;
             if (x + 3 > nx - 2) in &= (1u << (nx - 1 - x)) - 1u;
@@ -217,6 +221,26 @@ __device__ __forceinline__ void resident_lrs(const StepArgs& a, const StepIdx& I
     }
 }
 
+// Sources and receivers of all members, item t, t + threads, ... of the source
+// pairs (whole warps of them), then of the members' receivers (see src_rcv_role
+// for `record`).
+template <bool REF, typename T>
+__device__ __forceinline__ void src_rcv_items(const StepArgs& a, const StepIdx& I, const ResidentDev& R, int t,
+                                              int threads, bool record) {
+    const int pairs = (a.sr.n + 31) & ~31, all = pairs + (record ? a.rcv.n * a.batch : 0);
+    for (int u = t; u < all; u += threads) {
+        if (u >= pairs) {
+            const int r = u - pairs, b = (int)R.by_rcv.div((uint32_t)r);
+            const float ic = level_scales<T>(a, b, I.s5).ic;
+            record_receiver<T>(a, b, r - b * a.rcv.n, I.g - 1, level_ptr<T>(a, I.wc) + (size_t)b * a.g.vol, ic, 1.0f / ic);
+        } else if (u < a.sr.n) {
+            src_pair<REF, T, false>(a, I, __ldg(a.sr.member + u), u);
+        }
+    }
+    if constexpr (sizeof(T) == 2)
+        for (int b = t; b < a.batch; b += threads) a.f16.mx[(size_t)b * 5 + I.s5] = 0u;
+}
+
 // PML: 0 none, 1 without psi, 2 with psi.
 template <bool REF, int PML, typename T>
 __global__ void __launch_bounds__(kResGroups* kGroup, 1)
@@ -224,8 +248,8 @@ __global__ void __launch_bounds__(kResGroups* kGroup, 1)
     __shared__ unsigned int smax[kResGroups];
     const int group = (int)threadIdx.x / kGroup, tid = (int)threadIdx.x % kGroup;
     const ResidentGroup G = R.groups[blockIdx.x * kResGroups + group];
-    // the grid's last group takes the sources and receivers
-    const bool src_rcv = blockIdx.x == gridDim.x - 1 && group == kResGroups - 1;
+    // the last groups (group k: block k mod blocks) take the sources and receivers
+    const int sr_at = (kResGroups - 1 - group) * (int)gridDim.x + (int)(gridDim.x - 1 - blockIdx.x);
     StepIdx I = step_at(a, 0);
     const int K = a.lrs.K;
     // the thread's first boundary entry, kept over the steps
@@ -236,6 +260,7 @@ __global__ void __launch_bounds__(kResGroups* kGroup, 1)
         le = __ldg(R.order + (G.l0 + tid - lb * a.lrs.n));
         lc = __ldg(a.lrs.cell + le);
         linfo = __ldg(a.lrs.info + le);
+        if ((linfo & kSrcEntry) && !has_source(a, lb, lc)) linfo &= ~kSrcEntry;
     }
     if (threadIdx.x < kResGroups) smax[threadIdx.x] = 0u;
     __syncthreads();
@@ -260,15 +285,8 @@ __global__ void __launch_bounds__(kResGroups* kGroup, 1)
             resident_lrs<REF, T>(a, I, K, b, e, c, info);
         }
         if (G.i1 > G.i0) interior_role<T>(a, I, R, G, tid, smax + group);
-        if (src_rcv) {
-            // members side by side: `per` threads each
-            int per = kGroup;
-            while (per > 8 && per * a.batch > kGroup) per >>= 1;
-            for (int b = tid / per; b < a.batch; b += kGroup / per) {
-                src_rcv_role<REF, T, false>(a, I, b, tid % per, per, s > 0);
-                if (sizeof(T) == 2 && tid % per == 0) a.f16.mx[(size_t)b * 5 + I.s5] = 0u;
-            }
-        }
+        if (sr_at < R.sr_groups)
+            src_rcv_items<REF, T>(a, I, R, sr_at * kGroup + tid, R.sr_groups * kGroup, s > 0);
         if constexpr (sizeof(T) == 2) {
             __syncthreads();
             if (tid == 0 && G.i1 > G.i0 && smax[group]) {
