@@ -2440,10 +2440,11 @@ void Engine::Impl::build_resident() {
     const double c_plane = 1.0, c_item = 1.0, c_lrs = 4.0, c_pml = 6.0, c_pair = 6.0, c_rcv = 2.0;
     const int64_t lrs = (int64_t)lrs_cell.n * prm.batch, planes = nz - 2, units = pml ? pml_units * prm.batch : 0;
     const double fixed = (lrs + 255) / 256 * c_lrs + (units + 255) / 256 * c_pml;
-    // groups that take the sources and receivers alone: as many as leave each no
-    // more of them than another group's share, in whole passes of 256 (one group
+    // Groups that take the sources and receivers alone: as many as leave each no
+    // more of them than another group's share, in whole passes of 256. One group
     // for all of them, every member walking all source cells, took 257 us a step
-    // for 256 members of 28x22x18 with a source each)
+    // for 256 members of 28x22x18 with a source each (24 now) and 35 for 16 members
+    // with 1000 receivers (6.5 now).
     const double cols = (double)R.ncol * prm.batch / 256.0;
     const int64_t rcv = (int64_t)rcv_n_dev * prm.batch, sr_items = (sr_n + 31) / 32 * 32 + rcv;
     const double sr_cost = sr_n / 256.0 * c_pair + rcv / 256.0 * c_rcv;
@@ -2453,9 +2454,12 @@ void Engine::Impl::build_resident() {
         {std::max<int64_t>((int64_t)std::ceil(sr_cost / std::max(share, c_pair)), 1), passes, (int64_t)sms});
     R.by_rcv.set((uint32_t)std::max(rcv_n_dev, 1));
     const int64_t all = (int64_t)sms * kResGroups - R.sr_groups;
-    // columns of zc planes: about one item per thread of the remaining groups
+    // columns of zc planes: about one item per thread of the remaining groups, but
+    // of 8 planes at most: whole passes of 256 longer ones leave the groups uneven
+    // (64x48x40 by 42 members 43.9 us a step with up to 16 planes, slower than
+    // launches, 36.3 with 8; by 32 26.5 and 23.0; 192x176x154 23.7 and 22.4)
     int zc = 1;
-    while (zc < 16 && zc < planes &&
+    while (zc < 8 && zc < planes &&
            cols * ((planes + zc - 1) / zc) * (zc * c_plane + c_item) + fixed > all * (zc * c_plane + c_item))
         ++zc;
     R.zc = zc;

@@ -13,9 +13,10 @@
 // barrier here is 1.5 us, the boundary role 2.2, an interior column 0.9 and the
 // sources and receivers 3.0. So what does not change from step to step is kept
 // in registers across them (the first boundary entry of a thread, the rotating
-// indices) and the items are found without divisions. A step measured 4.9 us
+// indices) and the items are found without divisions. A step measured 3.9 us
 // for 28x22x18 (13.5 as launches), 15.0 for 160x120x100 with one PML face (20)
-// and 48.8 for 204x157x131 with six (62).
+// and 47.5 for 204x157x131 with six (62); 24.3 for 256 members of 28x22x18 with a
+// source each and 6.5 for 16 with 1000 receivers (42 and 25).
 #pragma once
 
 constexpr int kGroup = 256;
