@@ -5,7 +5,6 @@
 // the FP32 results reproducible operation by operation on the CPU.
 #pragma once
 
-#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <cuda_fp16.h>
@@ -20,29 +19,14 @@ struct GridDev {
     int64_t pitch, plane, vol;
 };
 
-// a / b rounded to nearest from y = recip_of(b), for divisors that many
-// quotients share: two residual corrections (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34, 1990: with a correctly rounded reciprocal and a quotient within one
-// unit, q + y (a - b q) is correctly rounded). The residuals are exact while
-// their last bits stay above the smallest subnormal: b in 2^-40 .. 2^40 (y is
-// NaN elsewhere) and a quotient in 2^-60 .. 2^80. A zero is its own quotient
-// (silent cells are common); everything else takes the division itself.
-__host__ __device__ inline float recip_of(float b) { return b >= 0x1p-40f && b <= 0x1p40f ? 1.0f / b : NAN; }
-__device__ __forceinline__ float div_shared(float a, float b, float y) {
-    const float q0 = a * y;
-    const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
-    float q = __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
-    if (!(fabsf(q) >= 0x1p-60f && fabsf(q) <= 0x1p80f)) q = a == 0.0f && y == y ? q0 : a / b;
-    return q;
-}
-
 // Quotients of one material that every point of it uses, each formed by the
 // point update's own operations, so that using them changes no rounding:
-// ratio = l a0 / b0, t1 = l2 / b0, t3 = a0 / (l b0), t4 = 1 / a0; rb = 1 / b0
-// and rden = 1 / (1 + ratio) for div_shared.
+// ratio = l a0 / b0, t1 = l2 / b0, t3 = a0 / (l b0), t4 = 1 / a0. (Without the
+// table the 16-member 256x192x160 case takes 88.1 to 88.7 ms instead of 87.7, the
+// others the same; dividing by reciprocal and residuals where many quotients share
+// a divisor changed no case and was left out: 416x160x288 56.8 us a step, 57.3 with.)
 struct alignas(16) LrsMat {
-    float b0, ratio, t1, t3, t4, rb, rden, pad;
+    float b0, ratio, t1, t3, t4, pad[3];
 };
 
 // Compact boundary (LRS) list. Entry e: linear cell index, packed info
@@ -401,8 +385,9 @@ __constant__ uint8_t c_group_mask[26];
 
 __device__ __forceinline__ LrsMat lrs_mat(const LrsDev& L, int m) {
     const float4* p = reinterpret_cast<const float4*>(L.mat + m);
-    const float4 u = __ldg(p), v = __ldg(p + 1);
-    return LrsMat{u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    const float4 u = __ldg(p);
+    const float t4 = __ldg(&L.mat[m].t4);
+    return LrsMat{u.x, u.y, u.z, u.w, t4, {0.0f, 0.0f, 0.0f}};
 }
 
 // One boundary point update. Returns p^{n+1} of the cell and writes the
@@ -460,11 +445,10 @@ __device__ __forceinline__ float lrs_point(const LrsDev& L, int e, int b, uint32
     const float S = lrs_neighbour_sum(c_group_mask[group], nb);
     float gb[3];  // gn / b0
 #pragma unroll
-    for (int f = 0; f < 3; ++f) gb[f] = f < nf ? div_shared(gn[f], M[f].b0, M[f].rb) : 0.0f;
+    for (int f = 0; f < 3; ++f) gb[f] = f < nf ? gn[f] / M[f].b0 : 0.0f;
     float pn;
     if (nf == 1) {
-        pn = div_shared(l2 * S + L.c2 * pc + M[0].t1 * gn[0] + (M[0].ratio - 1.0f) * pold, 1.0f + M[0].ratio,
-                        M[0].rden);
+        pn = (l2 * S + L.c2 * pc + M[0].t1 * gn[0] + (M[0].ratio - 1.0f) * pold) / (1.0f + M[0].ratio);
     } else if (nf == 2 || REF) {
         if (REF && group == 25) {
             pn = pint;  // no variant define reaches lrs_3.cl for this group
@@ -536,8 +520,8 @@ __device__ __forceinline__ float lrs_face(const LrsDev& L, int e, int b, int d, 
         S = S + nb[3];
         S = S + 2.0f * nb[d == 4 ? 5 : 4];
     }
-    const float pn = div_shared(L.l2 * S + L.c2 * pc + M.t1 * gn + (M.ratio - 1.0f) * pold, 1.0f + M.ratio, M.rden);
-    const float xn = M.t3 * (pn - pold) - div_shared(gn, M.b0, M.rb);
+    const float pn = (L.l2 * S + L.c2 * pc + M.t1 * gn + (M.ratio - 1.0f) * pold) / (1.0f + M.ratio);
+    const float xn = M.t3 * (pn - pold) - gn / M.b0;
     sin_[at(ix_buf)] = xn;
     sout[at(ix_buf)] = M.t4 * (M.b0 * xn + gn);
     return pn;

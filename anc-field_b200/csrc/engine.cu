@@ -1981,14 +1981,12 @@ void Engine::Impl::init_device() {
         for (int m = 0; m < model.nmat; ++m) {
             const float a0 = model.a[(size_t)m * model.ncoef], b0 = model.b[(size_t)m * model.ncoef];
             LrsMat& q = t[(size_t)m];
+            q = LrsMat{};
             q.b0 = b0;
             q.ratio = l * a0 / b0;
             q.t1 = l2 / b0;
             q.t3 = a0 / (l * b0);
             q.t4 = 1.0f / a0;
-            q.rb = recip_of(b0);
-            q.rden = recip_of(1.0f + q.ratio);
-            q.pad = 0.0f;
         }
         lrs_mat_dev.upload(t);
     }
