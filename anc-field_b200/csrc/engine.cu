@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(256) k_interior(StepArgs a, int j) {
 // compact list.
 // KT: filter length fixed at compile time (1..4), 0 for any length.
 // T: level storage (FP16 only with the FIXED scheme).
-// Memory-latency-bound gathers: 5 blocks per SM (48 registers, no spills
-// for the FIXED variants) keep more loads in flight than 4.
+// Memory-latency-bound gathers: 5 blocks per SM (48 registers; 16 to 48 bytes spill
+// around the calls of the source cells) keep more loads in flight than 4.
 // One boundary point e of batch member b at global step g: reads p^n and
 // p^{n-1} around the cell, returns p^{n+1} of the cell (unscaled) and writes
 // its filter state. `info`: the entry's packed info. NC: the levels are
@@ -757,8 +757,9 @@ __device__ __forceinline__ BoxThread box_thread(const BoxLaunch& L) {
     return t;
 }
 
-// PML pressure over every box of the disjoint box cover in one launch. Four
-// blocks per SM (64 registers in every variant).
+// PML pressure over every box of the disjoint box cover in one launch. Three
+// blocks per SM (80 registers; a few values spill in the FP32 variants): two and four
+// were slower on 512x384x320, 203 us a step against 203 to 215.
 template <bool PSI, typename T>
 __global__ void __launch_bounds__(256, 3) k_pml_p_all(const __grid_constant__ StepArgs a,
                                                       const __grid_constant__ BoxLaunch L, int j) {
@@ -1536,14 +1537,19 @@ struct Source {
 
 // Source cells that the step's own kernels take (one block's table).
 constexpr int kMaxSrcCells = 256;
-// Cells (all members, rows as padded) up to which the resident kernel runs.
-// Against replayed launches it measured (us a step; FP32 without a PML, FP32
-// with six PML faces, FP16 with two): 5.2 / 14.2 / 13.5 to 10.3 / 20.6 / 19.2 at
-// 0.06 M cells, 7.6 / 20.3 / 15.5 to 12.1 / 27.7 / 22.4 at 0.94 M, 13.8 / 27.0 /
-// 21.2 to 15.3 / 43.5 / 28.2 at 2.1 M, 24.9 / 58.3 / 34.1 to 25.0 / 73.6 / 40.3
-// at 5.6 M (26.1 in another form of the dealing), and 42.2 / 79.8 / 45.7 to 33.8
-// / 90.8 / 48.2 at 8.7 M, where the streaming kernel's TMA tiles beat the
-// columns of plain loads; with a PML, whose launches it saves, the lines cross later.
+// Cells (all members, rows as padded) up to which the resident kernel runs. Against
+// replayed launches (us a step, resident and launches):
+//   cells      FP32, no PML   FP32, one face  FP32, six faces  FP16, two faces
+//   0.06 M      5.2 / 10.3     10.0 / 16.3     14.2 / 20.6      13.5 / 19.2
+//   0.94 M      7.6 / 12.1     13.1 / 17.2     20.3 / 27.7      15.5 / 22.4
+//   2.1 M      13.8 / 15.3     16.9 / 20.2     27.0 / 43.5      21.2 / 28.2
+//   5.2 M      22.6 / 23.5          -               -                -
+//   5.6 M      24.9 / 25.0     29.9 / 32.5     58.3 / 73.6      34.1 / 40.3
+//   6.3 M           -          32.3 / 32.1     53.0 / 63.8      35.2 / 44.6
+//   8.7 M      42.2 / 33.8     47.5 / 42.8     79.8 / 90.8      45.7 / 48.2
+// Without a PML, and with one face from about 6.3 M cells on, the streaming kernel's
+// TMA tiles beat the columns of plain loads; two and six faces stay ahead to the
+// largest size measured. One limit for every PML: where one face stops gaining.
 constexpr int64_t kResidentCells = 5 << 20, kResidentCellsPml = 6 << 20;
 
 struct Engine::Impl {

@@ -12,7 +12,7 @@
 // steps of 64 through a ring of TMA stages. Warp 0 streams tiles, warp 1
 // allocates TMEM, issues tcgen05.mma (K = 16 per instruction) and commits stage
 // releases, warps 2-5 read the accumulator with tcgen05.ld and run the
-// epilogue. Four forms, chosen by gemm_cost:
+// epilogue. Four forms, chosen by plan_gemm:
 //   k_gemm_p  persistent, one CTA per SM looping over 128 x 256 output
 //             tiles, 4-stage ring of 48 KB, two 256-column TMEM accumulators so
 //             that the epilogue of one tile overlaps the MMAs of the next;
