@@ -442,24 +442,24 @@ __device__ __forceinline__ float face4(float v0, float v1, float v2, float v3) {
     return 0.25f * (((v0 + v1) + v2) + v3);
 }
 
-// Adds axis AX's term of the divergence of the auxiliary fields to d[0..3],
+// Adds axis AX's term of the divergence of the auxiliary fields to d[0..N-1],
 // from the rows r00 (y, z), r01 (y, z+1), r10 (y+1, z), r11 (y+1, z+1), cells
-// x..x+4 (pml.cl:189-195; axes in x, y, z order).
-template <int AX>
-__device__ __forceinline__ void pml_div(const float r00[5], const float r01[5], const float r10[5],
-                                        const float r11[5], float d[4]) {
+// x..x+N (pml.cl:189-195; axes in x, y, z order).
+template <int AX, int N = 4>
+__device__ __forceinline__ void pml_div(const float* r00, const float* r01, const float* r10, const float* r11,
+                                        float* d) {
     if constexpr (AX == 0) {
-        float av[5];
+        float av[N + 1];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) av[q] = face4(r00[q], r01[q], r10[q], r11[q]);
+        for (int q = 0; q < N + 1; ++q) av[q] = face4(r00[q], r01[q], r10[q], r11[q]);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) d[q] = av[q + 1] - av[q];
+        for (int q = 0; q < N; ++q) d[q] = av[q + 1] - av[q];
     } else {
         // y: rows of y+1 against rows of y; z: rows of z+1 against rows of z
         const float* u0 = AX == 1 ? r10 : r01;
         const float* l1 = AX == 1 ? r01 : r10;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < N; ++q) {
             d[q] = d[q] + face4(u0[q], r11[q], u0[q + 1], r11[q + 1]);
             d[q] = d[q] - face4(r00[q], l1[q], r00[q + 1], l1[q + 1]);
         }
@@ -468,8 +468,8 @@ __device__ __forceinline__ void pml_div(const float r00[5], const float r01[5], 
 
 // Difference of the face averages along AX of the rows as in pml_div.
 template <int AX>
-__device__ __forceinline__ void face_ends(const float r00[5], const float r01[5], const float r10[5],
-                                          const float r11[5], int q, float* hi, float* lo) {
+__device__ __forceinline__ void face_ends(const float* r00, const float* r01, const float* r10, const float* r11,
+                                          int q, float* hi, float* lo) {
     if constexpr (AX == 0) {
         *hi = face4(r00[q + 1], r01[q + 1], r10[q + 1], r11[q + 1]);
         *lo = face4(r00[q], r01[q], r10[q], r11[q]);
@@ -506,73 +506,100 @@ __device__ __forceinline__ void row5n(const T* p, float r[5], float inv, bool fi
     }
 }
 
-// PML pressure (pml.cl:185-207) of the cells x..x+3 of row (y, z) into v, not
+// The N values x..x+N-1 of a row (x a multiple of 4 for N = 4) and, with `last`,
+// the one after them.
+template <bool NC, int N, typename T>
+__device__ __forceinline__ void rown(const T* p, float* r, float inv, bool last) {
+    if constexpr (N == 4) {
+        row5n<NC>(p, r, inv, last);
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; ++q) r[q] = lvl<NC>(p + q, inv);
+        r[N] = last ? lvl<NC>(p + N, inv) : 0.0f;
+    }
+}
+template <int N>
+__device__ __forceinline__ void storen(float* p, const float* v, unsigned m) {
+    if constexpr (N == 4) {
+        store4(p, v, m);
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            if (m >> q & 1u) p[q] = v[q];
+    }
+}
+
+// PML pressure (pml.cl:185-207) of the cells x..x+N-1 of row (y, z) into v, not
 // stored, with their damping sums ks and the old and new psi (pmh, ps; PSI:
 // psi is kept). ra: axes whose auxiliary fields are read; elsewhere they are
-// identically zero. row0 receives p^n of x..x+4.
-template <bool PSI, typename T, bool NC>
+// identically zero. row0 receives p^n of x..x+N.
+template <bool PSI, typename T, bool NC, int N = 4>
 __device__ __forceinline__ void pml_p_calc(const StepArgs& a, size_t base, int x, int y, int z, const StepIdx& I,
-                                           const LevelScales& sc, unsigned ra, float v[4], float ps[4],
-                                           float row0[5]) {
+                                           const LevelScales& sc, unsigned ra, float* v, float* ps, float* row0) {
     const PmlDev& P = a.pml;
     const int pitch = (int)a.g.pitch, plane = (int)a.g.plane;
     const int i = z * plane + y * pitch + x;  // a member has fewer than 2^31 cells
     const T* pc = level_ptr<T>(a, I.wc) + base;
     const T* po = level_ptr<T>(a, I.wo) + base;
     const float ic = sc.ic;
-    // x+4 is read only where it lies in the row (the unit's last cell can be
+    // x+N is read only where it lies in the row (the unit's last cell can be
     // a PML cell only then)
-    const bool hi = x + 4 < pitch;
+    const bool hi = x + N < pitch;
     float* const c = row0;
-    float ym4[5], yp4[5], zm4[5], zp4[5], o[5];
-    row5n<NC>(pc + i, c, ic, hi);
+    float ym[N + 1], yp[N + 1], zm[N + 1], zp[N + 1], o[N + 1], kx[N + 1];
+    rown<NC, N>(pc + i, c, ic, hi);
     const float xm = x >= 1 ? lvl<NC>(pc + i - 1, ic) : 0.0f;
-    row5n<NC>(pc + (i - pitch), ym4, ic, false);
-    row5n<NC>(pc + (i + pitch), yp4, ic, false);
-    row5n<NC>(pc + (i - plane), zm4, ic, false);
-    row5n<NC>(pc + (i + plane), zp4, ic, false);
-    row5n<NC>(po + i, o, sc.io, false);
-    const float4 kx4 = __ldg(reinterpret_cast<const float4*>(P.ksi[0] + x));
-    const float kx[4] = {kx4.x, kx4.y, kx4.z, kx4.w};
+    rown<NC, N>(pc + (i - pitch), ym, ic, false);
+    rown<NC, N>(pc + (i + pitch), yp, ic, false);
+    rown<NC, N>(pc + (i - plane), zm, ic, false);
+    rown<NC, N>(pc + (i + plane), zp, ic, false);
+    rown<NC, N>(po + i, o, sc.io, false);
+    rown<true, N>(P.ksi[0] + x, kx, 1.0f, false);
     const float ky = __ldg(P.ksi[1] + y), kz = __ldg(P.ksi[2] + z);
-    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float d[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) d[q] = 0.0f;
     auto field = [&](int ax, auto add) {
         const float* f = P.fi[ax][I.lv ^ 1] + base;
-        float r00[5], r01[5], r10[5], r11[5];
-        row5n<NC>(f + i, r00, 1.0f, hi);
-        row5n<NC>(f + (i + plane), r01, 1.0f, hi);
-        row5n<NC>(f + (i + pitch), r10, 1.0f, hi);
-        row5n<NC>(f + (i + pitch + plane), r11, 1.0f, hi);
+        float r00[N + 1], r01[N + 1], r10[N + 1], r11[N + 1];
+        rown<NC, N>(f + i, r00, 1.0f, hi);
+        rown<NC, N>(f + (i + plane), r01, 1.0f, hi);
+        rown<NC, N>(f + (i + pitch), r10, 1.0f, hi);
+        rown<NC, N>(f + (i + pitch + plane), r11, 1.0f, hi);
         add(r00, r01, r10, r11);
     };
-    if (ra & 1u) field(0, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<0>(q, r, s, t, d); });
-    if (ra & 2u) field(1, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<1>(q, r, s, t, d); });
-    if (ra & 4u) field(2, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<2>(q, r, s, t, d); });
-    float pmh[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (ra & 1u) field(0, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<0, N>(q, r, s, t, d); });
+    if (ra & 2u) field(1, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<1, N>(q, r, s, t, d); });
+    if (ra & 4u) field(2, [&](auto& q, auto& r, auto& s, auto& t) { pml_div<2, N>(q, r, s, t, d); });
+    float pmh[N + 1];
     if (PSI) {
-        const float4 h = *reinterpret_cast<const float4*>(P.psi[I.lv ^ 1] + base + i);
-        pmh[0] = h.x;
-        pmh[1] = h.y;
-        pmh[2] = h.z;
-        pmh[3] = h.w;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) ps[q] = PSI ? P.dt * c[q] + pmh[q] : 0.0f;
-    // ks depends on kx only within the row: one division when the four agree
-    float ks[4];
-    if (kx[0] == kx[1] && kx[1] == kx[2] && kx[2] == kx[3]) {
-        ks[0] = ks[1] = ks[2] = ks[3] = (kx[0] + ky + kz) / P.two_dt;
+        rown<false, N>(P.psi[I.lv ^ 1] + base + i, pmh, 1.0f, false);
     } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) ks[q] = (kx[q] + ky + kz) / P.two_dt;
+        for (int q = 0; q < N; ++q) pmh[q] = 0.0f;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < N; ++q) ps[q] = PSI ? P.dt * c[q] + pmh[q] : 0.0f;
+    // ks depends on kx only within the row: one division when all agree
+    float ks[N];
+    bool same = N > 1;
+#pragma unroll
+    for (int q = 1; q < N; ++q) same = same && kx[q - 1] == kx[q];
+    if (same) {
+        const float k0 = (kx[0] + ky + kz) / P.two_dt;
+#pragma unroll
+        for (int q = 0; q < N; ++q) ks[q] = k0;
+    } else {
+#pragma unroll
+        for (int q = 0; q < N; ++q) ks[q] = (kx[q] + ky + kz) / P.two_dt;
+    }
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
         float s6 = c[q + 1] + (q == 0 ? xm : c[q - 1]);
-        s6 = s6 + yp4[q];
-        s6 = s6 + ym4[q];
-        s6 = s6 + zp4[q];
-        s6 = s6 + zm4[q];
+        s6 = s6 + yp[q];
+        s6 = s6 + ym[q];
+        s6 = s6 + zp[q];
+        s6 = s6 + zm[q];
         v[q] = pml_p_cell(P, s6, c[q], o[q], kx[q], ky, kz, ks[q], d[q], ps[q], pmh[q],
                           [](float n, float den) { return n / den; });
     }
@@ -671,25 +698,36 @@ __device__ __forceinline__ void pml_aux_unit(const StepArgs& a, int b, int x, in
 // (pml.cl:185-188): first the auxiliary fields, with the cell's own new
 // pressure and psi formed locally, then pressure and psi. Units of four cells
 // as in FIXED mode: the kernels are bound by load instructions (every array of
-// a grid stays in L2), of which a thread per cell issued 60.
+// a grid stays in L2), of which a thread per cell issued 60. Grids too small to
+// fill the chip with such units take one cell a thread, whose chain of
+// arithmetic is a quarter as long (see kRefOneCell).
 //
-// The cells 2..nx-3 of unit x..x+3 as a mask.
+// Units of a row that hold a cell 2..nx-3, and the first cell of one.
+__host__ __device__ inline int ref_row_units(int nx, int n) { return n == 4 ? (nx + 1) / 4 : nx - 4; }
+template <int N>
+__device__ __forceinline__ int ref_unit_x(int u) {
+    return N == 4 ? 4 * u : 2 + u;
+}
+// The cells 2..nx-3 of unit x..x+N-1 as a mask (units of one cell are all inside).
+template <int N>
 __device__ __forceinline__ unsigned ref_cells(const StepArgs& a, int x) {
+    if constexpr (N == 1) return 1u;
     unsigned m = x == 0 ? 12u : 15u;
     if (x + 3 > a.g.nx - 3) m &= (1u << (a.g.nx - 2 - x)) - 1u;
     return m;
 }
-// Unit u of plane z of the launch: cells x..x+3, valid ones as the mask m.
+// Unit u of plane z of the launch: cells x..x+N-1, valid ones as the mask m.
+template <int N>
 __device__ __forceinline__ bool ref_unit(const StepArgs& a, int* b, int* x, int* y, int* z, unsigned* m) {
-    const unsigned nu = (unsigned)(a.g.nx + 1) / 4;  // units that hold a cell 2..nx-3
+    const unsigned nu = (unsigned)ref_row_units(a.g.nx, N);
     const unsigned u = blockIdx.x * blockDim.x + threadIdx.x, row = u / nu;
     const int zn = a.g.nz - 4;
     *b = (int)blockIdx.y / zn;
     *z = 2 + (int)blockIdx.y % zn;
     *y = 2 + (int)row;
-    *x = 4 * (int)(u - row * nu);
+    *x = ref_unit_x<N>((int)(u - row * nu));
     if (*y > a.g.ny - 3) return false;
-    *m = ref_cells(a, *x);
+    *m = ref_cells<N>(a, *x);
     return true;
 }
 // axes whose slabs meet x0..x1, y0..y1, z0..z1
@@ -699,20 +737,21 @@ __device__ __forceinline__ unsigned ref_axes(const StepArgs& a, int x0, int x1, 
            (z0 < W || z1 > a.g.nz - W - 1 ? 4u : 0u);
 }
 
-// Pressure and psi of every cell 2..n-3 (pml.cl:182-207).
+// Pressure and psi of every cell 2..n-3 (pml.cl:182-207), N cells a thread.
+template <int N>
 __global__ void __launch_bounds__(256) k_pml_ref_p(StepArgs a, int j) {
     const StepIdx I = step_at(a, j);
     const TlMark tl(a, 2, I.g, blockIdx.y < (unsigned)(a.g.nz - 4));
     int b, x, y, z;
     unsigned m;
-    if (!ref_unit(a, &b, &x, &y, &z, &m)) return;
+    if (!ref_unit<N>(a, &b, &x, &y, &z, &m)) return;
     const size_t base = (size_t)b * a.g.vol;
     const int i = z * (int)a.g.plane + y * (int)a.g.pitch + x;
-    float v[4], ps[4], c[5];
-    pml_p_calc<true, float, true>(a, base, x, y, z, I, level_scales<float>(a, b, I.s5),
-                                  ref_axes(a, x, x + 4, y, y + 1, z, z + 1), v, ps, c);
-    store4(a.pml.psi[I.lv] + base + i, ps, m);
-    store4(a.p[I.wn] + base + i, v, m);
+    float v[N], ps[N], c[N + 1];
+    pml_p_calc<true, float, true, N>(a, base, x, y, z, I, level_scales<float>(a, b, I.s5),
+                                     ref_axes(a, x, x + N, y, y + 1, z, z + 1), v, ps, c);
+    storen<N>(a.pml.psi[I.lv] + base + i, ps, m);
+    storen<N>(a.p[I.wn] + base + i, v, m);
 }
 
 // One launch over several PML boxes: a flat grid whose blocks are dealt to
@@ -778,48 +817,59 @@ __global__ void __launch_bounds__(256, 3) k_pml_p_all(const __grid_constant__ St
 // pml.cl:247). The cell's own p and psi are the first of the four values of
 // its lower faces. The launch covers the slabs' units with boxes: as one flat
 // grid over all units, two thirds of the warps held a few slab units each and
-// the pass took 24 us at 160x120x100.
+// the pass took 24 us at 160x120x100. A box's rows follow one another through all
+// its planes: by planes, thin slabs of small grids left most of a block idle (the x
+// slabs of 28x22x18 14 of 256 threads; 64 members 56.8 us a step, now 36.2, and 46.7
+// with the thread per cell of all cells from which this came; 256 members 180, 91, 142).
+template <int N>
 __global__ void __launch_bounds__(256) k_pml_ref_aux(const __grid_constant__ StepArgs a,
                                                      const __grid_constant__ BoxLaunch L, int j) {
     const StepIdx I = step_at(a, j);
-    const BoxThread t = box_thread(L);
-    const TlMark tl(a, 3, I.g, t.b == 0);
-    if (!t.ok) return;
-    const int b = t.b, x = t.x, y = t.y, z = t.z0;
-    const unsigned m = ref_cells(a, x), axes = ref_axes(a, x, x + 3, y, y, z, z);
+    int k = 0;
+    while (k + 1 < L.n && (int)blockIdx.x >= L.start[k + 1]) ++k;
+    const PmlBox& bx = L.box[k];
+    const int w = L.w[k], rows = L.gzc[k];
+    int r = (int)blockIdx.x - L.start[k];
+    const int ux = r % L.gx[k] * w + (int)threadIdx.x % w;
+    r /= L.gx[k];
+    const int row = r % L.gy[k] * rows + (int)threadIdx.x / w, b = r / L.gy[k];
+    const TlMark tl(a, 3, I.g, b == 0);
+    if ((int)threadIdx.x >= rows * w || ux >= bx.units || row >= bx.height * bx.depth) return;
+    const int zi = row / bx.height;
+    const int x = bx.x0 + N * ux, y = bx.y0 + (row - zi * bx.height), z = bx.z0 + zi;
+    const unsigned m = ref_cells<N>(a, x), axes = ref_axes(a, x, x + N - 1, y, y, z, z);
     if (!axes) return;
     const PmlDev& P = a.pml;
     const size_t base = (size_t)b * a.g.vol;
     const int pitch = (int)a.g.pitch, plane = (int)a.g.plane, i = z * plane + y * pitch + x;
-    const bool hi = x + 4 < pitch;
+    const bool hi = x + N < pitch;
     const LevelScales sc = level_scales<float>(a, b, I.s5);
-    float own[4], ps[4], m00[5];
-    pml_p_calc<true, float, true>(a, base, x, y, z, I, sc, ref_axes(a, x, x + 4, y, y + 1, z, z + 1), own, ps, m00);
+    float own[N], ps[N], m00[N + 1];
+    pml_p_calc<true, float, true, N>(a, base, x, y, z, I, sc, ref_axes(a, x, x + N, y, y + 1, z, z + 1), own, ps, m00);
     const float *pn = a.p[I.wn] + base, *pc = a.p[I.wc] + base, *sp = P.psi[I.lv] + base;
-    float n00[5], n01[5], n10[5], n11[5], m01[5], m10[5], m11[5], s00[5], s01[5], s10[5], s11[5];
-    row5(pn + i, n00, hi);
-    row5(pn + (i + plane), n01, hi);
-    row5(pn + (i + pitch), n10, hi);
-    row5(pn + (i + pitch + plane), n11, hi);
-    row5(pc + (i + plane), m01, hi);
-    row5(pc + (i + pitch), m10, hi);
-    row5(pc + (i + pitch + plane), m11, hi);
-    row5(sp + i, s00, hi);
-    row5(sp + (i + plane), s01, hi);
-    row5(sp + (i + pitch), s10, hi);
-    row5(sp + (i + pitch + plane), s11, hi);
-    float kxs[5];
-    row5(P.ksi[0] + x, kxs, hi);
+    float n00[N + 1], n01[N + 1], n10[N + 1], n11[N + 1], m01[N + 1], m10[N + 1], m11[N + 1], s00[N + 1], s01[N + 1],
+        s10[N + 1], s11[N + 1], kxs[N + 1];
+    rown<true, N>(pn + i, n00, 1.0f, hi);
+    rown<true, N>(pn + (i + plane), n01, 1.0f, hi);
+    rown<true, N>(pn + (i + pitch), n10, 1.0f, hi);
+    rown<true, N>(pn + (i + pitch + plane), n11, 1.0f, hi);
+    rown<true, N>(pc + (i + plane), m01, 1.0f, hi);
+    rown<true, N>(pc + (i + pitch), m10, 1.0f, hi);
+    rown<true, N>(pc + (i + pitch + plane), m11, 1.0f, hi);
+    rown<true, N>(sp + i, s00, 1.0f, hi);
+    rown<true, N>(sp + (i + plane), s01, 1.0f, hi);
+    rown<true, N>(sp + (i + pitch), s10, 1.0f, hi);
+    rown<true, N>(sp + (i + pitch + plane), s11, 1.0f, hi);
+    rown<true, N>(P.ksi[0] + x, kxs, 1.0f, hi);
     const float kay = 0.5f * (__ldg(P.ksi[1] + y) + __ldg(P.ksi[1] + y + 1));
     const float kaz = 0.5f * (__ldg(P.ksi[2] + z) + __ldg(P.ksi[2] + z + 1));
     const float kxy = 0.5f * (__ldg(P.ksi[0] + y) + __ldg(P.ksi[0] + y + 1));
     auto field = [&](auto axis, unsigned cells) {
         constexpr int AX = decltype(axis)::value;
-        const float4 f14 = *reinterpret_cast<const float4*>(P.fi[AX][I.lv ^ 1] + base + i);
-        const float f1[4] = {f14.x, f14.y, f14.z, f14.w};
-        float out[4];
+        float f1[N + 1], out[N];
+        rown<false, N>(P.fi[AX][I.lv ^ 1] + base + i, f1, 1.0f, false);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
+        for (int q = 0; q < N; ++q) {
             float nh, nl, mh, ml, sh, sl;
             face_ends<AX>(n00, n01, n10, n11, q, &nh, &nl);
             face_ends<AX>(m00, m01, m10, m11, q, &mh, &ml);
@@ -841,12 +891,12 @@ __global__ void __launch_bounds__(256) k_pml_ref_aux(const __grid_constant__ Ste
             out[q] = pml_aux_cell(P, f1[q], AX == 0 ? kax : (AX == 1 ? kay : kaz), k1, k2, dp,
                                   AX == 1 ? kxy * kaz : k1 * k2, dpsi, [](float n, float den) { return n / den; });
         }
-        store4(P.fi[AX][I.lv] + base + i, out, cells);
+        storen<N>(P.fi[AX][I.lv] + base + i, out, cells);
     };
     if (axes & 1u) {
         unsigned cells = 0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < N; ++q)
             if (x + q < P.width || x + q > a.g.nx - P.width - 1) cells |= 1u << q;
         field(std::integral_constant<int, 0>{}, m & cells);
     }
@@ -1552,6 +1602,16 @@ constexpr int kMaxSrcCells = 256;
 // largest size measured. One limit for every PML: where one face stops gaining.
 constexpr int64_t kResidentCells = 5 << 20, kResidentCellsPml = 6 << 20;
 
+// Cells 2..n-3 (all members) up to which the REF-mode PML takes one cell a thread
+// instead of four, and up to which the rows of its slabs are spread over more blocks
+// (us a step, layers of 4 and 12 cells, six faces): 32x32x32 20.5 and 21.0 against
+// 22.5 and 22.9 with four cells, 64x48x40 21.1 and 21.5 against 22.7 and 23.2,
+// 64x64x48 (158000 cells) 22.6 and 23.0 against 22.8 and 23.3 but 26.0 against 23.3
+// with a layer that fills the grid, 80x72x60 23.8 and 27.9 against 23.9 and 25.4.
+// 64 rows a block: 96x72x64 24.2 and 25.2 against 26.3 and 25.7, 160x120x100 43.9
+// against 42.7 with a layer of 8.
+constexpr int64_t kRefOneCell = 120000, kRefSpread = 1000000;
+
 struct Engine::Impl {
     afd_params prm{};
     // geometry
@@ -1596,6 +1656,7 @@ struct Engine::Impl {
     DBuf<float> fi[3][2], psi[2];
     DBuf<float> ksi_dev[3];
     std::vector<PmlBox> pml_boxes;
+    int ref_n = 4;  // cells a thread of the REF-mode PML kernels
     std::vector<PmlBox> pml_axis_boxes[3];
     // the launches over all pressure boxes and over all (axis, slab box) pairs
     BoxLaunch pml_p_all{}, pml_aux_all{};
@@ -2154,8 +2215,11 @@ void Engine::Impl::build_fused() {
 // The flat launch over `entries` (box, axis): blocks of 256 threads, w =
 // min(units, 32) units across, zc planes per thread; *blocks receives the
 // grid size.
+// zc = 0 (k_pml_ref_aux): the rows of all planes of a box follow one another, one
+// unit a thread; spread: at most 64 rows a block, for grids whose thin x slabs
+// would leave most SMs idle.
 static BoxLaunch make_box_launch(const std::vector<std::pair<PmlBox, int>>& entries, int batch, int zc,
-                                 int* blocks, int max_w = 32) {
+                                 int* blocks, int max_w = 32, bool spread = false) {
     if ((int)entries.size() > kMaxLaunchBoxes) throw Error(AFD_ERR_ARG, "too many PML boxes for one launch");
     BoxLaunch L{};
     L.n = (int32_t)entries.size();
@@ -2163,15 +2227,22 @@ static BoxLaunch make_box_launch(const std::vector<std::pair<PmlBox, int>>& entr
     int64_t start = 0;
     for (size_t k = 0; k < entries.size(); ++k) {
         const PmlBox& bx = entries[k].first;
-        const int w = std::min(bx.units, max_w), rows = 256 / w;
+        const int w = std::min(bx.units, max_w);
+        int rows = 256 / w;
+        if (zc == 0 && spread) {
+            rows = std::min(rows, 64);
+        } else if (zc == 0) {  // blocks that end with a plane where one fills half of them
+            const int n = (bx.height + rows - 1) / rows, even = (bx.height + n - 1) / n;
+            if (even * w >= 128) rows = even;
+        }
         L.box[k] = bx;
         L.axis[k] = entries[k].second;
         L.w[k] = w;
         L.gx[k] = (bx.units + w - 1) / w;
-        L.gy[k] = (bx.height + rows - 1) / rows;
-        L.gzc[k] = (bx.depth + zc - 1) / zc;
+        L.gy[k] = ((zc ? bx.height : bx.height * bx.depth) + rows - 1) / rows;
+        L.gzc[k] = zc ? (bx.depth + zc - 1) / zc : rows;
         L.start[k] = (int32_t)start;
-        start += (int64_t)L.gx[k] * L.gy[k] * L.gzc[k] * batch;
+        start += (int64_t)L.gx[k] * L.gy[k] * (zc ? L.gzc[k] : 1) * batch;
     }
     if (start >= ((int64_t)1 << 31)) throw Error(AFD_ERR_ARG, "PML launch too large");
     L.start[entries.size()] = (int32_t)start;
@@ -2217,11 +2288,13 @@ void Engine::Impl::setup_pml() {
     }
     if (ref() && nx > 4 && ny > 4 && nz > 4) {
         // REF: the units of the cells 2..n-3 that lie in a slab, z slabs first
-        const int W = pml_width, units = (nx + 1) / 4;
+        const int64_t cells = (int64_t)(nx - 4) * (ny - 4) * (nz - 4) * prm.batch;
+        ref_n = cells <= kRefOneCell ? 1 : 4;
+        const int W = pml_width, units = ref_row_units(nx, ref_n), x_first = ref_n == 4 ? 0 : 2;
         std::vector<std::pair<PmlBox, int>> e;
         auto add = [&](int u0, int u1, int y0, int y1, int z0, int z1) {  // inclusive
             if (u0 > u1 || y0 > y1 || z0 > z1) return;
-            e.emplace_back(PmlBox{4 * u0, u1 - u0 + 1, y0, y1 - y0 + 1, z0, z1 - z0 + 1, 0}, 0);
+            e.emplace_back(PmlBox{x_first + ref_n * u0, u1 - u0 + 1, y0, y1 - y0 + 1, z0, z1 - z0 + 1, 0}, 0);
         };
         // last cell of the lower slab, first of the upper one (2..n-3, disjoint)
         auto ends = [&](int n, int* lo, int* hi) {
@@ -2235,10 +2308,12 @@ void Engine::Impl::setup_pml() {
         add(0, units - 1, 2, ny - 3, hz, nz - 3);
         add(0, units - 1, 2, ly, lz + 1, hz - 1);
         add(0, units - 1, hy, ny - 3, lz + 1, hz - 1);
-        const int lu = W > 2 ? std::min((W - 1) / 4, units - 1) : -1, hu = std::max(std::max(nx - W, 0) / 4, lu + 1);
+        // last unit of the lower x slab, first of the upper one
+        const int lu = W > 2 ? std::min((W - 1 - x_first) / ref_n, units - 1) : -1;
+        const int hu = std::max(std::max(nx - W - x_first, 0) / ref_n, lu + 1);
         add(0, lu, ly + 1, hy - 1, lz + 1, hz - 1);
         add(hu, units - 1, ly + 1, hy - 1, lz + 1, hz - 1);
-        pml_aux_all = make_box_launch(e, prm.batch, 1, &pml_aux_blocks, 256);
+        pml_aux_all = make_box_launch(e, prm.batch, 0, &pml_aux_blocks, 256, cells <= kRefSpread);
     }
     if (!ref()) {
         // FIXED: PML cells are the plain air cells (not solid, not boundary)
@@ -2885,13 +2960,15 @@ void Engine::Impl::launch_step_t(int j, bool profile) {
         if (a.pml.width > 0) {
             if (ref()) {
                 if (sizeof(T) == 4 && nx > 4 && ny > 4 && nz > 4) {
-                    const int64_t units = (int64_t)((nx + 1) / 4) * (ny - 4);
+                    const int64_t units = (int64_t)ref_row_units(nx, ref_n) * (ny - 4);
                     const dim3 grd((unsigned)((units + 255) / 256), (unsigned)((nz - 4) * prm.batch));
                     begin(KK_PML_AUX);
-                    if (pml_aux_blocks > 0) k_pml_ref_aux<<<pml_aux_blocks, 256, 0, stream>>>(a, pml_aux_all, j);
+                    if (pml_aux_blocks > 0 && ref_n == 1) k_pml_ref_aux<1><<<pml_aux_blocks, 256, 0, stream>>>(a, pml_aux_all, j);
+                    else if (pml_aux_blocks > 0) k_pml_ref_aux<4><<<pml_aux_blocks, 256, 0, stream>>>(a, pml_aux_all, j);
                     end();
                     begin(KK_PML_P);
-                    k_pml_ref_p<<<grd, 256, 0, stream>>>(a, j);
+                    if (ref_n == 1) k_pml_ref_p<1><<<grd, 256, 0, stream>>>(a, j);
+                    else k_pml_ref_p<4><<<grd, 256, 0, stream>>>(a, j);
                     end();
                     launches += 2;
                 }
