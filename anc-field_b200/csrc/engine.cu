@@ -1675,8 +1675,10 @@ struct Engine::Impl {
     DBuf<float> src_data;
     DBuf<int32_t> rcv_cell;
     // sources and receivers taken by the step's kernels (SrcRcvDev)
-    DBuf<int32_t> sr_first, sr_member, sr_cell, sr_entry, sr_begin;
-    DBuf<int64_t> sr_len, sr_off;
+    // (one block of each type; few allocations, since a new source uploads them again)
+    DBuf<int32_t> sr_table, sr_mark;
+    DBuf<int64_t> sr_signals;
+    SrcRcvDev sr_dev{};
     int32_t sr_n = 0;
     bool sr_same = true;  // every member has sources in the same cells
     bool sr_ok = false;  // the distinct source cells fit one block's table
@@ -2463,14 +2465,17 @@ void Engine::Impl::upload_source_cells(const std::vector<int32_t>& cell, const s
         where.push_back(inner ? kSrcInterior : kSrcOuter);
     }
     if (lrs_info.n) {
-        DBuf<int32_t> d, w;
-        d.upload(distinct);
-        w.upload(where);
+        if (!sr_mark.ptr) sr_mark.alloc(2 * kMaxSrcCells, false);
+        int32_t *d = sr_mark.ptr, *w = d + kMaxSrcCells;
+        const size_t bytes = distinct.size() * sizeof(int32_t);
+        if (bytes) {
+            CK(cudaMemcpyAsync(d, distinct.data(), bytes, cudaMemcpyHostToDevice, stream));
+            CK(cudaMemcpyAsync(w, where.data(), bytes, cudaMemcpyHostToDevice, stream));
+        }
         k_mark_sources<<<(unsigned)std::min<size_t>((lrs_info.n + 255) / 256, 1184), 256, 0, stream>>>(
-            lrs_cell.ptr, lrs_info.ptr, (int)lrs_info.n, d.ptr, (int)distinct.size(), w.ptr);
+            lrs_cell.ptr, lrs_info.ptr, (int)lrs_info.n, d, (int)distinct.size(), w);
         CK(cudaGetLastError());
-        if (!where.empty())
-            CK(cudaMemcpyAsync(where.data(), w.ptr, where.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        if (bytes) CK(cudaMemcpyAsync(where.data(), w, bytes, cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
     }
     std::vector<int32_t> first{0}, m, c, e, b{0};
@@ -2493,13 +2498,18 @@ void Engine::Impl::upload_source_cells(const std::vector<int32_t>& cell, const s
     }
     sr_n = (int32_t)c.size();
     sr_same = c.size() == distinct.size() * (size_t)prm.batch;
-    sr_first.upload(first);
-    sr_member.upload(m);
-    sr_cell.upload(c);
-    sr_entry.upload(e);
-    sr_begin.upload(b);
-    sr_len.upload(l);
-    sr_off.upload(o);
+    std::vector<int32_t> table;
+    std::vector<size_t> at;
+    for (const auto* v : {&first, &m, &c, &e, &b}) {
+        at.push_back(table.size());
+        table.insert(table.end(), v->begin(), v->end());
+    }
+    sr_table.upload(table);
+    l.insert(l.end(), o.begin(), o.end());
+    sr_signals.upload(l);
+    const int32_t* p = sr_table.ptr;
+    sr_dev = SrcRcvDev{0, sr_n, p + at[0], p + at[1], p + at[2], p + at[3], p + at[4], sr_signals.ptr,
+                       sr_signals.ptr + o.size()};
     res_dirty = true;
 }
 
@@ -2633,7 +2643,8 @@ void Engine::Impl::build_resident() {
         CK(cudaMemcpyAsync(res_owned.ptr + have * words, res_owned.ptr, std::min(have, masks - have) * words * sizeof(uint32_t),
                            cudaMemcpyDeviceToDevice, stream));
     if (sr_n)
-        k_set_bits<<<(sr_n + 255) / 256, 256, 0, stream>>>(sr_cell.ptr, sr_member.ptr, sr_n, R.owned_words, res_owned.ptr);
+        k_set_bits<<<(sr_n + 255) / 256, 256, 0, stream>>>(sr_dev.cell, sr_dev.member, sr_n, R.owned_words,
+                                                           res_owned.ptr);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream));
     R.groups = res_groups.ptr;
@@ -2793,14 +2804,7 @@ void Engine::Impl::build_args() {
     a.src.off = src_off.ptr;
     a.src.len = src_len.ptr;
     a.src.data = src_data.ptr;
-    a.sr.n = sr_n;
-    a.sr.first = sr_first.ptr;
-    a.sr.member = sr_member.ptr;
-    a.sr.cell = sr_cell.ptr;
-    a.sr.entry = sr_entry.ptr;
-    a.sr.begin = sr_begin.ptr;
-    a.sr.len = sr_len.ptr;
-    a.sr.off = sr_off.ptr;
+    a.sr = sr_dev;
     a.rcv.n = rcv_n_dev;
     a.rcv.cell = rcv_cell.ptr;
     a.rcv.out = rcv_out.ptr;
