@@ -1,9 +1,7 @@
 // The estimator's recursion by forward substitution, block by block: the path of
-// the calls whose explicit inverses overflow (a step size so far above the stable
-// range that an error would grow 1e308-fold within a block; the recursion itself
-// stays finite where the errors are zero or small enough, and its values are the
-// answer). Included by lms.cu inside namespace afd::lms. Per block of 128
-// samples
+// the calls whose explicit inverses have large entries (kMaxEntry), or leave the
+// range of FP64 where the recursion itself stays in it because its errors are zero
+// or small. Included by lms.cu inside namespace afd::lms. Per block of 128 samples
 //   k_lms_y0     y0 for the block, taps and samples split over CTAs
 //                (partial sums per tap chunk)
 //   k_lms_solve  one CTA: y0 from the partials, R by lag, the errors

@@ -37,6 +37,21 @@ def test_near_the_stability_limit(pkg, level, kind):
     assert rel(pkg.lms.estimate_ir(x, d, N, mu, epochs=1), want) < TOL
 
 
+# few taps near the limit: within a block an error grows by several orders before
+# it falls again, and the weights converge or stay small all the same. The bar is
+# that of the other tests; by the inverses of 512 samples 1e-9 to 1e-7
+@pytest.mark.parametrize("N,level,seed", [(2, 0.8, 4), (4, 0.85, 1), (4, 0.85, 2), (4, 0.85, 3), (8, 0.9, 4)])
+def test_errors_that_grow_within_a_block(pkg, N, level, seed):
+    rng = np.random.default_rng([N, seed])
+    n = 2600
+    x = rng.standard_normal(n)
+    d = np.convolve(x, [1, 0.5, 0.2])[:n] + 0.01 * rng.standard_normal(n)
+    mu = level / (N * np.mean(x * x))
+    want = lms_oracle.estimate(x, d, N, mu, epochs=1)
+    assert np.abs(want).max() < 1e4
+    assert rel(pkg.lms.estimate_ir(x, d, N, mu, epochs=1), want) < TOL
+
+
 def test_silence_stays_silent_at_any_step_size(pkg):
     """No output to identify: the weights stay zero although an error would grow
     beyond every bound within a block."""
