@@ -1694,8 +1694,12 @@ struct Engine::Impl {
     int32_t rcv_n_dev = 0;
     DBuf<long long> d_step;
     DBuf<StepIdx> step_table;  // [kChunkSteps]
+    int table_K = -1;           // what the table was filled for
+    int64_t table_pml_g0 = -1;
     void advance_table(int n) {
-        k_advance<<<1, kChunkSteps, 0, stream>>>(d_step.ptr, n, step_table.ptr, have_model ? model.ncoef : 1, pml_g0);
+        table_K = have_model ? model.ncoef : 1;
+        table_pml_g0 = pml_g0;
+        k_advance<<<1, kChunkSteps, 0, stream>>>(d_step.ptr, n, step_table.ptr, table_K, pml_g0);
     }
     // headless visualisation (afd_set_capture)
     int32_t cap_batch = 0, cap_axis = 1, cap_index = 0, cap_every = 0, cap_max = 0;
@@ -3474,7 +3478,9 @@ void Engine::Impl::setup_run(int64_t steps) {
         CK(cudaStreamSynchronize(stream));
     }
     build_args();
-    advance_table(0);  // the table follows the filter length and the PML's first step
+    // the table follows the filter length and the PML's first step; a split step
+    // sets up each time (a launch more cost two slabs of one GPU 4 % of a step)
+    if (table_K != (have_model ? model.ncoef : 1) || table_pml_g0 != pml_g0) advance_table(0);
     if (res_dirty && resident()) build_resident();
 }
 

@@ -105,3 +105,26 @@ def test_resident_rooms_on_threads(pkg):
     for k, got in enumerate(beside):
         for a, b in zip(got, alone[k % 4]):
             assert np.array_equal(a, b), forms[k % 4]
+
+
+@pytest.mark.parametrize("route", ["resident", "capture", "plan"])
+@pytest.mark.parametrize("mode,storage", [(0, 0), (1, 0), (1, 1)])
+def test_pml_set_again_between_runs(pkg, route, mode, storage):
+    """A PML set, set again and taken off between runs starts its fields anew at that
+    step on every route: the bits of the serial one."""
+    dims, out = (48, 45, 43), []
+    W = pkg.workloads
+    for r in (route, "serial"):
+        sim, _, _ = build(pkg, dims, mode, 0, storage, graphs=0 if r == "serial" else 1)
+        if r == "capture":
+            sim.set_capture(2, 20, 50)
+        if r == "plan":
+            sim.set_plan()
+        for k, n in enumerate((31, 202, 7, 40)):
+            if k:
+                width = (0, 8, 8, 0)[k]
+                sim.SetPml(width, faces=63 if width else 0, ksi=W.ksi_arrays(dims, 8, 63, kmax=3000.0 * k))
+            sim.Run(n)
+        out.append((sim.mics(), sim.field()))
+        sim.close()
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
