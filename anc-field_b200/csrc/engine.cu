@@ -2547,14 +2547,19 @@ void Engine::Impl::build_resident() {
         {std::max<int64_t>((int64_t)std::ceil(sr_cost / std::max(share, c_pair)), 1), passes, (int64_t)sms});
     R.by_rcv.set((uint32_t)std::max(rcv_n_dev, 1));
     const int64_t all = (int64_t)sms * kResGroups - R.sr_groups;
-    // columns of zc planes: about one item per thread of the remaining groups, but
-    // of 8 planes at most: whole passes of 256 longer ones leave the groups uneven
-    // (64x48x40 by 42 members 43.9 us a step with up to 16 planes, slower than
-    // launches, 36.3 with 8; by 32 26.5 and 23.0; 192x176x154 23.7 and 22.4)
+    // columns of zc planes: about one item per thread of the remaining groups, 16 planes
+    // at most. Where 16 still leave several passes and much of the last column empty
+    // (38 planes in three), even ones of about 10: 64x48x40 by 42 members 43.9 us a
+    // step, slower than launches, and 28.4; by 32 26.3 and 24.8.
+    auto passes_left = [&](int q) {
+        return cols * ((planes + q - 1) / q) * (q * c_plane + c_item) + fixed > all * (q * c_plane + c_item);
+    };
     int zc = 1;
-    while (zc < 8 && zc < planes &&
-           cols * ((planes + zc - 1) / zc) * (zc * c_plane + c_item) + fixed > all * (zc * c_plane + c_item))
-        ++zc;
+    while (zc < 16 && zc < planes && passes_left(zc)) ++zc;
+    if (zc == 16 && passes_left(zc) && (planes + 15) / 16 * 16 > planes + planes / 8) {
+        const int64_t columns = (planes + 9) / 10;
+        zc = (int)((planes + columns - 1) / columns);
+    }
     R.zc = zc;
     R.n_zc = (int32_t)((planes + zc - 1) / zc);
     R.per_member = (int32_t)(((int64_t)R.ncol * R.n_zc + 31) / 32 * 32);
